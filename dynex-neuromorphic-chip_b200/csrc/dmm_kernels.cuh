@@ -278,7 +278,14 @@ __device__ __forceinline__ double sort_sum_vals(double (&a)[R], int d, int lane)
   return acc;
 }
 
-template <int R, bool DIRECT, class Idx>
+// Entry j of a slot list in global (GLOBAL) or shared memory.
+template <bool GLOBAL, class Idx>
+__device__ __forceinline__ int list_at(const Idx* vs, int j) {
+  if constexpr (GLOBAL) return __ldg(vs + j);
+  else return vs[j];
+}
+
+template <int R, bool DIRECT, class Idx, bool GLOBAL>
 __device__ __forceinline__ double sorted_sum_reg(const double* u,
                                                  const Idx* __restrict__ vs, int d,
                                                  int lane) {
@@ -287,14 +294,14 @@ __device__ __forceinline__ double sorted_sum_reg(const double* u,
 #pragma unroll
   for (int r = 0; r < R; r++) {
     const int j = r * 32 + lane;
-    a[r] = (j < d) ? (DIRECT ? u[j] : u[__ldg(vs + j)]) : pinf;
+    a[r] = (j < d) ? (DIRECT ? u[j] : u[list_at<GLOBAL>(vs, j)]) : pinf;
   }
   return sort_sum_vals<R>(a, d, lane);
 }
 
 // Long lists: repeated selection of the next (value, position) pair in lexicographic
 // order; O(d^2 / 32) loads, no scratch memory.
-template <class Idx>
+template <class Idx, bool GLOBAL>
 __device__ __noinline__ double sorted_sum_select(const double* u,
                                                  const Idx* __restrict__ vs, int d,
                                                  int lane) {
@@ -306,7 +313,7 @@ __device__ __noinline__ double sorted_sum_select(const double* u,
     double bv = inf_val<double>();
     int bi = 0x7fffffff;
     for (int j = lane; j < d; j += 32) {
-      const double x = vs ? u[__ldg(vs + j)] : u[j];
+      const double x = vs ? u[list_at<GLOBAL>(vs, j)] : u[j];
       const bool after = (x > lv) || (x == lv && j > li);
       const bool better = (x < bv) || (x == bv && j < bi);
       if (after && better) {
@@ -410,14 +417,14 @@ __device__ __forceinline__ double seg_sort_sum(double (&a)[RQ], int d, int lane)
   return acc;
 }
 
-template <bool DIRECT = false, class Idx = int32_t>
+template <bool DIRECT = false, class Idx = int32_t, bool GLOBAL = true>
 __device__ __forceinline__ double sorted_sum(const double* u,
                                              const Idx* __restrict__ vs, int d, int lane) {
-  if (d <= 32) return sorted_sum_reg<1, DIRECT, Idx>(u, vs, d, lane);
-  if (d <= 64) return sorted_sum_reg<2, DIRECT, Idx>(u, vs, d, lane);
-  if (d <= 128) return sorted_sum_reg<4, DIRECT, Idx>(u, vs, d, lane);
-  if (d <= 256) return sorted_sum_reg<8, DIRECT, Idx>(u, vs, d, lane);
-  return sorted_sum_select<Idx>(u, DIRECT ? nullptr : vs, d, lane);
+  if (d <= 32) return sorted_sum_reg<1, DIRECT, Idx, GLOBAL>(u, vs, d, lane);
+  if (d <= 64) return sorted_sum_reg<2, DIRECT, Idx, GLOBAL>(u, vs, d, lane);
+  if (d <= 128) return sorted_sum_reg<4, DIRECT, Idx, GLOBAL>(u, vs, d, lane);
+  if (d <= 256) return sorted_sum_reg<8, DIRECT, Idx, GLOBAL>(u, vs, d, lane);
+  return sorted_sum_select<Idx, GLOBAL>(u, DIRECT ? nullptr : vs, d, lane);
 }
 
 // ---- setup, state I/O and the reference function-pair mirrors ---------------------------

@@ -11,6 +11,7 @@
 #include <vector>
 
 #include "../../include/dmm.h"
+#include "dmm_cluster.h"
 #include "dmm_device.cuh"
 
 namespace dmm {
@@ -191,6 +192,13 @@ class Pack {
   dmm_status capture(int32_t steps);
   dmm_status launch_persist(int32_t nsteps);
   dmm_status launch_inst(int32_t nsteps);
+  dmm_status launch_cluster(int32_t nsteps);
+  // cluster form: which of the formulas `cand` it runs, and its launches
+  dmm_status plan_clusters(const std::vector<int32_t>& cand, std::vector<int32_t>* taken);
+  struct ClusterLaunch;
+  dmm_status cluster_config(const ClusterLaunch& L, cudaLaunchConfig_t* cfg,
+                            cudaLaunchAttribute* at);
+  struct TileForms;
   dmm_status prepare_xpose(int32_t idx, int TC, int TV, bool mt, bool* ok);
   // several-tiles-per-block staged form for a formula too large for one tile per block:
   // retiles formula idx and builds the tables for the first tiling that fits
@@ -296,6 +304,25 @@ class Pack {
                                // [3] formula queue of the one-block-per-formula kernel
   int32_t* order_d_ = nullptr; // formulas run one block each, largest first
   int32_t n_small_ = 0;
+  // cluster form: launches over formulas order_d_[first, first + count), one cluster each
+  struct ClusterLaunch {
+    int32_t first = 0, count = 0, R = 1, smem = 0;
+    bool general = false;
+    ClusterCaps caps{};
+  };
+  std::vector<ClusterLaunch> clusters_;
+  // every runnable formula is in a cluster launch
+  bool cluster_only() const {
+    return !clusters_.empty() && ctiles_h_.empty() && vtiles_h_.empty() && n_small_ == 0;
+  }
+  bool no_cluster_ = false;  // tile forms only (phase timing and barrier hooks)
+  std::vector<std::pair<cudaStream_t, cudaEvent_t>> side_;  // forked launches
+  // largest bucket and slot count of a block for each cluster size, per formula
+  struct ClusterNeed {
+    uint64_t serial = 0;
+    int32_t bk[kClusterSizes] = {}, ts[kClusterSizes] = {};
+  };
+  std::vector<ClusterNeed> cl_need_;
   int grid_p_ = 148;           // blocks of the cooperative step kernel
 
   // host mirrors

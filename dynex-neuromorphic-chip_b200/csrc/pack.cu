@@ -9,6 +9,7 @@
 #include <thread>
 #include <vector>
 
+#include "dmm_cluster.h"
 #include "dmm_inst.cuh"
 #include "dmm_step.cuh"
 #include "dmm_xprep.cuh"
@@ -228,6 +229,7 @@ constexpr int kXpSmemMax = 220 * 1024;  // dynamic shared memory of the staged f
 // shared-memory carve-out, and the L1 left to the gathers shrinks (measured at 0.4-1.5 million
 // variables: every tiling above the cap ran 8-30 % slower than the best one below it)
 constexpr int kXpSmemMaxMT = 193 * 1024;  // with the form's ~1.4 KB of static shared memory
+constexpr int kClusterChunk = 8;        // launches of steps_per_graph steps run() makes one of
 constexpr int kXpMaxTiles = 1 << 14;    // clause or variable tiles of the staged form, at most
 constexpr int kMiscInts = 48;            // misc_d_: 192 bytes
 constexpr int kMiscLaunch = 16;          // misc_d_ index of the per-launch area (byte 64)
@@ -264,6 +266,11 @@ Pack::~Pack() {
     if (p) dev_free(p);
   for (auto& e : ev_)
     if (e) cudaEventDestroy(e);
+  for (auto& x : side_) {
+    if (x.first) cudaStreamSynchronize(x.first);
+    if (x.first) cudaStreamDestroy(x.first);
+    if (x.second) cudaEventDestroy(x.second);
+  }
   if (pinned_) pinned_free(pinned_);
   if (stream_) cudaStreamDestroy(stream_);
 }
@@ -338,6 +345,7 @@ dmm_status Pack::init(const PackCaps& caps_in, bool with_alpha_cm, bool fixed_gr
   inst_h_.assign(I, InstDesc{});
   live_.assign(I, 0);
   add_serial_.assign(I, 0);
+  cl_need_.assign(I, ClusterNeed{});
   tun_ = dmm_tuning{};
   DMM_TRY(set_tuning(&tun_));
   DMM_CUDA(cudaStreamSynchronize(stream_));
@@ -389,7 +397,8 @@ dmm_status Pack::set_tuning(const dmm_tuning* t) {
   }
   tun_ = n;
   graph_stale_ = true;
-  if (!ctiles_h_.empty() || !vtiles_h_.empty()) return commit_tiles();
+  if (!ctiles_h_.empty() || !vtiles_h_.empty() || n_small_ > 0 || !clusters_.empty())
+    return commit_tiles();
   return DMM_OK;
 }
 
@@ -1244,7 +1253,7 @@ dmm_status Pack::commit_tiles() {
   std::vector<int32_t> live_list;
   // formulas that one block integrates alone (FP32, V and dV fit in shared memory): used
   // when there are enough of them to fill the GPU (auto) or when forced (launch_mode 3)
-  std::vector<int32_t> small_list;
+  std::vector<int32_t> small_list, cluster_list;
   {
     std::vector<int32_t> eligible, others;
     for (int32_t i = 0; i < (int32_t)live_.size(); i++) {
@@ -1260,10 +1269,23 @@ dmm_status Pack::commit_tiles() {
       others.insert(others.end(), eligible.begin(), eligible.end());
       std::sort(others.begin(), others.end());
     }
+    // the cluster form takes the formulas that fit it, when the launch shape is left open
+    clusters_.clear();
+    if (!no_cluster_ && tun_.launch_mode == 0 && tun_.u_layout == 0 && tun_.clause_tile == 0 &&
+        tun_.var_tile == 0) {
+      DMM_TRY(plan_clusters(others, &cluster_list));
+      std::vector<int32_t> rest;
+      for (int32_t i : others)
+        if (std::find(cluster_list.begin(), cluster_list.end(), i) == cluster_list.end())
+          rest.push_back(i);
+      others = rest;
+    }
     live_list = others;
     std::stable_sort(small_list.begin(), small_list.end(),
                      [&](int32_t a, int32_t b) { return inst_h_[a].m > inst_h_[b].m; });
   }
+  n_small_ = (int32_t)small_list.size();
+  small_list.insert(small_list.end(), cluster_list.begin(), cluster_list.end());
   for (int32_t i : small_list) {
     inst_h_[i].ctile0 = inst_h_[i].nctile = inst_h_[i].vtile0 = inst_h_[i].nvtile = 0;
     DMM_TRY(upload_desc(i));
@@ -1271,7 +1293,7 @@ dmm_status Pack::commit_tiles() {
   if (!small_list.empty())
     DMM_CUDA(cudaMemcpyAsync(order_d_, small_list.data(), small_list.size() * sizeof(int32_t),
                              cudaMemcpyHostToDevice, stream_));
-  n_small_ = (int32_t)small_list.size();
+  for (auto& c : clusters_) c.first += n_small_;
   // grids
   int bc, bv;
   if (prec_ == DMM_FP64) {
@@ -1387,6 +1409,169 @@ dmm_status Pack::launch_persist(int32_t nsteps) {
   return DMM_OK;
 }
 
+dmm_status Pack::plan_clusters(const std::vector<int32_t>& cand, std::vector<int32_t>* taken) {
+  taken->clear();
+  const bool fp64 = prec_ == DMM_FP64;
+  const int ts = (int)tsize_;
+  std::vector<int32_t> list, fresh;
+  for (int32_t i : cand) {
+    const InstDesc& I = inst_h_[i];
+    if (I.n > kClusterMaxVars || 2 * (int64_t)ts * I.n > kClusterSmemMax ||
+        3 * (int64_t)ts * I.m / kClusterMax > kClusterSmemMax)
+      continue;
+    list.push_back(i);
+    if (cl_need_[i].serial != add_serial_[i]) fresh.push_back(i);
+  }
+  if (list.empty()) return DMM_OK;
+  if (!fresh.empty()) {
+    const int64_t need = 2 * kClusterSizes * (int64_t)fresh.size();
+    DMM_TRY(ensure_stage(need));
+    DMM_CUDA(cudaMemcpyAsync(order_d_, fresh.data(), fresh.size() * sizeof(int32_t),
+                             cudaMemcpyHostToDevice, stream_));
+    DMM_CUDA(cluster_need(inst_d_, order_d_, (int)fresh.size(), vend_, coff_,
+                          reinterpret_cast<int2*>(stage_), stream_));
+    std::vector<int2> h(fresh.size() * kClusterSizes);
+    DMM_CUDA(cudaMemcpyAsync(h.data(), stage_, h.size() * sizeof(int2), cudaMemcpyDeviceToHost,
+                             stream_));
+    DMM_CUDA(cudaStreamSynchronize(stream_));
+    for (size_t f = 0; f < fresh.size(); f++) {
+      ClusterNeed& q = cl_need_[fresh[f]];
+      q.serial = add_serial_[fresh[f]];
+      for (int r = 0; r < kClusterSizes; r++) {
+        q.bk[r] = h[f * kClusterSizes + r].x;
+        q.ts[r] = h[f * kClusterSizes + r].y;
+      }
+    }
+  }
+  // Cluster size: the SMs shared out evenly over the formulas (one formula: 16 blocks, the
+  // fastest size from n = 500 on and within 6 % of the best below), or the next larger size
+  // that holds the formula.  Formulas of one size and clause kind share a launch.
+  int q0 = kClusterSizes - 1;
+  while (q0 > 0 && ((int64_t)list.size() << q0) > sms_) q0--;
+  std::vector<std::vector<int32_t>> member;
+  for (int32_t i : list) {
+    const InstDesc& I = inst_h_[i];
+    for (int q = q0; q < kClusterSizes; q++) {
+      const bool general = I.k3 == 0;
+      size_t g = 0;
+      while (g < clusters_.size() && (clusters_[g].R != 1 << q || clusters_[g].general != general)) g++;
+      ClusterLaunch L;
+      if (g < clusters_.size()) L = clusters_[g];
+      L.R = 1 << q;
+      L.general = general;
+      L.caps.n = std::max(L.caps.n, I.n);
+      L.caps.tc = std::max(L.caps.tc, cluster_tc(I.m, L.R));
+      L.caps.ts = std::max(L.caps.ts, cl_need_[i].ts[q]);
+      L.caps.tv = std::max(L.caps.tv, cluster_tv(I.n, L.R));
+      L.caps.bk = std::max(L.caps.bk, cl_need_[i].bk[q]);
+      L.smem = cluster_smem(L.caps, fp64, general);
+      if (L.smem > kClusterSmemMax) continue;
+      if (g == clusters_.size()) {
+        ClusterLaunch one = L;  // the device must be able to hold such a cluster
+        one.count = 1;
+        cudaLaunchConfig_t cfg;
+        cudaLaunchAttribute at;
+        DMM_TRY(cluster_config(one, &cfg, &at));
+        int act = 0;
+        if (cudaOccupancyMaxActiveClusters(&act, cluster_kernel(fp64, general), &cfg) !=
+                cudaSuccess || act < 1) {
+          cudaGetLastError();
+          continue;
+        }
+        clusters_.push_back(L);
+        member.emplace_back();
+      }
+      L.count++;
+      clusters_[g] = L;
+      member[g].push_back(i);
+      break;
+    }
+  }
+  // the launches of large clusters first: they take longest
+  std::vector<size_t> by(clusters_.size());
+  for (size_t g = 0; g < by.size(); g++) by[g] = g;
+  std::stable_sort(by.begin(), by.end(),
+                   [&](size_t a, size_t b) { return clusters_[a].R > clusters_[b].R; });
+  std::vector<ClusterLaunch> sorted;
+  for (size_t g : by) {
+    clusters_[g].first = (int32_t)taken->size();
+    sorted.push_back(clusters_[g]);
+    taken->insert(taken->end(), member[g].begin(), member[g].end());
+  }
+  clusters_ = sorted;
+  return DMM_OK;
+}
+
+// Launch parameters of a cluster launch; sets the kernel's attributes (per device, cheap).
+dmm_status Pack::cluster_config(const ClusterLaunch& L, cudaLaunchConfig_t* cfg,
+                                cudaLaunchAttribute* at) {
+  const bool fp64 = prec_ == DMM_FP64;
+  const void* fn = cluster_kernel(fp64, L.general);
+  DMM_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, L.smem));
+  if (L.R > 8) DMM_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+  *cfg = cudaLaunchConfig_t{};
+  *at = cudaLaunchAttribute{};
+  at->id = cudaLaunchAttributeClusterDimension;
+  at->val.clusterDim.x = (unsigned)L.R;
+  at->val.clusterDim.y = at->val.clusterDim.z = 1;
+  cfg->gridDim = dim3((unsigned)(L.count * L.R));
+  cfg->blockDim = dim3((unsigned)cluster_threads(L.caps, fp64));
+  cfg->dynamicSmemBytes = (size_t)L.smem;
+  cfg->stream = stream_;
+  cfg->attrs = at;
+  cfg->numAttrs = 1;
+  return DMM_OK;
+}
+
+dmm_status Pack::launch_cluster(int32_t nsteps) {
+  const bool fp64 = prec_ == DMM_FP64;
+  PackView<float> vf;
+  PackView<double> vd;
+  void* view;
+  if (fp64) {
+    fill_view<double>(&vd);
+    vd.upos = upos_;
+    view = &vd;
+  } else {
+    fill_view<float>(&vf);
+    vf.upos = upos_;
+    view = &vf;
+  }
+  // launches of different cluster sizes run side by side: the first on the pack's stream,
+  // the others on streams forked from it and joined again
+  const size_t G = clusters_.size();
+  if (G > 1) {
+    while (side_.size() + 1 < G) {
+      cudaStream_t s = nullptr;
+      cudaEvent_t e = nullptr;
+      DMM_CUDA(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
+      side_.push_back({s, e});
+      DMM_CUDA(cudaStreamCreateWithFlags(&side_.back().first, cudaStreamNonBlocking));
+    }
+    DMM_CUDA(cudaEventRecord(ev_[3], stream_));
+  }
+  dmm_status st = DMM_OK;
+  for (size_t g = 0; g < G && st == DMM_OK; g++) {
+    const ClusterLaunch& L = clusters_[g];
+    cudaLaunchConfig_t cfg;
+    cudaLaunchAttribute at;
+    DMM_TRY(cluster_config(L, &cfg, &at));
+    const int32_t* order = order_d_ + L.first;
+    ClusterCaps caps = L.caps;
+    void* args[] = {view, &order, &nsteps, &caps};
+    if (g > 0) {
+      cfg.stream = side_[g - 1].first;
+      DMM_CUDA(cudaStreamWaitEvent(cfg.stream, ev_[3], 0));
+    }
+    DMM_CUDA(cudaLaunchKernelExC(&cfg, cluster_kernel(fp64, L.general), args));
+    if (g > 0) {
+      DMM_CUDA(cudaEventRecord(side_[g - 1].second, cfg.stream));
+      DMM_CUDA(cudaStreamWaitEvent(stream_, side_[g - 1].second, 0));
+    }
+  }
+  return st;
+}
+
 template <int G>
 static dmm_status launch_inst_g(const PackView<float>& v, const int32_t* order, int count,
                                 int nsteps, int* queue, int grid, cudaStream_t s) {
@@ -1431,8 +1616,27 @@ dmm_status Pack::check_error() {
   return DMM_OK;
 }
 
+// Commits the tile forms for the scope of a call that times or tests their kernels, when the
+// cluster form runs some of the pack's formulas.
+struct Pack::TileForms {
+  Pack& p;
+  const bool on;
+  dmm_status st = DMM_OK;
+  explicit TileForms(Pack& pack) : p(pack), on(!pack.clusters_.empty()) {
+    if (!on) return;
+    p.no_cluster_ = true;
+    st = p.commit_tiles();
+  }
+  ~TileForms() {
+    p.no_cluster_ = false;
+    if (on) p.commit_tiles();
+  }
+};
+
 dmm_status Pack::test_barrier_timeout() {
   DMM_CUDA(cudaSetDevice(dev_));
+  TileForms tile_forms(*this);
+  DMM_TRY(tile_forms.st);
   if (tun_.launch_mode == 1 || (ctiles_h_.empty() && vtiles_h_.empty())) {
     set_error("the barrier test needs the cooperative launch of tile-path formulas");
     return DMM_ERR_STATE;
@@ -1473,13 +1677,17 @@ dmm_status Pack::capture(int32_t steps) {
 
 dmm_status Pack::launch_steps(int32_t nsteps) {
   DMM_CUDA(cudaSetDevice(dev_));
-  if (ctiles_h_.empty() && vtiles_h_.empty() && n_small_ == 0) return DMM_OK;
+  if (ctiles_h_.empty() && vtiles_h_.empty() && n_small_ == 0 && clusters_.empty()) return DMM_OK;
   const int32_t S = tun_.steps_per_graph;
   if (tun_.launch_mode != 1) {
+    // cluster launches alone take all the steps at once: their steps are a few microseconds,
+    // and a launch's prologue costs about as much as two of them
+    const bool clusters_only = cluster_only();
     while (nsteps > 0) {
-      const int32_t k = std::min(nsteps, S);
+      const int32_t k = clusters_only ? nsteps : std::min(nsteps, S);
       if (!ctiles_h_.empty() || !vtiles_h_.empty()) DMM_TRY(launch_persist(k));
       if (n_small_ > 0) DMM_TRY(launch_inst(k));
+      if (!clusters_.empty()) DMM_TRY(launch_cluster(k));
       nsteps -= k;
     }
     return DMM_OK;
@@ -1556,6 +1764,8 @@ dmm_status Pack::preload_kernels() {
       default: fns.push_back((const void*)k_inst<32>); break;
     }
   }
+  fns.push_back(cluster_kernel(prec_ == DMM_FP64, false));
+  fns.push_back(cluster_kernel(prec_ == DMM_FP64, true));
   for (const void* f : fns) {
     cudaFuncAttributes a;
     DMM_CUDA(cudaFuncGetAttributes(&a, f));
@@ -1566,6 +1776,8 @@ dmm_status Pack::preload_kernels() {
 int Pack::launch_form() const {
   if (tun_.launch_mode == 1) return 1;
   if (ctiles_h_.empty() && vtiles_h_.empty() && n_small_ > 0) return 5;
+  if (ctiles_h_.empty() && vtiles_h_.empty() && !clusters_.empty())
+    return prec_ == DMM_FP32 && !clusters_[0].general ? 4 : 3;
   if (xp_active_) return xp_mt_ ? 6 : 4;
   if (one_active_) return 3;
   return 2;
@@ -1573,6 +1785,8 @@ int Pack::launch_form() const {
 
 dmm_status Pack::trace_phases(int32_t nsteps, double* out) {
   DMM_CUDA(cudaSetDevice(dev_));
+  TileForms tile_forms(*this);
+  DMM_TRY(tile_forms.st);
   if (tun_.launch_mode == 1 || n_small_ > 0 || nsteps <= 0) {
     set_error("phase tracing needs the cooperative launch of tile-path formulas");
     return DMM_ERR_STATE;
@@ -1641,6 +1855,8 @@ dmm_status Pack::trace_phases(int32_t nsteps, double* out) {
 
 dmm_status Pack::profile_steps(int32_t nsteps, int64_t flush_bytes, StepTimes* t) {
   DMM_CUDA(cudaSetDevice(dev_));
+  TileForms tile_forms(*this);
+  DMM_TRY(tile_forms.st);
   if (flush_bytes > flush_cap_) {
     if (flush_) retire(flush_);
     flush_ = nullptr;
@@ -1690,7 +1906,7 @@ dmm_status Pack::run(double wall_s, int64_t* steps_launched, bool* timed_out,
   DMM_CUDA(cudaMemcpyAsync(&tail0, ring_tail_d_, sizeof(int32_t), cudaMemcpyDeviceToHost, stream_));
   DMM_CUDA(cudaStreamSynchronize(stream_));
   if (active <= 0) return DMM_OK;
-  const int32_t S = tun_.steps_per_graph;
+  const int32_t S = tun_.steps_per_graph * (cluster_only() ? kClusterChunk : 1);
   // chunk k: S steps, then copies of the running count and the finished-ring tail
   auto chunk = [&](int slot) -> dmm_status {
     DMM_TRY(launch_steps(S));

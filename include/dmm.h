@@ -103,7 +103,8 @@ typedef struct dmm_tuning {
                                over the grid for one instance, else 4 x block size)          */
   int32_t var_group;        /* lanes per variable in the dV reduction: 1,2,4,8,16,32         */
   int32_t var_tile;         /* variables per variable tile (>= 32; 0: as clause_tile)         */
-  int32_t steps_per_graph;  /* steps per launch: per cooperative launch, or per CUDA graph   */
+  int32_t steps_per_graph;  /* steps per launch: per cooperative launch, or per CUDA graph (a
+                               run of cluster launches alone takes 8 times as many)          */
   int32_t blocks_per_sm;    /* two-kernel form: persistent blocks per SM (0: occupancy)      */
   int32_t launch_mode;      /* 0: automatic (cooperative launches running steps_per_graph
                                steps with grid barriers between phases; one block per small
@@ -250,7 +251,11 @@ dmm_status dmm_instance_assignment(dmm_instance* inst, int8_t* pre, int8_t* post
  *   6  the staged kernel with several clause and variable tiles per block (formulas whose
  *      tiles are too large for one of each per block)
  *   5  one block per formula
- * or a negative dmm_status. */
+ * A small formula (about n <= 4,000 at 8 clauses per variable) with the default tiles, layout
+ * and launch mode is run by one thread-block cluster, its data and exchanges in shared memory
+ * (two cluster barriers per step), and reported as the form it stands in for: 4 for FP32 with
+ * 3-literal clauses, else 3.
+ * A negative dmm_status on error. */
 int32_t dmm_instance_launch_form(const dmm_instance* inst);
 /* No counterpart in the reference.  Test hook for the failure path of the cooperative step
  * kernels: one launch whose first grid barrier waits for one arrival more than the grid has,
