@@ -244,11 +244,12 @@ __device__ __forceinline__ double row_net_sum(const double* u, const uint4* row,
 // the entries before its own (by value, then place), the values go to their ranks in shared
 // memory (buf: 2 kRankMax doubles) and every lane adds them in order.  A few hundred cycles
 // where a 64-entry network over the lanes with its shuffled sum takes some 3,000.
+template <bool GLOBAL = false>  // where the list is
 __device__ __forceinline__ double rank_sum(const double* u, const uint16_t* idx, int d,
                                            double* buf, int lane) {
   const double pinf = inf_val<double>();
-  const double x0 = lane < d ? u[idx[lane]] : pinf;
-  const double x1 = lane + 32 < d ? u[idx[lane + 32]] : pinf;
+  const double x0 = lane < d ? u[list_at<GLOBAL>(idx, lane)] : pinf;
+  const double x1 = lane + 32 < d ? u[list_at<GLOBAL>(idx, lane + 32)] : pinf;
   buf[lane] = x0;
   buf[lane + 32] = x1;
   __syncwarp();

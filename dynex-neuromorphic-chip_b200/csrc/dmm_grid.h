@@ -1,0 +1,90 @@
+// Host interface of the resident grid form (dmm_grid.cuh, dmm_gridprep.cuh, grid.cu).
+#pragma once
+
+#include <cuda_runtime.h>
+
+#include <cstdint>
+
+#include "dmm_device.cuh"
+
+namespace dmm {
+
+constexpr int kGridThreads = 512;    // block size
+constexpr int kGridThreads64 = 512;  // ... in FP64 (the sorted sums' registers)
+constexpr int kGridSmemMax = 222 * 1024;  // dynamic shared memory, at most
+constexpr int kGridMaxTiles = 24;         // clause or variable tiles of a block
+constexpr int kGridMaxDistinct = 32767;   // 16-bit tile-local literals
+
+// One formula of a launch: B blocks of the grid from blk0 on, each with kc clause tiles of TC
+// clauses and kv variable tiles of TV variables.  The o_* are where its part of each shared
+// table array starts (elements).
+struct GridGroup {
+  int32_t inst, blk0, B, kc, kv, TC, TV, TVr;  // TVr: TV rounded up to 32 (table rows)
+  int32_t nct, nvt;                            // B * kc, B * kv
+  int32_t n, m, L, k3;
+  int64_t var0, cls0, slot0;
+  int64_t o_pair, o_blk, o_ct, o_vt, o_list, o_slot, o_ux, o_word, o_row, o_push, o_bb;
+};
+
+// Table arrays of all groups.
+struct GridTables {
+  // built at commit, read by the steps
+  int32_t* dlist;   // [o_list] distinct variables of each block's clauses, ascending
+  int2* dinfo;      // [o_blk + b] start and count in dlist and in the inbox
+  int16_t* llit;    // [o_slot + s] block-local literal, +-(1 + place in the list)
+  uint16_t* spos;   // [o_slot + s] place in the tile's staging area
+  uint32_t* wdst;   // [o_word + w] 16-byte word of ux each staging word goes to
+  int32_t* woff;    // [o_ct + t] first staging word of each clause tile (nct + 1 of them)
+  int32_t* boff;    // [o_vt + v] start of each variable tile's bucket in ux (nvt + 1)
+  uint16_t* rows;   // [o_row] bucket places of each variable's first 32 contributions
+  uint16_t* idx;    // [o_slot + j] bucket place of the contribution in CSR position j
+  int2* pinfo;      // [o_bb + b (B + 1) + c] start in sends and inbox place of block c's chunk
+  uint32_t* sends;  // [o_push] block-local variable, destination block << 16
+  // exchanged within a step, each twice (steps of even and odd number): unset entries hold a
+  // value no arithmetic gives
+  void* ux;         // [2 o_ux] contributions, bucket after bucket
+  void* inbox;      // [2 o_list] dV of each block's distinct variables
+  int64_t ux_len, inbox_len;  // elements of one copy
+  // scratch of the build
+  int32_t *cnt, *sb, *bt;       // [o_pair]
+  int32_t *st, *dcnt, *dlo;     // [o_ct], [o_blk], [o_bb]
+  int32_t* out;                 // [8 x group]
+};
+
+// Results of the build, per group: [0] 0 ok, else which limit failed; [1] largest distinct
+// list, [2] largest staging area, [3] largest bucket, [4] largest send list (entries), [5]
+// largest literal-slot count of a block.
+constexpr int kGridOut = 8;
+
+struct GridCaps {
+  int dl;      // distinct variables of a block (a multiple of 4)
+  int st, bk;  // staging entries, bucket entries
+  int tv;      // variables of a block
+  int B;       // blocks of a group
+  // resident tables: clauses, slots, staging words, table rows, CSR entries, sends of a block
+  int tc, ts, wd, row, csr, snd;
+};
+
+constexpr int kGridSyncBytes = 256;  // per group
+// Byte offsets of a block's dynamic shared memory.
+struct GridLayout {
+  int sv, raw, cur, dv, vend, unit, pinfo, rank;
+  int xs, xl, cp, lit, spos, off, wdst, row, csr, snd, total;
+};
+
+// resident: 0 no tables in shared memory, 1 those of the variable phase, 2 all and the clause
+// memories
+GridLayout grid_shape(const GridCaps& c, bool fp64, bool general, int resident);
+inline int grid_smem(const GridCaps& c, bool fp64, bool general, int resident) {
+  return grid_shape(c, fp64, general, resident).total;
+}
+const void* grid_kernel(bool fp64, bool general, int resident);
+// Queues the marking of all exchange entries as unset.
+cudaError_t grid_unset(const GridTables& t, bool fp64, cudaStream_t s);
+// Queues the table build of all groups (blk_group: group of every block of the grid).
+cudaError_t grid_build(const GridGroup* groups, const int32_t* blk_group, int ngroups,
+                       int nblocks, int max_n, int max_nvt, const int32_t* lit,
+                       const int32_t* upos, const int32_t* vend, const int32_t* coff,
+                       const GridTables& t, bool fp64, cudaStream_t s);
+
+}  // namespace dmm

@@ -13,6 +13,7 @@
 #include "../../include/dmm.h"
 #include "dmm_cluster.h"
 #include "dmm_device.cuh"
+#include "dmm_grid.h"
 
 namespace dmm {
 
@@ -199,6 +200,13 @@ class Pack {
   dmm_status cluster_config(const ClusterLaunch& L, cudaLaunchConfig_t* cfg,
                             cudaLaunchAttribute* at);
   struct TileForms;
+  // resident grid form: splits the SMs over the formulas `cand`, builds their tables; leaves
+  // in *taken those it runs
+  dmm_status plan_grid(const std::vector<int32_t>& cand, std::vector<int32_t>* taken);
+  dmm_status launch_grid(int32_t nsteps);
+  double cluster_step_us() const;
+  double grid_step_us(const std::vector<int32_t>& list) const;
+  dmm_status grid_buffer(int which, int64_t bytes);
   dmm_status prepare_xpose(int32_t idx, int TC, int TV, bool mt, bool* ok);
   // several-tiles-per-block staged form for a formula too large for one tile per block:
   // retiles formula idx and builds the tables for the first tiling that fits
@@ -313,10 +321,26 @@ class Pack {
   std::vector<ClusterLaunch> clusters_;
   // every runnable formula is in a cluster launch
   bool cluster_only() const {
-    return !clusters_.empty() && ctiles_h_.empty() && vtiles_h_.empty() && n_small_ == 0;
+    return !clusters_.empty() && gr_groups_.empty() && ctiles_h_.empty() && vtiles_h_.empty() &&
+           n_small_ == 0;
   }
   bool no_cluster_ = false;  // tile forms only (phase timing and barrier hooks)
   std::vector<std::pair<cudaStream_t, cudaEvent_t>> side_;  // forked launches
+  // resident grid form: groups of the current launch and their tables
+  std::vector<GridGroup> gr_groups_;
+  std::vector<uint64_t> gr_key_;  // what the tables were built for
+  int32_t gr_blocks_ = 0;
+  bool gr_general_ = false;
+  int gr_resident_ = 0;
+  bool gr_clean_ = false;  // group counters zeroed (every launch leaves them so)
+  bool no_grid_ = false;
+  GridLayout gr_layout_{};
+  GridTables gr_tables_{};
+  enum { kGrGroups, kGrBlk, kGrDlist, kGrDinfo, kGrLlit, kGrSpos, kGrWdst, kGrWoff, kGrBoff,
+         kGrRows, kGrIdx, kGrPinfo, kGrSends, kGrUx, kGrInbox, kGrCnt, kGrSb, kGrBt, kGrSt, kGrDcnt,
+         kGrDlo, kGrOut, kGrSync, kGrEpart, kGrBufs };
+  void* gbuf_[kGrBufs] = {};
+  int64_t gbuf_cap_[kGrBufs] = {};
   // largest bucket and slot count of a block for each cluster size, per formula
   struct ClusterNeed {
     uint64_t serial = 0;

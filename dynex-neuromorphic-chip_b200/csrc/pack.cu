@@ -264,6 +264,8 @@ Pack::~Pack() {
     if (p) dev_free(p);
   for (void* p : xbuf_)
     if (p) dev_free(p);
+  for (void* p : gbuf_)
+    if (p) dev_free(p);
   for (auto& e : ev_)
     if (e) cudaEventDestroy(e);
   for (auto& x : side_) {
@@ -397,7 +399,8 @@ dmm_status Pack::set_tuning(const dmm_tuning* t) {
   }
   tun_ = n;
   graph_stale_ = true;
-  if (!ctiles_h_.empty() || !vtiles_h_.empty() || n_small_ > 0 || !clusters_.empty())
+  if (!ctiles_h_.empty() || !vtiles_h_.empty() || n_small_ > 0 || !clusters_.empty() ||
+      !gr_groups_.empty())
     return commit_tiles();
   return DMM_OK;
 }
@@ -1065,6 +1068,305 @@ static const void* staged_fn(int G, bool mt) {
   return mt ? staged_fn_x<true>(G) : staged_fn_x<false>(G);
 }
 
+// Estimated microseconds per step, fitted to single formulas of 500 to 30,000 variables at 4.3
+// and 8 clauses per variable: the cluster form by a block's clauses (FP32 3.1 us at 250 and
+// 4.8 at 1,000; FP64 4.7 and 9.9), in waves when the clusters do not all fit at once; the
+// resident grid form by a block's share of the clauses (FP32 5.1 us at 54, 9.8 at 1,600; FP64
+// 7.5 and 15.9).  The two meet at about 18,000 clauses (FP32) and 13,000 (FP64) for one formula.
+double Pack::cluster_step_us() const {
+  int64_t blocks = 0;
+  int tc = 0;
+  for (const ClusterLaunch& L : clusters_) {
+    blocks += (int64_t)L.R * L.count;
+    tc = std::max(tc, L.caps.tc);
+  }
+  const double waves = (double)((blocks + sms_ - 1) / sms_);
+  return waves * (prec_ == DMM_FP64 ? 3.6 + 5.0e-3 * tc : 2.6 + 2.2e-3 * tc);
+}
+
+double Pack::grid_step_us(const std::vector<int32_t>& list) const {
+  if ((int)list.size() > sms_) return 1e9;
+  double total = 0, most = 0;
+  for (int32_t i : list) {
+    total += inst_h_[i].m;
+    most = std::max(most, (double)inst_h_[i].m);
+  }
+  const double share = std::max(total / sms_, most / (sms_ - (double)list.size() + 1));
+  return prec_ == DMM_FP64 ? 7.0 + 5.2e-3 * share : 4.9 + 3.2e-3 * share;
+}
+
+dmm_status Pack::grid_buffer(int which, int64_t bytes) {
+  bytes = std::max<int64_t>(bytes, 16);
+  if (bytes <= gbuf_cap_[which]) return DMM_OK;
+  if (gbuf_[which]) retire(gbuf_[which]);
+  gbuf_[which] = nullptr;
+  gbuf_cap_[which] = 0;
+  DMM_CUDA(dev_alloc(&gbuf_[which], bytes));
+  gbuf_cap_[which] = bytes;
+  return DMM_OK;
+}
+
+dmm_status Pack::plan_grid(const std::vector<int32_t>& cand, std::vector<int32_t>* taken) {
+  taken->clear();
+  gr_groups_.clear();
+  const bool fp64 = prec_ == DMM_FP64;
+  const int T = (int)tsize_, kw = 16 / T;
+  std::vector<int32_t> list;
+  for (int32_t i : cand)
+    if (inst_h_[i].m > 0 && inst_h_[i].nslots > 0) list.push_back(i);
+  // rounds: the tilings are estimates, corrected by what a build reports
+  std::vector<int> kc_min(live_.size(), 1), kv_min(live_.size(), 1);
+  for (int round = 0; round < 4; round++) {
+    if (list.empty() || (int)list.size() > sms_) return DMM_OK;
+    // the SMs shared out by literal count, at least one block each
+    double total = 0;
+    for (int32_t i : list) total += inst_h_[i].nslots;
+    std::vector<int> B(list.size());
+    int used = 0;
+    for (size_t k = 0; k < list.size(); k++) {
+      B[k] = std::max(1, (int)(inst_h_[list[k]].nslots / total * sms_));
+      used += B[k];
+    }
+    while (used != sms_) {  // take from, or give to, the formula with least / most per block
+      size_t at = 0;
+      for (size_t k = 1; k < list.size(); k++) {
+        const double a = inst_h_[list[k]].nslots / (double)B[k],
+                     c = inst_h_[list[at]].nslots / (double)B[at];
+        if (used > sms_ ? (B[at] == 1 || (B[k] > 1 && a < c)) : a > c) at = k;
+      }
+      if (used > sms_ && B[at] == 1) return DMM_OK;
+      B[at] += used > sms_ ? -1 : 1;
+      used += used > sms_ ? -1 : 1;
+    }
+    std::vector<GridGroup> groups;
+    std::vector<int32_t> blk, next;
+    int64_t pair = 0, blks = 0, ct = 0, vt = 0, lst = 0, slot = 0, ux = 0, word = 0, row = 0,
+            push = 0, bb = 0;
+    bool general = false;
+    int max_n = 0, max_nvt = 0;
+    for (size_t k = 0; k < list.size(); k++) {
+      const InstDesc& I = inst_h_[list[k]];
+      GridGroup g{};
+      g.inst = list[k];
+      g.blk0 = (int32_t)blk.size();
+      g.B = B[k];
+      g.n = I.n;
+      g.m = I.m;
+      g.L = I.nslots;
+      g.k3 = I.k3;
+      g.var0 = I.var0;
+      g.cls0 = I.cls0;
+      g.slot0 = I.slot0;
+      // fewest tiles per block whose areas fit beside the block's voltages
+      const double n = I.n, L = I.nslots;
+      const double distinct = n * (1.0 - std::exp(-L / (B[k] * n))) * 1.02 + 16;
+      bool fits = false;
+      for (int sum = 2; sum <= kGridMaxTiles && !fits; sum++)
+        for (int kc = (sum + 1) / 2; kc < sum && !fits; kc++) {
+          const int kv = sum - kc;
+          if (kc < kc_min[list[k]] || kv < kv_min[list[k]] || kv > kc) continue;
+          const double stage = L / (B[k] * kc) * 1.02 + 0.5 * kw * B[k] * kv + 64;
+          const double bucket = L / (B[k] * kv) * 1.06 + 0.5 * kw * B[k] * kc + 64;
+          const double tvb = n / B[k] + 8 * kv;
+          const double smem = T * distinct + T * std::max(stage, bucket) + tvb * (2 * T + 5) +
+                              8 * B[k] + (fp64 ? 16384 : 0) + 2048;
+          if (distinct > kGridMaxDistinct || stage > 65000 || bucket > 65000 ||
+              smem > kGridSmemMax || B[k] * kv > 1024 || B[k] * kc > 1024)
+            continue;
+          g.kc = kc;
+          g.kv = kv;
+          fits = true;
+        }
+      // one large formula: the staged and tile forms are faster once a block's share is large
+      // (n at 8 clauses per variable, us per step against them: FP32 50,000 12.5 / 13.4, 70,000
+      // 16.9 / 15.5; FP64 70,000 31.6 / 32.5, 100,000, with two tiles per block, 58 / 44)
+      if (list.size() == 1 && ((!fp64 && I.k3 && L / B[k] > 9000) || (fp64 && g.kc + g.kv > 2)))
+        fits = false;
+      if (!fits) continue;
+      g.TC = ((I.m + g.B * g.kc - 1) / (g.B * g.kc) + 3) & ~3;
+      g.TV = ((I.n + g.B * g.kv - 1) / (g.B * g.kv) + 3) & ~3;
+      g.TVr = (g.TV + 31) & ~31;
+      g.nct = g.B * g.kc;
+      g.nvt = g.B * g.kv;
+      g.o_pair = pair;
+      g.o_blk = blks;
+      g.o_ct = ct;
+      g.o_vt = vt;
+      g.o_list = lst;
+      g.o_slot = slot;
+      g.o_ux = ux;
+      g.o_word = word;
+      g.o_row = row;
+      g.o_push = push;
+      g.o_bb = bb;
+      const int64_t pairs = (int64_t)g.nct * g.nvt, Ls = RangeAlloc::round(I.nslots);
+      const int64_t uxn = RangeAlloc::round(I.nslots + (kw - 1) * pairs + 32);
+      pair += pairs;
+      blks += g.B + 1;
+      ct += g.nct + 1;
+      vt += g.nvt + 1;
+      lst += RangeAlloc::round(I.nslots + 4 * g.B);
+      slot += Ls;
+      ux += uxn;
+      word += uxn / kw;
+      row += (int64_t)g.nvt * g.TVr * 32;
+      push += Ls;
+      bb += (int64_t)g.B * (g.B + 1);
+      general |= I.k3 == 0;
+      max_n = std::max(max_n, I.n);
+      max_nvt = std::max(max_nvt, g.nvt);
+      for (int b = 0; b < g.B; b++) blk.push_back((int32_t)groups.size());
+      groups.push_back(g);
+      next.push_back(list[k]);
+    }
+    if (next.size() != list.size()) {  // share the SMs among those that fit
+      list = next;
+      continue;
+    }
+    if (ux > INT32_MAX / 2 || row > INT32_MAX / 2) return DMM_OK;
+    // (the tables of the same formulas in the same tiles are still valid: only this function
+    // writes them, and a live formula's device arrays do not change)
+    std::vector<uint64_t> key;
+    for (const GridGroup& g : groups) {
+      key.push_back(add_serial_[g.inst]);
+      key.push_back(((uint64_t)g.B << 40) | ((uint64_t)g.kc << 20) | (uint64_t)g.kv);
+    }
+    if (key == gr_key_) {
+      gr_groups_ = groups;
+      *taken = list;
+      return DMM_OK;
+    }
+    gr_key_.clear();
+    const int64_t bytes[kGrBufs] = {
+        (int64_t)(groups.size() * sizeof(GridGroup)), (int64_t)blk.size() * 4, lst * 4, blks * 8,
+        slot * 2, slot * 2, word * 4, ct * 4, vt * 4, row * 2, slot * 2, bb * 8, push * 4,
+        2 * ux * T, 2 * lst * T, pair * 4, pair * 4, pair * 4, ct * 4, blks * 4, bb * 4,
+        (int64_t)groups.size() * kGridOut * 4, (int64_t)groups.size() * kGridSyncBytes,
+        (int64_t)blk.size() * 8};
+    for (int q = 0; q < kGrBufs; q++) DMM_TRY(grid_buffer(q, bytes[q]));
+    GridTables t{};
+    t.dlist = static_cast<int32_t*>(gbuf_[kGrDlist]);
+    t.dinfo = static_cast<int2*>(gbuf_[kGrDinfo]);
+    t.llit = static_cast<int16_t*>(gbuf_[kGrLlit]);
+    t.spos = static_cast<uint16_t*>(gbuf_[kGrSpos]);
+    t.wdst = static_cast<uint32_t*>(gbuf_[kGrWdst]);
+    t.woff = static_cast<int32_t*>(gbuf_[kGrWoff]);
+    t.boff = static_cast<int32_t*>(gbuf_[kGrBoff]);
+    t.rows = static_cast<uint16_t*>(gbuf_[kGrRows]);
+    t.idx = static_cast<uint16_t*>(gbuf_[kGrIdx]);
+    t.pinfo = static_cast<int2*>(gbuf_[kGrPinfo]);
+    t.sends = static_cast<uint32_t*>(gbuf_[kGrSends]);
+    t.ux_len = ux;
+    t.inbox_len = lst;
+    t.ux = gbuf_[kGrUx];
+    t.inbox = gbuf_[kGrInbox];
+    t.cnt = static_cast<int32_t*>(gbuf_[kGrCnt]);
+    t.sb = static_cast<int32_t*>(gbuf_[kGrSb]);
+    t.bt = static_cast<int32_t*>(gbuf_[kGrBt]);
+    t.st = static_cast<int32_t*>(gbuf_[kGrSt]);
+    t.dcnt = static_cast<int32_t*>(gbuf_[kGrDcnt]);
+    t.dlo = static_cast<int32_t*>(gbuf_[kGrDlo]);
+    t.out = static_cast<int32_t*>(gbuf_[kGrOut]);
+    DMM_CUDA(cudaMemcpyAsync(gbuf_[kGrGroups], groups.data(), bytes[kGrGroups],
+                             cudaMemcpyHostToDevice, stream_));
+    DMM_CUDA(cudaMemcpyAsync(gbuf_[kGrBlk], blk.data(), bytes[kGrBlk], cudaMemcpyHostToDevice,
+                             stream_));
+    DMM_CUDA(cudaMemsetAsync(t.rows, 0, (size_t)bytes[kGrRows], stream_));
+    DMM_CUDA(grid_build(static_cast<const GridGroup*>(gbuf_[kGrGroups]),
+                        static_cast<const int32_t*>(gbuf_[kGrBlk]), (int)groups.size(),
+                        (int)blk.size(), max_n, max_nvt, lit_, upos_, vend_, coff_, t, fp64,
+                        stream_));
+    std::vector<int32_t> out(groups.size() * kGridOut);
+    DMM_CUDA(cudaMemcpyAsync(out.data(), t.out, bytes[kGrOut], cudaMemcpyDeviceToHost, stream_));
+    DMM_CUDA(cudaStreamSynchronize(stream_));
+    // what the tables need; a formula whose tiles came out too large gets more of them
+    GridCaps caps{};
+    bool again = false;
+    for (size_t k = 0; k < groups.size(); k++) {
+      const int32_t* o = &out[k * kGridOut];
+      const GridGroup& g = groups[k];
+      if (o[0] == 1) {
+        list.erase(list.begin() + (long)k);
+        again = true;
+        break;
+      }
+      GridCaps one{o[1], o[2], o[3], g.TV * g.kv, g.B, g.TC * g.kc, o[5], o[6],
+                   g.kv * g.TVr * 32, o[7], o[4]};
+      if (o[0] == 2 || o[0] == 3 || grid_smem(one, fp64, g.k3 == 0, 0) > kGridSmemMax) {
+        if (o[0] == 2 || (o[0] == 0 && one.st > one.bk)) kc_min[g.inst] = g.kc + 1;
+        else kv_min[g.inst] = g.kv + 1, kc_min[g.inst] = std::max(g.kc, g.kv + 1);
+        again = true;
+      }
+      caps.dl = std::max(caps.dl, one.dl);
+      caps.st = std::max(caps.st, one.st);
+      caps.bk = std::max(caps.bk, one.bk);
+      caps.tv = std::max(caps.tv, one.tv);
+      caps.B = std::max(caps.B, one.B);
+      caps.tc = std::max(caps.tc, one.tc);
+      caps.ts = std::max(caps.ts, one.ts);
+      caps.wd = std::max(caps.wd, one.wd);
+      caps.row = std::max(caps.row, one.row);
+      caps.csr = std::max(caps.csr, one.csr);
+      caps.snd = std::max(caps.snd, one.snd);
+    }
+    if (again) continue;
+    if (grid_smem(caps, fp64, general, 0) > kGridSmemMax) {
+      // formulas whose maxima do not fit together: the one with the largest areas goes elsewhere
+      size_t at = 0;
+      for (size_t k = 1; k < groups.size(); k++)
+        if (inst_h_[groups[k].inst].nslots > inst_h_[groups[at].inst].nslots) at = k;
+      list.erase(list.begin() + (long)at);
+      continue;
+    }
+    gr_resident_ = 2;
+    while (gr_resident_ > 0 && grid_smem(caps, fp64, general, gr_resident_) > kGridSmemMax)
+      gr_resident_--;
+    gr_layout_ = grid_shape(caps, fp64, general, gr_resident_);
+    const void* fn = grid_kernel(fp64, general, gr_resident_);
+    if (occupancy_blocks(fn, fp64 ? kGridThreads64 : kGridThreads, gr_layout_.total) < 1) return DMM_OK;
+    gr_general_ = general;
+    gr_tables_ = t;
+    gr_blocks_ = (int32_t)blk.size();
+    gr_key_ = key;
+    gr_clean_ = false;
+    gr_groups_ = groups;
+    *taken = list;
+    return DMM_OK;
+  }
+  return DMM_OK;
+}
+
+dmm_status Pack::launch_grid(int32_t nsteps) {
+  const bool fp64 = prec_ == DMM_FP64;
+  PackView<float> vf;
+  PackView<double> vd;
+  void* view;
+  if (fp64) {
+    fill_view<double>(&vd);
+    view = &vd;
+  } else {
+    fill_view<float>(&vf);
+    view = &vf;
+  }
+  void* sync = gbuf_[kGrSync];
+  if (!gr_clean_) {
+    DMM_CUDA(cudaMemsetAsync(sync, 0, gr_groups_.size() * kGridSyncBytes, stream_));
+    DMM_CUDA(grid_unset(gr_tables_, fp64, stream_));
+  }
+  gr_clean_ = true;
+  const void* fn = grid_kernel(fp64, gr_general_, gr_resident_);
+  DMM_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, gr_layout_.total));
+  const void* groups = gbuf_[kGrGroups];
+  const void* blk = gbuf_[kGrBlk];
+  void* epart = gbuf_[kGrEpart];
+  int* err = misc_d_ + 1;
+  void* args[] = {view, &gr_tables_, &groups, &blk, &gr_layout_, &nsteps, &sync, &epart, &err};
+  DMM_CUDA(cudaLaunchCooperativeKernel(fn, dim3((unsigned)gr_blocks_),
+                                       dim3(fp64 ? kGridThreads64 : kGridThreads), args,
+                                       (size_t)gr_layout_.total, stream_));
+  return DMM_OK;
+}
+
 const void* Pack::persist_fn() const {
   if (xp_active_) return staged_fn(tun_.var_group, xp_mt_);
   if (one_active_) return persist_fn_x<true>(prec_, tun_.var_group);
@@ -1269,17 +1571,32 @@ dmm_status Pack::commit_tiles() {
       others.insert(others.end(), eligible.begin(), eligible.end());
       std::sort(others.begin(), others.end());
     }
-    // the cluster form takes the formulas that fit it, when the launch shape is left open
+    // with the launch shape left open, the cluster form takes the formulas that fit it and the
+    // resident grid form the others, or the latter takes all of them when the estimated step
+    // is shorter (the server's formulas change between launches: no tables are built for them)
     clusters_.clear();
-    if (!no_cluster_ && tun_.launch_mode == 0 && tun_.u_layout == 0 && tun_.clause_tile == 0 &&
-        tun_.var_tile == 0) {
-      DMM_TRY(plan_clusters(others, &cluster_list));
+    gr_groups_.clear();
+    const bool open_shape = tun_.launch_mode == 0 && tun_.u_layout == 0 && tun_.clause_tile == 0 &&
+                            tun_.var_tile == 0;
+    auto without = [](const std::vector<int32_t>& all, const std::vector<int32_t>& some) {
       std::vector<int32_t> rest;
-      for (int32_t i : others)
-        if (std::find(cluster_list.begin(), cluster_list.end(), i) == cluster_list.end())
-          rest.push_back(i);
-      others = rest;
+      for (int32_t i : all)
+        if (std::find(some.begin(), some.end(), i) == some.end()) rest.push_back(i);
+      return rest;
+    };
+    if (open_shape && !no_cluster_) DMM_TRY(plan_clusters(others, &cluster_list));
+    if (open_shape && !no_grid_ && !fixed_grid_) {
+      const std::vector<int32_t> rest = without(others, cluster_list);
+      if (!cluster_list.empty() &&
+          grid_step_us(others) < cluster_step_us() + (rest.empty() ? 0.0 : grid_step_us(rest))) {
+        clusters_.clear();
+        cluster_list.clear();
+      }
+      std::vector<int32_t> grid_list;
+      DMM_TRY(plan_grid(without(others, cluster_list), &grid_list));
+      cluster_list.insert(cluster_list.end(), grid_list.begin(), grid_list.end());
     }
+    others = without(others, cluster_list);
     live_list = others;
     std::stable_sort(small_list.begin(), small_list.end(),
                      [&](int32_t a, int32_t b) { return inst_h_[a].m > inst_h_[b].m; });
@@ -1608,6 +1925,7 @@ dmm_status Pack::check_error() {
   DMM_CUDA(cudaStreamSynchronize(stream_));
   if (e) {
     launch_area_clean_ = false;
+    gr_clean_ = false;
     DMM_CUDA(cudaMemsetAsync(misc_d_ + 1, 0, sizeof(int32_t), stream_));  // reported once
     DMM_CUDA(cudaStreamSynchronize(stream_));
     set_error("grid barrier wait gave up in the cooperative step kernel");
@@ -1616,33 +1934,35 @@ dmm_status Pack::check_error() {
   return DMM_OK;
 }
 
-// Commits the tile forms for the scope of a call that times or tests their kernels, when the
-// cluster form runs some of the pack's formulas.
+// Commits the grid-wide forms for the scope of a call that traces or tests their barriers, or
+// (tiles) the forms over the tile tables, when other forms run some of the pack's formulas.
 struct Pack::TileForms {
   Pack& p;
   const bool on;
   dmm_status st = DMM_OK;
-  explicit TileForms(Pack& pack) : p(pack), on(!pack.clusters_.empty()) {
+  TileForms(Pack& pack, bool tiles)
+      : p(pack), on(!pack.clusters_.empty() || (tiles && !pack.gr_groups_.empty())) {
     if (!on) return;
     p.no_cluster_ = true;
+    p.no_grid_ = tiles;
     st = p.commit_tiles();
   }
   ~TileForms() {
-    p.no_cluster_ = false;
+    p.no_cluster_ = p.no_grid_ = false;
     if (on) p.commit_tiles();
   }
 };
 
 dmm_status Pack::test_barrier_timeout() {
   DMM_CUDA(cudaSetDevice(dev_));
-  TileForms tile_forms(*this);
+  TileForms tile_forms(*this, false);
   DMM_TRY(tile_forms.st);
-  if (tun_.launch_mode == 1 || (ctiles_h_.empty() && vtiles_h_.empty())) {
+  if (tun_.launch_mode == 1 || (ctiles_h_.empty() && vtiles_h_.empty() && gr_groups_.empty())) {
     set_error("the barrier test needs the cooperative launch of tile-path formulas");
     return DMM_ERR_STATE;
   }
   barrier_extra_ = 1;
-  const dmm_status st = launch_persist(1);
+  const dmm_status st = gr_groups_.empty() ? launch_persist(1) : launch_grid(1);
   barrier_extra_ = 0;
   DMM_TRY(st);
   DMM_CUDA(cudaStreamSynchronize(stream_));
@@ -1677,7 +1997,9 @@ dmm_status Pack::capture(int32_t steps) {
 
 dmm_status Pack::launch_steps(int32_t nsteps) {
   DMM_CUDA(cudaSetDevice(dev_));
-  if (ctiles_h_.empty() && vtiles_h_.empty() && n_small_ == 0 && clusters_.empty()) return DMM_OK;
+  if (ctiles_h_.empty() && vtiles_h_.empty() && n_small_ == 0 && clusters_.empty() &&
+      gr_groups_.empty())
+    return DMM_OK;
   const int32_t S = tun_.steps_per_graph;
   if (tun_.launch_mode != 1) {
     // cluster launches alone take all the steps at once: their steps are a few microseconds,
@@ -1687,6 +2009,7 @@ dmm_status Pack::launch_steps(int32_t nsteps) {
       const int32_t k = clusters_only ? nsteps : std::min(nsteps, S);
       if (!ctiles_h_.empty() || !vtiles_h_.empty()) DMM_TRY(launch_persist(k));
       if (n_small_ > 0) DMM_TRY(launch_inst(k));
+      if (!gr_groups_.empty()) DMM_TRY(launch_grid(k));
       if (!clusters_.empty()) DMM_TRY(launch_cluster(k));
       nsteps -= k;
     }
@@ -1778,6 +2101,8 @@ int Pack::launch_form() const {
   if (ctiles_h_.empty() && vtiles_h_.empty() && n_small_ > 0) return 5;
   if (ctiles_h_.empty() && vtiles_h_.empty() && !clusters_.empty())
     return prec_ == DMM_FP32 && !clusters_[0].general ? 4 : 3;
+  if (ctiles_h_.empty() && vtiles_h_.empty() && gr_groups_.size() == 1)
+    return prec_ == DMM_FP32 && !gr_general_ ? 4 : 3;
   if (xp_active_) return xp_mt_ ? 6 : 4;
   if (one_active_) return 3;
   return 2;
@@ -1785,15 +2110,18 @@ int Pack::launch_form() const {
 
 dmm_status Pack::trace_phases(int32_t nsteps, double* out) {
   DMM_CUDA(cudaSetDevice(dev_));
-  TileForms tile_forms(*this);
+  TileForms tile_forms(*this, false);
   DMM_TRY(tile_forms.st);
   if (tun_.launch_mode == 1 || n_small_ > 0 || nsteps <= 0) {
     set_error("phase tracing needs the cooperative launch of tile-path formulas");
     return DMM_ERR_STATE;
   }
   constexpr int K = kTraceK;
-  const int64_t half = (int64_t)nsteps * K * grid_p_;
-  const int64_t need = 2 * half;  // timer stamps, then clock counts
+  const bool grid = !gr_groups_.empty();
+  const int G = grid ? gr_blocks_ : grid_p_;
+  const int64_t half = (int64_t)nsteps * K * G;
+  // timer stamps, clock counts, then every block's entry and exit times (trace_launch)
+  const int64_t need = 2 * half + 2 * G;
   if (need > trace_cap_) {
     if (trace_) retire(trace_);
     trace_ = nullptr;
@@ -1803,14 +2131,13 @@ dmm_status Pack::trace_phases(int32_t nsteps, double* out) {
   DMM_CUDA(cudaMemsetAsync(trace_, 0, need * sizeof(long long), stream_));
   trace_on_ = true;
   trace_steps_ = nsteps;
-  dmm_status st = launch_persist(nsteps);  // one launch: trace step s = launch step s
+  dmm_status st = grid ? launch_grid(nsteps) : launch_persist(nsteps);  // one launch: trace step s = launch step s
   trace_on_ = false;
   DMM_TRY(st);
   std::vector<long long> h(need);
   DMM_CUDA(cudaMemcpyAsync(h.data(), trace_, need * sizeof(long long), cudaMemcpyDeviceToHost, stream_));
   DMM_CUDA(cudaStreamSynchronize(stream_));
   DMM_TRY(check_error());
-  const int G = grid_p_;
   auto at = [&](int64_t s, int k, int b) { return h[(s * K + k) * G + b]; };
   double mean[K] = {}, mx[K] = {};
   int used = 0;
@@ -1850,12 +2177,22 @@ dmm_status Pack::trace_phases(int32_t nsteps, double* out) {
     const long long c0 = h[half + 0], c1 = h[half + (int64_t)used * K * G];
     if (t1 > t0) out[2 * K] = (double)(c1 - c0) / (double)(t1 - t0) * 1000.0;  // MHz
   }
+  // launch entry to the first step, last step's end to exit (forms that stamp them)
+  out[2 * K + 1] = out[2 * K + 2] = 0.0;
+  for (int b = 0; b < G; b++) {
+    const long long in = h[2 * half + b], ex = h[2 * half + G + b];
+    if (in == 0 || ex == 0 || at(0, 0, b) == 0) continue;
+    int32_t last = nsteps - 1;
+    while (last > 0 && at(last, K - 1, b) == 0) last--;
+    out[2 * K + 1] += (double)(at(0, 0, b) - in) / G / 1000.0;
+    if (at(last, K - 1, b) != 0) out[2 * K + 2] += (double)(ex - at(last, K - 1, b)) / G / 1000.0;
+  }
   return DMM_OK;
 }
 
 dmm_status Pack::profile_steps(int32_t nsteps, int64_t flush_bytes, StepTimes* t) {
   DMM_CUDA(cudaSetDevice(dev_));
-  TileForms tile_forms(*this);
+  TileForms tile_forms(*this, true);
   DMM_TRY(tile_forms.st);
   if (flush_bytes > flush_cap_) {
     if (flush_) retire(flush_);

@@ -251,10 +251,11 @@ dmm_status dmm_instance_assignment(dmm_instance* inst, int8_t* pre, int8_t* post
  *   6  the staged kernel with several clause and variable tiles per block (formulas whose
  *      tiles are too large for one of each per block)
  *   5  one block per formula
- * A small formula (about n <= 4,000 at 8 clauses per variable) with the default tiles, layout
- * and launch mode is run by one thread-block cluster, its data and exchanges in shared memory
- * (two cluster barriers per step), and reported as the form it stands in for: 4 for FP32 with
- * 3-literal clauses, else 3.
+ * With the default tiles, layout and launch mode a small formula (about 18,000 clauses in FP32,
+ * 13,000 in FP64) is run by one thread-block cluster, its data and exchanges in shared memory,
+ * and a larger one (up to about 450,000 clauses) by blocks that keep their voltages resident
+ * and exchange without grid barriers; both are reported as the form they stand in for: 4 for
+ * FP32 with 3-literal clauses, else 3.
  * A negative dmm_status on error. */
 int32_t dmm_instance_launch_form(const dmm_instance* inst);
 /* No counterpart in the reference.  Test hook for the failure path of the cooperative step
