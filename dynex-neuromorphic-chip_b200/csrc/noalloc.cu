@@ -8,19 +8,26 @@
 // counters) lives in one file-scope __device__ array of fixed size, so the call performs
 // no device allocation of its own.
 //
-// The array, g_na_scratch, is NA_SCRATCH_BYTES (about 2.1 MB) on every GPU that loads the
+// The array, g_na_scratch, is about 2.1 MB on every GPU that loads the
 // library, for the life of the process.  It bounds the formula: at most NA_MAX_VARS
 // variables and NA_MAX_CLAUSES clauses of exactly three literals, each variable in at
 // most NA_MAX_OCC literal slots.  The clause memory rate is the scalar alpha of the
 // parameters (no per-clause alpha).
 //
-// The call validates the formula on the device and reads two counters back (literals out
-// of range, over-long variable lists), waiting for the caller's stream each time, so it
-// blocks the calling thread until the work queued before it and its own checks finish; the
-// right-hand side itself is then queued on the stream without waiting for it.
+// One cooperative launch does everything: it checks the literals, evaluates the clauses and
+// counts occurrences, lays out and fills the variables' slot lists, and sums them; a failed
+// check ends it before dxdt or loc is written.  The call then reads the counters (literals out
+// of range, over-long variable lists; written to page-locked host memory), waiting for the
+// caller's stream once, so it blocks the calling thread until the work queued before it and
+// its own finish.
 //
-// Every call uses the same array and leaves its contents behind; each call clears the
-// parts that must start at zero.  Calls whose work overlaps on the GPU (different streams,
+// As nine launches and two waits a call took 105 us at n = 8,009, m = 64,007, nearly all of it
+// launch gaps and host round trips; with the one launch it takes 52, about 30 of them the
+// kernel (three grid barriers and the atomics that count and place 192,021 slots).
+//
+// Every call uses the same array and leaves its contents behind, but for the parts that must
+// start at zero: it zeroes them at its end and checks them at its start (counts left by calls
+// that raced are cleared and the launch repeated).  Calls whose work overlaps on the GPU (different streams,
 // or different host threads on one device) race on the array and must be serialized by
 // the caller.
 //
@@ -32,8 +39,8 @@
 // functions), so the output equals dmm_instance_rhs on an FP32 instance bit for bit.
 #include <mutex>
 
-#include "dmm_kernels.cuh"
 #include "dmm_pack.h"
+#include "dmm_step.cuh"
 
 namespace dmm {
 namespace {
@@ -41,114 +48,181 @@ namespace {
 constexpr int NA_MAX_VARS = 1 << 15;
 constexpr int NA_MAX_CLAUSES = 1 << 16;
 constexpr int NA_MAX_SLOTS = 3 * NA_MAX_CLAUSES;
-constexpr int NA_MAX_OCC = kSortCap;  // longest per-variable slot list the sorter handles
-constexpr int NA_THREADS = 256;
+constexpr int NA_MAX_OCC = 1024;  // longest per-variable slot list the sorter handles
+constexpr int NA_THREADS = 512;
 constexpr int NA_MAX_DEVICES = 64;
 
 struct NaScratch {
-  float u[NA_MAX_SLOTS];        // contribution of each literal slot
-  int32_t vslot[NA_MAX_SLOTS];  // variable-ordered slot lists
+  int2 list[NA_MAX_SLOTS];      // slots of the variables with their contributions
   float C[NA_MAX_CLAUSES];      // C_m of each clause
-  int32_t vend[NA_MAX_VARS];    // inclusive ends of the slot lists
-  int32_t fill[NA_MAX_VARS];    // scatter cursors
-  int32_t longv[NA_MAX_SLOTS / kSortCap + 2];  // variables with too many occurrences
-  int32_t counters[8];          // [0] unsatisfied clauses, [1] long lists, [2] bad literals
+  int32_t cnt[NA_MAX_VARS];     // occurrences (zero between calls)
+  int32_t fill[NA_MAX_VARS];    // list cursors: the lists' ends once filled
+  // [0] unsatisfied clauses, [1] long lists, [2] bad literals, [3] slots handed out (zero
+  // between calls), [4] a grid-barrier wait gave up
+  int32_t counters[8];
+  unsigned int bar[kLaunchAreaInts];  // grid barrier, left zeroed by every call
 };
-constexpr size_t NA_SCRATCH_BYTES = sizeof(NaScratch);
+static_assert(sizeof(NaScratch) < (size_t(22) << 20) / 10, "about 2.1 MB, as documented");
 
 __device__ __align__(256) NaScratch g_na_scratch;
 
 std::mutex g_na_mu;
 NaScratch* g_na_addr[NA_MAX_DEVICES] = {nullptr};
+int32_t* g_na_flags[NA_MAX_DEVICES] = {nullptr};  // page-locked host memory, four ints
 
-// Clears the counters and degree array (everything that accumulates).
-__global__ void k_na_clear(NaScratch* s, int n) {
-  for (int v = blockIdx.x * blockDim.x + threadIdx.x; v < n; v += gridDim.x * blockDim.x)
-    s->vend[v] = 0;
-  if (blockIdx.x == 0 && threadIdx.x < 8) s->counters[threadIdx.x] = 0;
-}
-
-// Inclusive scan of vend[0..n) (n <= NA_MAX_VARS) in one block of NA_THREADS threads: the
-// block walks the array in chunks of NA_THREADS consecutive entries (coalesced loads and
-// stores), scans each chunk with warp shuffles and carries the running total forward.
-__global__ void k_na_scan(NaScratch* s, int n) {
-  __shared__ int32_t wsum[NA_THREADS / 32];
-  __shared__ int32_t carry;
-  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-  if (threadIdx.x == 0) carry = 0;
-  __syncthreads();
-  for (int base = 0; base < n; base += NA_THREADS) {
-    const int i = base + threadIdx.x;
-    const int32_t v = i < n ? s->vend[i] : 0;
-    int32_t x = v;
+// Canonical sum (tree_sum) of variable v's contributions, by one warp: its d slots, in no
+// particular order in the list, are ranked (by shuffles up to 32 of them, else sorted in buf)
+// so that the slot of rank j is added to the j mod 32-th partial.
+__device__ __forceinline__ float na_sum(const NaScratch* s, int first, int d, int32_t* buf,
+                                        int lane) {
+  float p = 0.f;
+  if (d <= 32) {
+    int2 e = make_int2(0x7fffffff, 0);
+    if (lane < d) e = __ldcg(s->list + first + lane);
+    int rank = 0;
 #pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-      const int32_t y = __shfl_up_sync(0xffffffffu, x, o);
-      if (lane >= o) x += y;
+    for (int j = 0; j < 32; j++) rank += __shfl_sync(0xffffffffu, e.x, j) < e.x;
+    if (lane < d) buf[rank] = e.y;
+    __syncwarp();
+    if (lane < d) p = add(0.f, __int_as_float(buf[lane]));
+    __syncwarp();
+  } else {
+    int N = 64;
+    while (N < d) N <<= 1;
+    int32_t* val = buf + NA_MAX_OCC;
+    for (int j = lane; j < N; j += 32) {
+      int2 e = make_int2(0x7fffffff, 0);
+      if (j < d) e = __ldcg(s->list + first + j);
+      buf[j] = e.x;
+      val[j] = e.y;
     }
-    if (lane == 31) wsum[w] = x;
-    __syncthreads();
-    int32_t before = carry;
-    for (int k = 0; k < w; k++) before += wsum[k];
-    if (i < n) s->vend[i] = before + x;
-    __syncthreads();  // every thread has read carry and wsum
-    if (threadIdx.x == NA_THREADS - 1) carry = before + x;
-    __syncthreads();
+    __syncwarp();
+    for (int k = 2; k <= N; k <<= 1)
+      for (int j = k >> 1; j > 0; j >>= 1) {
+        for (int e = lane; e < N; e += 32) {
+          const int q = e ^ j;
+          if (q > e) {
+            const bool up = (e & k) == 0;
+            const int32_t a = buf[e], b = buf[q];
+            if (up ? (b < a) : (a < b)) {
+              const int32_t t = val[e];
+              buf[e] = b;
+              buf[q] = a;
+              val[e] = val[q];
+              val[q] = t;
+            }
+          }
+        }
+        __syncwarp();
+      }
+    for (int j = lane; j < d; j += 32) p = add(p, __int_as_float(val[j]));
+    __syncwarp();
   }
+#pragma unroll
+  for (int off = 16; off >= 1; off >>= 1) p = add(p, __shfl_xor_sync(0xffffffffu, p, off));
+  return p;
 }
 
-// Counts literals outside [-n, n] \ {0} (the caller's buffer is never indexed before this).
-__global__ void k_na_check(NaScratch* s, const int32_t* __restrict__ lits, int L, int n) {
-  int bad = 0;
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < L; i += gridDim.x * blockDim.x) {
-    const int32_t l = lits[i];
-    bad += (l == 0 || l > n || l < -n);
-  }
-  bad = warp_sum_i(bad);
-  if ((threadIdx.x & 31) == 0 && bad) atomicAdd(&s->counters[2], bad);
-}
-
-__global__ void k_na_clause(NaScratch* s, const int32_t* __restrict__ lits, int n, int m,
-                            const float* __restrict__ x, ClauseConsts<float> kc) {
-  int unsat = 0;
-  for (int c = blockIdx.x * blockDim.x + threadIdx.x; c < m; c += gridDim.x * blockDim.x) {
-    const int l0 = lits[3 * c], l1 = lits[3 * c + 1], l2 = lits[3 * c + 2];
-    float u0, u1, u2;
-    bool ss;
-    const float C = clause3(l0, l1, l2, x[abs(l0) - 1], x[abs(l1) - 1], x[abs(l2) - 1], x[n + c],
-                            x[n + m + c], kc, u0, u1, u2, ss);
-    s->u[3 * c] = u0;
-    s->u[3 * c + 1] = u1;
-    s->u[3 * c + 2] = u2;
-    s->C[c] = C;
-    unsat += !(C < 0.5f);
-  }
-  unsat = warp_sum_i(unsat);
-  if ((threadIdx.x & 31) == 0 && unsat) atomicAdd(&s->counters[0], unsat);
-}
-
-// dV of every variable in the canonical order (8 lanes per variable), then dXs / dXl.
-__global__ void k_na_var(NaScratch* s, int n, int m, const float* __restrict__ x,
-                         ClauseConsts<float> kc, float* __restrict__ dxdt) {
-  constexpr int G = 8;
-  const int lane = threadIdx.x % G;
-  const int warps_total = gridDim.x * (blockDim.x / G);
-  const int rounds = (n + warps_total - 1) / warps_total;
-  for (int r = 0; r < rounds; r++) {
-    const int v = r * warps_total + blockIdx.x * (blockDim.x / G) + threadIdx.x / G;
-    int s0 = 0, s1 = 0;
-    if (v < n) {
-      s1 = s->vend[v];
-      s0 = v > 0 ? s->vend[v - 1] : 0;
+// flags (host memory): counters [1], [2] and [4] of the call.
+__global__ void __launch_bounds__(NA_THREADS, 1)
+    k_na_rhs(NaScratch* s, const int32_t* __restrict__ lits, int n, int m, const float* x,
+             ClauseConsts<float> kc, float* dxdt, int32_t* loc, volatile int32_t* flags) {
+  extern __shared__ int32_t na_smem[];  // 2 NA_MAX_OCC per warp
+  __shared__ int s_ok;
+  const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
+  const int gt = blockIdx.x * NA_THREADS + tid, GT = gridDim.x * NA_THREADS;
+  unsigned int target = 0;
+  auto counter = [&](int k) { return *reinterpret_cast<volatile int32_t*>(&s->counters[k]); };
+  auto barrier = [&]() {
+    return grid_barrier<NA_THREADS>(s->bar, target, &s->counters[4], &s_ok);
+  };
+  {  // literals and occurrence counts
+    int bad = 0;
+    for (int q = gt; q < 3 * m; q += GT) {
+      const int l = lits[q];
+      if (l == 0 || l > n || l < -n) bad++;
+      else atomicAdd(&s->cnt[abs(l) - 1], 1);
     }
-    const float dv = tree_sum<float, G>(s->u, s->vslot + s0, s1 - s0, lane);
-    if (v < n && lane == 0) dxdt[v] = dv;
+    bad = warp_sum_i(bad);
+    if (lane == 0 && bad) atomicAdd(&s->counters[2], bad);
   }
-  for (int c = blockIdx.x * blockDim.x + threadIdx.x; c < m; c += gridDim.x * blockDim.x) {
-    const float xs = clampv(x[n + c], 0.f, 1.f);
-    const float C = s->C[c];
-    dxdt[n + c] = mul(mul(kc.beta, add(xs, kc.eps)), sub(C, kc.gamma));
-    dxdt[n + m + c] = mul(kc.alpha, sub(C, kc.delta));
+  bool ok = barrier();
+  const int bad_all = ok ? counter(2) : 0;  // grid-uniform
+  if (ok) {  // a range for every list (their order does not matter)
+    for (int v0 = blockIdx.x * NA_THREADS + 32 * w; v0 < n; v0 += GT) {
+      const int v = v0 + lane;
+      const int c = v < n ? __ldcg(s->cnt + v) : 0;
+      int incl = c;
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const int y = __shfl_up_sync(0xffffffffu, incl, o);
+        if (lane >= o) incl += y;
+      }
+      int first = 0;
+      if (lane == 31) first = atomicAdd(&s->counters[3], incl);
+      first = __shfl_sync(0xffffffffu, first, 31);
+      if (v < n) s->fill[v] = first + incl - c;
+      if (c > NA_MAX_OCC) atomicAdd(&s->counters[1], 1);
+    }
+    ok = barrier();
+  }
+  const int long_all = ok ? counter(1) : 0;
+  // the counts must add up: they were not all zero before this call otherwise
+  const bool dirty = ok && counter(3) + bad_all != 3 * m;
+  if (ok && (bad_all || long_all || dirty)) {  // nothing is written to dxdt and loc
+    if (dirty && gt == 0) atomicExch(&s->counters[4], 2);
+    for (int v = gt; v < n; v += GT) s->cnt[v] = 0;
+    ok = false;
+  } else if (ok) {
+    int unsat = 0;
+    for (int c = gt; c < m; c += GT) {
+      const int l0 = lits[3 * c], l1 = lits[3 * c + 1], l2 = lits[3 * c + 2];
+      const int p0 = atomicAdd(&s->fill[abs(l0) - 1], 1), p1 = atomicAdd(&s->fill[abs(l1) - 1], 1),
+                p2 = atomicAdd(&s->fill[abs(l2) - 1], 1);
+      float u0, u1, u2;
+      bool ss;
+      const float C = clause3(l0, l1, l2, x[abs(l0) - 1], x[abs(l1) - 1], x[abs(l2) - 1],
+                              x[n + c], x[n + m + c], kc, u0, u1, u2, ss);
+      s->list[p0] = make_int2(3 * c, __float_as_int(u0));
+      s->list[p1] = make_int2(3 * c + 1, __float_as_int(u1));
+      s->list[p2] = make_int2(3 * c + 2, __float_as_int(u2));
+      s->C[c] = C;
+      unsat += !(C < 0.5f);
+    }
+    unsat = warp_sum_i(unsat);
+    if (lane == 0 && unsat) atomicAdd(&s->counters[0], unsat);
+    ok = barrier();
+  }
+  if (ok) {  // dV of every variable, dXs and dXl of every clause
+    for (int v = blockIdx.x * (NA_THREADS / 32) + w; v < n; v += gridDim.x * (NA_THREADS / 32)) {
+      const int d = __ldcg(s->cnt + v), end = __ldcg(s->fill + v);
+      const float dv = na_sum(s, end - d, d, na_smem + w * 2 * NA_MAX_OCC, lane);
+      if (lane == 0) {
+        dxdt[v] = dv;
+        s->cnt[v] = 0;
+      }
+    }
+    for (int c = gt; c < m; c += GT) {
+      const float xs = clampv(x[n + c], 0.f, 1.f);
+      const float C = s->C[c];  // this thread's own
+      dxdt[n + c] = mul(mul(kc.beta, add(xs, kc.eps)), sub(C, kc.gamma));
+      dxdt[n + m + c] = mul(kc.alpha, sub(C, kc.delta));
+    }
+    if (gt == 0) *loc = counter(0);
+  }
+  // the last block to leave reports, and clears what must start at zero
+  __syncthreads();
+  if (tid == 0) {
+    __threadfence();
+    if (atomicAdd(s->bar + 1, 1u) == gridDim.x - 1) {
+      flags[0] = counter(1);
+      flags[1] = counter(2);
+      flags[2] = counter(4);
+      for (int k = 0; k < 8; k++) *reinterpret_cast<volatile int32_t*>(&s->counters[k]) = 0;
+      for (int k = 0; k < kLaunchAreaInts; k++)
+        *reinterpret_cast<volatile unsigned int*>(&s->bar[k]) = 0u;
+      __threadfence_system();
+    }
   }
 }
 
@@ -177,14 +251,19 @@ extern "C" dmm_status dmm_rhs3_f32_noalloc(const int32_t* lits, int32_t n, int32
     return DMM_ERR_ARG;
   }
   NaScratch* s = nullptr;
+  int32_t* flags = nullptr;
   {
     std::lock_guard<std::mutex> g(g_na_mu);
     if (!g_na_addr[dev]) {
       void* a = nullptr;
       DMM_CUDA(cudaGetSymbolAddress(&a, g_na_scratch));
+      void* h = nullptr;
+      DMM_CUDA(cudaHostAlloc(&h, 4 * sizeof(int32_t), cudaHostAllocPortable));
+      g_na_flags[dev] = static_cast<int32_t*>(h);
       g_na_addr[dev] = static_cast<NaScratch*>(a);
     }
     s = g_na_addr[dev];
+    flags = g_na_flags[dev];
   }
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   dmm_params d;
@@ -204,35 +283,36 @@ extern "C" dmm_status dmm_rhs3_f32_noalloc(const int32_t* lits, int32_t n, int32
     kc.xlmax = float((double)v);
   }
   const int L = 3 * m;
-  const int gb = (std::max(L, n) + NA_THREADS - 1) / NA_THREADS;
-  const int grid = std::max(1, std::min(gb, 148 * 8));
-  k_na_clear<<<grid, NA_THREADS, 0, st>>>(s, n);
-  if (L > 0) k_na_check<<<grid, NA_THREADS, 0, st>>>(s, lits, L, n);
-  DMM_CUDA(cudaGetLastError());
-  int32_t nbad = 0;
-  DMM_CUDA(cudaMemcpyAsync(&nbad, &s->counters[2], sizeof(int32_t), cudaMemcpyDeviceToHost, st));
-  DMM_CUDA(cudaStreamSynchronize(st));
-  if (nbad > 0) {
-    set_error("dmm_rhs3_f32_noalloc: %d literals outside [-n, n] or zero", nbad);
+  constexpr int kSmem = (NA_THREADS / 32) * 2 * NA_MAX_OCC * (int)sizeof(int32_t);
+  int sms = 0;
+  DMM_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+  DMM_CUDA(cudaFuncSetAttribute(k_na_rhs, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmem));
+  // a thread per slot, a warp per variable in a few rounds; at most a block per SM
+  const int want = std::max((L + NA_THREADS - 1) / NA_THREADS, (n + 63) / 64);
+  const int grid = std::max(1, std::min(want, sms));
+  volatile int32_t* hf = flags;
+  void* args[] = {&s, &lits, &n, &m, &x, &kc, &dxdt, &loc, &flags};
+  for (int attempt = 0; attempt < 2; attempt++) {
+    hf[0] = hf[1] = hf[2] = 0;
+    DMM_CUDA(cudaLaunchCooperativeKernel((const void*)k_na_rhs, dim3((unsigned)grid),
+                                         dim3(NA_THREADS), args, (size_t)kSmem, st));
+    DMM_CUDA(cudaStreamSynchronize(st));
+    if (hf[2] == 0) break;
+    // the scratch was not as a finished call leaves it (2), or a wait gave up (1)
+    DMM_CUDA(cudaMemsetAsync(s, 0, sizeof(NaScratch), st));
+    DMM_CUDA(cudaStreamSynchronize(st));
+    if (hf[2] == 1 || attempt == 1) {
+      set_error("dmm_rhs3_f32_noalloc: grid barrier wait gave up");
+      return DMM_ERR_CUDA;
+    }
+  }
+  if (hf[1] > 0) {
+    set_error("dmm_rhs3_f32_noalloc: %d literals outside [-n, n] or zero", hf[1]);
     return DMM_ERR_LITERAL;
   }
-  if (L > 0) k_count<<<grid, NA_THREADS, 0, st>>>(lits, L, n, s->vend, nullptr);
-  k_na_scan<<<1, NA_THREADS, 0, st>>>(s, n);
-  k_fill_start<<<grid, NA_THREADS, 0, st>>>(s->vend, n, s->fill);
-  if (L > 0) k_scatter<<<grid, NA_THREADS, 0, st>>>(lits, L, n, s->fill, s->vslot);
-  k_sort_lists<<<grid, kThreads, (kThreads / 32) * kSortCap * sizeof(int32_t), st>>>(
-      s->vend, n, s->vslot, s->longv, &s->counters[1], 0, NA_MAX_SLOTS / kSortCap + 2);
-  DMM_CUDA(cudaGetLastError());
-  int32_t nlong = 0;
-  DMM_CUDA(cudaMemcpyAsync(&nlong, &s->counters[1], sizeof(int32_t), cudaMemcpyDeviceToHost, st));
-  DMM_CUDA(cudaStreamSynchronize(st));
-  if (nlong > 0) {
+  if (hf[0] > 0) {
     set_error("dmm_rhs3_f32_noalloc: a variable occurs in more than %d literal slots", NA_MAX_OCC);
     return DMM_ERR_ARG;
   }
-  if (m > 0) k_na_clause<<<grid, NA_THREADS, 0, st>>>(s, lits, n, m, x, kc);
-  k_na_var<<<grid, NA_THREADS, 0, st>>>(s, n, m, x, kc, dxdt);
-  DMM_CUDA(cudaMemcpyAsync(loc, &s->counters[0], sizeof(int32_t), cudaMemcpyDeviceToDevice, st));
-  DMM_CUDA(cudaGetLastError());
   return DMM_OK;
 }
