@@ -43,6 +43,19 @@ struct dmm_batch {
   std::vector<int32_t> idx;
   std::vector<int32_t> m;
   bool dirty = true;
+  // The last run's control records, and (from the second result read after a run on) every
+  // formula's assignment: many results are read with one copy.  Any call that changes the
+  // batch discards them.
+  std::vector<InstCtrl> after;
+  std::vector<int8_t> post;
+  std::vector<int64_t> post_off;
+  int32_t reads = 0;
+  void changed() {
+    after.clear();
+    post.clear();
+    post_off.clear();
+    reads = 0;
+  }
 };
 
 extern "C" {
@@ -347,6 +360,7 @@ dmm_status dmm_batch_set_tuning(dmm_batch* b, const dmm_tuning* t) {
   dmm::clear_error();
   if (!b || !t) return DMM_ERR_ARG;
   b->dirty = true;
+  b->changed();
   return b->pack->set_tuning(t);
 }
 
@@ -356,6 +370,7 @@ dmm_status dmm_batch_add(dmm_batch* b, const int32_t* lits, const int64_t* claus
   dmm::clear_error();
   if (!b || !x0 || !index) return DMM_ERR_ARG;
   dmm::DeviceScope device_scope(b->pack->device());
+  b->changed();
   int32_t idx = -1;
   DMM_TRY(b->pack->add(lits, clause_off, n, m, p, nullptr, max_steps, &idx, x0));
   *index = (int32_t)b->idx.size();
@@ -374,6 +389,7 @@ dmm_status dmm_batch_run_until(dmm_batch* b, double wall_s, int32_t stop_after,
   dmm::clear_error();
   if (!b || stop_after < 0) return DMM_ERR_ARG;
   dmm::DeviceScope device_scope(b->pack->device());
+  b->changed();
   if (b->dirty) {
     DMM_TRY(b->pack->commit_tiles());
     b->dirty = false;
@@ -416,6 +432,7 @@ dmm_status dmm_batch_run_until(dmm_batch* b, double wall_s, int32_t stop_after,
     stats->wall_s = wall;
     stats->device_ms = ms;
   }
+  if (!timed_out && stop_after == 0) b->after = std::move(after);
   return DMM_OK;
 }
 
@@ -426,10 +443,20 @@ dmm_status dmm_batch_result(dmm_batch* b, int32_t index, dmm_report* rep, int8_t
   const int32_t i = b->idx[index];
   if (rep) {
     InstCtrl c;
-    DMM_TRY(b->pack->read_ctrl(i, &c));
+    if (!b->after.empty()) c = b->after[i];
+    else DMM_TRY(b->pack->read_ctrl(i, &c));
     fill_report(c, rep);
   }
-  if (post) DMM_TRY(b->pack->assignment(i, nullptr, post));
+  if (!post) return DMM_OK;
+  if (b->after.empty() || ++b->reads < 2) return b->pack->assignment(i, nullptr, post);
+  if (b->post_off.empty()) {
+    DMM_TRY(b->pack->assignments(b->idx, &b->post));
+    b->post_off.resize(b->idx.size() + 1);
+    for (size_t k = 0; k < b->idx.size(); k++)
+      b->post_off[k + 1] = b->post_off[k] + b->pack->desc(b->idx[k]).n;
+  }
+  std::memcpy(post, b->post.data() + b->post_off[index],
+              (size_t)(b->post_off[index + 1] - b->post_off[index]));
   return DMM_OK;
 }
 
@@ -451,6 +478,7 @@ dmm_status dmm_batch_set_state_at(dmm_batch* b, int32_t index, const double* x, 
                                   int32_t step) {
   dmm::clear_error();
   if (!b || !x || index < 0 || index >= (int32_t)b->idx.size() || step < 0) return DMM_ERR_ARG;
+  b->changed();
   dmm::DeviceScope device_scope(b->pack->device());
   return b->pack->set_state_at(b->idx[index], x, t, step, false);
 }

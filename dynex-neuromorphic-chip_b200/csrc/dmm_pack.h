@@ -114,6 +114,11 @@ class Pack {
   dmm_status add(const int32_t* lits, const int64_t* clause_off, int32_t n, int32_t m,
                  const dmm_params* p, const double* alpha_cm, int32_t max_steps, int32_t* idx,
                  const double* x0 = nullptr, bool device_literal_check = false);
+  // Unpacks the formulas that add() has only laid aside (small ones with an initial state);
+  // every call that reads or changes device state does so first.
+  dmm_status flush_adds();
+  // Reported assignments of several formulas, one after another.
+  dmm_status assignments(const std::vector<int32_t>& idx, std::vector<int8_t>* out);
   dmm_status remove(int32_t idx);
   dmm_status set_params(int32_t idx, const dmm_params* p, const double* alpha_cm);
   dmm_status set_max_steps(int32_t idx, int32_t max_steps);
@@ -185,6 +190,10 @@ class Pack {
   int sm_count() const { return sms_; }
 
  private:
+  // lays a small formula aside in the current page-locked block (dmm_admit.cuh); *done false
+  // when it does not go there
+  dmm_status stage_add(const InstDesc& I, int32_t idx, const int32_t* lits,
+                       const int64_t* clause_off, bool units, const double* x0, bool* done);
   dmm_status build_csr(const InstDesc& I, const int32_t* lits);
   // sorts the slot lists longer than the device sorter (reported by the CSR builds since
   // the last call); runs before the CSR is first used
@@ -341,6 +350,19 @@ class Pack {
          kGrDlo, kGrOut, kGrSync, kGrEpart, kGrBufs };
   void* gbuf_[kGrBufs] = {};
   int64_t gbuf_cap_[kGrBufs] = {};
+  // blocks of formulas laid aside (two, filled in turn) and their device copies
+  static constexpr int64_t kAdmitBytes = int64_t(16) << 20;
+  static constexpr int kAdmitRecs = 1024;
+  struct AdmitBlock {
+    unsigned char* host = nullptr;  // records, then data
+    unsigned char* dev = nullptr;
+    cudaEvent_t sent = nullptr;
+    bool busy = false;
+    int count = 0;
+    int64_t used = 0;
+  };
+  AdmitBlock admit_[2];
+  int admit_cur_ = 0;
   // largest bucket and slot count of a block for each cluster size, per formula
   struct ClusterNeed {
     uint64_t serial = 0;

@@ -9,6 +9,7 @@
 #include <thread>
 #include <vector>
 
+#include "dmm_admit.cuh"
 #include "dmm_cluster.h"
 #include "dmm_inst.cuh"
 #include "dmm_step.cuh"
@@ -268,6 +269,11 @@ Pack::~Pack() {
     if (p) dev_free(p);
   for (auto& e : ev_)
     if (e) cudaEventDestroy(e);
+  for (auto& a : admit_) {
+    if (a.host) pinned_free(a.host);
+    if (a.dev) dev_free(a.dev);
+    if (a.sent) cudaEventDestroy(a.sent);
+  }
   for (auto& x : side_) {
     if (x.first) cudaStreamSynchronize(x.first);
     if (x.first) cudaStreamDestroy(x.first);
@@ -463,12 +469,14 @@ __global__ void k_signs(const InstCtrl* __restrict__ ctrl, const T* __restrict__
 
 
 dmm_status Pack::upload_desc(int32_t idx) {
+  DMM_TRY(flush_adds());
   k_put_desc<<<1, 1, 0, stream_>>>(inst_d_ + idx, inst_h_[idx]);
   DMM_CUDA(cudaGetLastError());
   return DMM_OK;
 }
 
 dmm_status Pack::write_ctrl(int32_t idx, const InstCtrl& c) {
+  DMM_TRY(flush_adds());
   k_put_ctrl<<<1, 1, 0, stream_>>>(ctrl_d_ + idx, c);
   DMM_CUDA(cudaGetLastError());
   return DMM_OK;
@@ -487,12 +495,14 @@ dmm_status Pack::read_ctrl(int32_t idx, InstCtrl* c) {
     set_error("instance %d is not live", idx);
     return DMM_ERR_ARG;
   }
+  DMM_TRY(flush_adds());
   DMM_CUDA(cudaMemcpyAsync(c, ctrl_d_ + idx, sizeof(InstCtrl), cudaMemcpyDeviceToHost, stream_));
   DMM_CUDA(cudaStreamSynchronize(stream_));
   return DMM_OK;
 }
 
 dmm_status Pack::read_ctrls(std::vector<InstCtrl>* out) {
+  DMM_TRY(flush_adds());
   out->resize(caps_.insts);
   DMM_CUDA(cudaMemcpyAsync(out->data(), ctrl_d_, caps_.insts * sizeof(InstCtrl),
                            cudaMemcpyDeviceToHost, stream_));
@@ -559,6 +569,7 @@ dmm_status Pack::build_csr(const InstDesc& I, const int32_t* lits_host) {
 }
 
 dmm_status Pack::resolve_long_lists() {
+  DMM_TRY(flush_adds());
   if (!long_pending_) return DMM_OK;
   int32_t counts[2] = {0, 0};  // long lists, literals the CSR build found out of range
   DMM_CUDA(cudaMemcpyAsync(counts, ring_tail_d_ + 2, sizeof counts, cudaMemcpyDeviceToHost,
@@ -671,6 +682,107 @@ static dmm_status upload_alpha(T* dst, const double* a, int32_t m, cudaStream_t 
   return DMM_OK;
 }
 
+dmm_status Pack::stage_add(const InstDesc& I, int32_t idx, const int32_t* lits,
+                           const int64_t* clause_off, bool units, const double* x0, bool* done) {
+  *done = false;
+  const int64_t n = I.n, m = I.m, L = I.nslots;
+  auto al = [](int64_t b) { return (b + 15) & ~int64_t(15); };
+  const int64_t b_lit = al(4 * L), b_coff = I.k3 ? 0 : al(4 * m), b_unit = units ? al(n) : 0,
+                b_x = al((n + 2 * m) * (int64_t)tsize_);
+  const int64_t head = (int64_t)kAdmitRecs * sizeof(AdmitRec);
+  if (n > kAdmitVars || L > kAdmitSlots || head + b_lit + b_coff + b_unit + b_x > kAdmitBytes)
+    return DMM_OK;
+  if (admit_[admit_cur_].count == kAdmitRecs ||
+      head + admit_[admit_cur_].used + b_lit + b_coff + b_unit + b_x > kAdmitBytes)
+    DMM_TRY(flush_adds());
+  AdmitBlock& A = admit_[admit_cur_];
+  if (!A.host) {
+    void *h = nullptr, *dv = nullptr;
+    DMM_CUDA(pinned_alloc(&h, kAdmitBytes));
+    A.host = static_cast<unsigned char*>(h);
+    DMM_CUDA(dev_alloc(&dv, kAdmitBytes));
+    A.dev = static_cast<unsigned char*>(dv);
+    DMM_CUDA(cudaEventCreateWithFlags(&A.sent, cudaEventDisableTiming));
+  }
+  if (A.busy) {  // its previous contents are still on their way
+    DMM_CUDA(cudaEventSynchronize(A.sent));
+    A.busy = false;
+  }
+  AdmitRec R{};
+  R.I = I;
+  R.c = running_ctrl(I, 0.0, 0);
+  R.idx = idx;
+  int64_t at = head + A.used;
+  R.lit = at;
+  std::memcpy(A.host + at, lits, (size_t)L * 4);
+  at += b_lit;
+  R.coff = R.unit = -1;
+  if (!I.k3) {
+    R.coff = at;
+    int32_t* o = reinterpret_cast<int32_t*>(A.host + at);
+    for (int64_t c = 0; c < m; c++) o[c] = (int32_t)clause_off[c];
+    at += b_coff;
+  }
+  if (units) {
+    R.unit = at;
+    int8_t* u = reinterpret_cast<int8_t*>(A.host + at);
+    std::memset(u, 0, (size_t)n);
+    for (int64_t c = 0; c < m; c++)
+      if (clause_off[c + 1] - clause_off[c] == 1) {
+        const int32_t l = lits[clause_off[c]];
+        u[std::abs(l) - 1] = l > 0 ? 1 : -1;
+      }
+    at += b_unit;
+  }
+  R.x = at;
+  if (prec_ == DMM_FP64) {
+    std::memcpy(A.host + at, x0, (size_t)(n + 2 * m) * 8);
+  } else {
+    float* o = reinterpret_cast<float*>(A.host + at);
+    for (int64_t i = 0; i < n + 2 * m; i++) o[i] = (float)x0[i];
+  }
+  at += b_x;
+  std::memcpy(A.host + (int64_t)A.count * sizeof(AdmitRec), &R, sizeof R);
+  A.count++;
+  A.used = at - head;
+  *done = true;
+  return DMM_OK;
+}
+
+dmm_status Pack::flush_adds() {
+  AdmitBlock& A = admit_[admit_cur_];
+  if (A.count == 0) return DMM_OK;
+  const int64_t head = (int64_t)kAdmitRecs * sizeof(AdmitRec);
+  const int count = A.count;
+  const int64_t used = A.used;
+  A.count = 0;
+  A.used = 0;
+  DMM_CUDA(cudaMemcpyAsync(A.dev, A.host, (size_t)count * sizeof(AdmitRec), cudaMemcpyHostToDevice,
+                           stream_));
+  DMM_CUDA(cudaMemcpyAsync(A.dev + head, A.host + head, (size_t)used, cudaMemcpyHostToDevice, stream_));
+  const int smem = (kAdmitVars + (kAdmitThreads / 32) * kSortCap) * 4;
+  const AdmitRec* recs = reinterpret_cast<const AdmitRec*>(A.dev);
+  if (prec_ == DMM_FP64) {
+    DMM_CUDA(cudaFuncSetAttribute(k_admit<double>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+    k_admit<double><<<count, kAdmitThreads, smem, stream_>>>(
+        recs, A.dev, inst_d_, ctrl_d_, lit_, vslot_, upos_, vend_, coff_, unit_,
+        static_cast<double*>(cand_), static_cast<double*>(Xs_), static_cast<double*>(Xl_), active_d_,
+        longv_d_, ring_tail_d_ + 2, longv_cap_);
+  } else {
+    DMM_CUDA(cudaFuncSetAttribute(k_admit<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+    k_admit<float><<<count, kAdmitThreads, smem, stream_>>>(
+        recs, A.dev, inst_d_, ctrl_d_, lit_, vslot_, upos_, vend_, coff_, unit_,
+        static_cast<float*>(cand_), static_cast<float*>(Xs_), static_cast<float*>(Xl_), active_d_,
+        longv_d_, ring_tail_d_ + 2, longv_cap_);
+  }
+  DMM_CUDA(cudaGetLastError());
+  DMM_CUDA(cudaEventRecord(A.sent, stream_));
+  A.busy = true;
+  admit_cur_ ^= 1;
+  long_pending_ = true;
+  return DMM_OK;
+}
+
 dmm_status Pack::add(const int32_t* lits, const int64_t* clause_off, int32_t n, int32_t m,
                      const dmm_params* p, const double* alpha_cm, int32_t max_steps,
                      int32_t* idx_out, const double* x0, bool device_literal_check) {
@@ -699,6 +811,36 @@ dmm_status Pack::add(const int32_t* lits, const int64_t* clause_off, int32_t n, 
     if (cls0 >= 0) cls_alloc_.free(cls0, m);
     set_error("pack capacity exhausted (n=%d m=%d literals=%lld)", n, m, (long long)L);
     return DMM_ERR_BUDGET;
+  }
+  // small formulas with an initial state are laid aside and unpacked many at a time
+  if (x0 && !alpha_cm && !device_literal_check && n <= kAdmitVars && L <= kAdmitSlots) {
+    bool k3 = false, units = true, done = false;
+    dmm_status st = validate_formula(lits, clause_off, n, m, &k3, &units, true);
+    InstDesc I{};
+    I.n = n;
+    I.m = m;
+    I.var0 = var0;
+    I.cls0 = cls0;
+    I.slot0 = slot0;
+    I.nslots = (int32_t)L;
+    I.k3 = k3 ? 1 : 0;
+    I.max_steps = max_steps;
+    fill_params(I, p);
+    if (st == DMM_OK) st = stage_add(I, idx, lits, clause_off, units, x0, &done);
+    if (st != DMM_OK) {
+      var_alloc_.free(var0, n);
+      cls_alloc_.free(cls0, m);
+      slot_alloc_.free(slot0, L);
+      return st;
+    }
+    if (done) {
+      inst_h_[idx] = I;
+      live_[idx] = 1;
+      add_serial_[idx] = ++add_counter_;
+      if (!fixed_grid_) graph_stale_ = true;
+      *idx_out = idx;
+      return DMM_OK;
+    }
   }
   // the literal upload runs while the host checks the clauses (and literals)
   if (L > 0)
@@ -894,6 +1036,7 @@ InstCtrl Pack::running_ctrl(const InstDesc& I, double t, int32_t step) {
 
 dmm_status Pack::get_state(int32_t idx, double* x, double* t) {
   if (!live(idx)) return DMM_ERR_ARG;
+  DMM_TRY(flush_adds());
   const InstDesc& I = inst_h_[idx];
   const int64_t N = (int64_t)I.n + 2 * (int64_t)I.m;
   DMM_TRY(ensure_stage(3 * N));
@@ -2223,6 +2366,7 @@ dmm_status Pack::profile_steps(int32_t nsteps, int64_t flush_bytes, StepTimes* t
 }
 
 dmm_status Pack::read_active(int32_t* active) {
+  DMM_TRY(flush_adds());
   DMM_CUDA(cudaMemcpyAsync(active, active_d_, sizeof(int32_t), cudaMemcpyDeviceToHost, stream_));
   DMM_CUDA(cudaStreamSynchronize(stream_));
   return DMM_OK;
@@ -2375,6 +2519,7 @@ dmm_status Pack::rhs(int32_t idx, const double* x, double* dxdt, int32_t* loc, d
 
 dmm_status Pack::dostep(int32_t idx, const double* x, const double* dxdt, double h, double* xo) {
   if (!live(idx) || !x || !dxdt || !xo) return DMM_ERR_ARG;
+  DMM_TRY(flush_adds());
   const InstDesc& I = inst_h_[idx];
   const int64_t N = (int64_t)I.n + 2 * (int64_t)I.m;
   DMM_TRY(ensure_stage(3 * N));
@@ -2392,8 +2537,41 @@ dmm_status Pack::dostep(int32_t idx, const double* x, const double* dxdt, double
   return DMM_OK;
 }
 
+dmm_status Pack::assignments(const std::vector<int32_t>& idx, std::vector<int8_t>* out) {
+  DMM_TRY(flush_adds());
+  std::vector<int64_t> off(idx.size());
+  int64_t total = 0;
+  for (size_t k = 0; k < idx.size(); k++) {
+    if (!live(idx[k])) return DMM_ERR_ARG;
+    off[k] = total;
+    total += inst_h_[idx[k]].n;
+  }
+  out->resize((size_t)total);
+  if (idx.empty()) return DMM_OK;
+  // [offsets | indices | signs] in the staging buffer
+  const int64_t o_idx = (int64_t)idx.size() * 8, o_out = o_idx + (((int64_t)idx.size() * 4 + 15) & ~15);
+  DMM_TRY(ensure_stage((o_out + total + 7) / 8));
+  unsigned char* base = reinterpret_cast<unsigned char*>(stage_);
+  DMM_CUDA(cudaMemcpyAsync(base, off.data(), off.size() * 8, cudaMemcpyHostToDevice, stream_));
+  DMM_CUDA(cudaMemcpyAsync(base + o_idx, idx.data(), idx.size() * 4, cudaMemcpyHostToDevice, stream_));
+  int8_t* dst = reinterpret_cast<int8_t*>(base + o_out);
+  const auto* di = reinterpret_cast<const int32_t*>(base + o_idx);
+  const auto* doff = reinterpret_cast<const int64_t*>(base);
+  if (prec_ == DMM_FP64)
+    k_signs_all<double><<<(unsigned)idx.size(), kThreads, 0, stream_>>>(
+        inst_d_, ctrl_d_, di, doff, static_cast<const double*>(cand_), caps_.vars, dst);
+  else
+    k_signs_all<float><<<(unsigned)idx.size(), kThreads, 0, stream_>>>(
+        inst_d_, ctrl_d_, di, doff, static_cast<const float*>(cand_), caps_.vars, dst);
+  DMM_CUDA(cudaGetLastError());
+  DMM_CUDA(cudaMemcpyAsync(out->data(), dst, (size_t)total, cudaMemcpyDeviceToHost, stream_));
+  DMM_CUDA(cudaStreamSynchronize(stream_));
+  return DMM_OK;
+}
+
 dmm_status Pack::assignment(int32_t idx, int8_t* pre, int8_t* post) {
   if (!live(idx)) return DMM_ERR_ARG;
+  DMM_TRY(flush_adds());
   if (!pre && !post) return DMM_OK;
   const InstDesc& I = inst_h_[idx];
   // [flag | pre (n) | post (n)] in the staging buffer
