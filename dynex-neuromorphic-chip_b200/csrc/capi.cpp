@@ -94,7 +94,10 @@ void dmm_params_default(dmm_params* p) {
   p->reserved = 0;
 }
 
-void dmm_release_cached_memory(void) { dmm::release_cached(); }
+void dmm_release_cached_memory(void) {
+  dmm::release_xfers();
+  dmm::release_cached();
+}
 
 int32_t dmm_device_count(void) {
   int n = 0;

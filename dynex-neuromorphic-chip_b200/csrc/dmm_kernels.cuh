@@ -568,14 +568,14 @@ __global__ void k_set_state(const double* __restrict__ x, int n, int m, T* __res
   }
 }
 
-// Current state (after the last accepted step) -> x doubles; applies a pending Xs/Xl
-// update without storing it.
+// Current state (after the last accepted step) -> x; applies a pending Xs/Xl update without
+// storing it.
 template <class T>
 __global__ void k_get_state(const InstDesc* __restrict__ insts, const InstCtrl* __restrict__ ctrl,
                             int ii, const T* __restrict__ cand, int64_t var_cap,
                             const T* __restrict__ Xs, const T* __restrict__ Xl,
                             const T* __restrict__ Cp, const T* __restrict__ alpha_cm,
-                            double* __restrict__ x) {
+                            T* __restrict__ x) {
   const InstDesc I = insts[ii];
   const InstCtrl S = ctrl[ii];
   const ClauseConsts<T> kc = make_consts<T>(I, S.h_state);
@@ -584,7 +584,7 @@ __global__ void k_get_state(const InstDesc* __restrict__ insts, const InstCtrl* 
   for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < N;
        i += (int64_t)gridDim.x * blockDim.x) {
     if (i < I.n) {
-      x[i] = (double)V[i];
+      x[i] = V[i];
     } else {
       const int c = (int)((i < I.n + I.m) ? i - I.n : i - I.n - I.m);
       T xs = Xs[I.cls0 + c], xl = Xl[I.cls0 + c];
@@ -592,7 +592,7 @@ __global__ void k_get_state(const InstDesc* __restrict__ insts, const InstCtrl* 
         const T al = I.has_alpha_cm ? alpha_cm[I.cls0 + c] : kc.alpha;
         advance_memory(xs, xl, Cp[I.cls0 + c], al, kc);
       }
-      x[i] = (double)((i < I.n + I.m) ? xs : xl);
+      x[i] = (i < I.n + I.m) ? xs : xl;
     }
   }
 }

@@ -14,6 +14,7 @@
 #include "dmm_cluster.h"
 #include "dmm_device.cuh"
 #include "dmm_grid.h"
+#include "hostpool.h"
 
 namespace dmm {
 
@@ -232,6 +233,11 @@ class Pack {
   dmm_status write_ctrl(int32_t idx, const InstCtrl& c);
   dmm_status add_active(int32_t delta);
   dmm_status upload_state(const InstDesc& I, const double* x);
+  // count doubles between the host and device memory of this pack's stream
+  dmm_status upload_doubles(double* dst, const double* src, int64_t count);
+  template <class T>
+  dmm_status download_state(double* dst, const T* src, int64_t count);
+  dmm_status pinned();
   static InstCtrl running_ctrl(const InstDesc& I, double t, int32_t step);
   void retire(void* p);  // dev_free after this pack's queued work
 
@@ -299,7 +305,8 @@ class Pack {
   Tile* vtiles_d_ = nullptr;
   int32_t* ntiles_d_ = nullptr;  // [0..1] main tables, [2..3] auxiliary
   int32_t* queue_d_ = nullptr;
-  int32_t* active_d_ = nullptr;
+  int32_t* active_d_ = nullptr;  // (in ring_tail_d_)
+  int32_t* error_d_ = nullptr;   // (in ring_tail_d_)
   int32_t* ring_d_ = nullptr;
   int32_t* ring_tail_d_ = nullptr;
   int32_t* scan_tmp_ = nullptr;
@@ -315,7 +322,7 @@ class Pack {
   void* flush_ = nullptr;
   int64_t flush_cap_ = 0;
   cudaEvent_t ev_[4] = {nullptr, nullptr, nullptr, nullptr};
-  int32_t* pinned_ = nullptr;  // host copies of the running count and finished-ring tail
+  int32_t* pinned_ = nullptr;  // page-locked copies of the status words and control records
   int32_t* live_d_ = nullptr;  // indices of the instances with tiles
   int32_t* misc_d_ = nullptr;  // [0] live count, [1] barrier error, [2] barrier counter,
                                // [3] formula queue of the one-block-per-formula kernel

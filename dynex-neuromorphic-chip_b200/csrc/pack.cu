@@ -6,7 +6,6 @@
 #include <cstdarg>
 #include <cstdio>
 #include <cstring>
-#include <thread>
 #include <vector>
 
 #include "dmm_admit.cuh"
@@ -53,33 +52,16 @@ dmm_status validate_shape(const int32_t* lits, const int64_t* clause_off, int32_
   return DMM_OK;
 }
 
-// Runs f(lo, hi, t) over the chunks t of [0, len) on up to kValidateThreads host threads
-// when len is large (these passes are bound by memory bandwidth, which one core does not
-// reach); returns the number of chunks.  Falls back to one chunk on the calling thread
-// when no thread can be started.
-constexpr int kValidateThreads = 8;
-constexpr int64_t kValidateChunk = int64_t(1) << 18;  // elements per thread at least
+// Runs f(lo, hi, t) over the chunks t of [0, len) on the helper threads when len is large
+// (these passes are bound by memory bandwidth, which one core does not reach); returns the
+// number of chunks.
+constexpr int kValidateThreads = kPoolHelpers + 1;
+constexpr int64_t kValidateChunk = int64_t(1) << 14;  // elements per thread at least
 template <class F>
 static int host_parallel(int64_t len, F&& f) {
-  const int64_t hw = std::max(1u, std::thread::hardware_concurrency());
-  const int T = (int)std::max<int64_t>(
-      1, std::min<int64_t>({(int64_t)kValidateThreads, hw, len / kValidateChunk}));
-  if (T <= 1) {
-    f(int64_t(0), len, 0);
-    return 1;
-  }
+  const int T = (int)std::max<int64_t>(1, std::min<int64_t>(kValidateThreads, len / kValidateChunk));
   const int64_t per = (len + T - 1) / T;
-  std::vector<std::thread> th;
-  try {
-    for (int t = 1; t < T; t++)
-      th.emplace_back([&f, t, per, len] { f(t * per, std::min(len, (t + 1) * per), t); });
-  } catch (...) {
-    for (auto& x : th) x.join();
-    f(int64_t(0), len, 0);
-    return 1;
-  }
-  f(int64_t(0), std::min(len, per), 0);
-  for (auto& x : th) x.join();
+  pool_run(T, [&](int t) { f(t * per, std::min(len, (t + 1) * per), t); });
   return T;
 }
 
@@ -232,6 +214,8 @@ constexpr int kXpSmemMax = 220 * 1024;  // dynamic shared memory of the staged f
 constexpr int kXpSmemMaxMT = 193 * 1024;  // with the form's ~1.4 KB of static shared memory
 constexpr int kClusterChunk = 8;        // launches of steps_per_graph steps run() makes one of
 constexpr int kXpMaxTiles = 1 << 14;    // clause or variable tiles of the staged form, at most
+constexpr int kStatusInts = 8;           // ring_tail_d_
+constexpr int64_t kDirectCopy = 1 << 13; // doubles the driver's own pageable copies move
 constexpr int kMiscInts = 48;            // misc_d_: 192 bytes
 constexpr int kMiscLaunch = 16;          // misc_d_ index of the per-launch area (byte 64)
 constexpr int kMiscAcc2 = 20;            // misc_d_ index of the StepAcc pair (byte 80)
@@ -258,7 +242,7 @@ Pack::~Pack() {
   void* ptrs[] = {Xs_,      Xl_,        Cp_,      alpha_cm_,   u_,         cand_,
                   coff_,    lit_,       vslot_,   vend_,       fill_,      unit_,
                   epart_,   inst_d_,    ctrl_d_,  ctiles_d_,   vtiles_d_,  ntiles_d_,
-                  queue_d_, active_d_,  ring_d_,  ring_tail_d_, scan_tmp_, longv_d_,
+                  queue_d_, ring_d_,  ring_tail_d_, scan_tmp_, longv_d_,
                   stage_,   aux_ctiles_d_, aux_vtiles_d_, flush_, live_d_, misc_d_, order_d_,
                   upos_,    trace_};
   for (void* p : ptrs)
@@ -330,9 +314,12 @@ dmm_status Pack::init(const PackCaps& caps_in, bool with_alpha_cm, bool fixed_gr
   DMM_CUDA(dev_alloc(&vtiles_d_, vtile_cap_ * sizeof(Tile)));
   DMM_CUDA(dev_alloc(&ntiles_d_, 4 * sizeof(int32_t)));
   DMM_CUDA(dev_alloc(&queue_d_, 2 * sizeof(int32_t)));
-  DMM_CUDA(dev_alloc(&active_d_, sizeof(int32_t)));
   DMM_CUDA(dev_alloc(&ring_d_, I * sizeof(int32_t)));
-  DMM_CUDA(dev_alloc(&ring_tail_d_, 4 * sizeof(int32_t)));
+  // status words: [0] finished-ring tail, [2] long lists, [3] bad literals, [4] running
+  // formulas, [5] barrier error
+  DMM_CUDA(dev_alloc(&ring_tail_d_, kStatusInts * sizeof(int32_t)));
+  active_d_ = ring_tail_d_ + 4;
+  error_d_ = ring_tail_d_ + 5;
   longv_cap_ = (int32_t)(S / kSortCap + 2);
   DMM_CUDA(dev_alloc(&longv_d_, longv_cap_ * sizeof(int32_t)));
   DMM_CUDA(dev_alloc(&live_d_, I * sizeof(int32_t)));
@@ -344,8 +331,7 @@ dmm_status Pack::init(const PackCaps& caps_in, bool with_alpha_cm, bool fixed_gr
   DMM_CUDA(cudaMemsetAsync(ctrl_d_, 0, I * sizeof(InstCtrl), stream_));
   DMM_CUDA(cudaMemsetAsync(ntiles_d_, 0, 4 * sizeof(int32_t), stream_));
   DMM_CUDA(cudaMemsetAsync(queue_d_, 0, 2 * sizeof(int32_t), stream_));
-  DMM_CUDA(cudaMemsetAsync(active_d_, 0, sizeof(int32_t), stream_));
-  DMM_CUDA(cudaMemsetAsync(ring_tail_d_, 0, 4 * sizeof(int32_t), stream_));
+  DMM_CUDA(cudaMemsetAsync(ring_tail_d_, 0, kStatusInts * sizeof(int32_t), stream_));
   DMM_CUDA(cudaMemsetAsync(cand_, 0, 2 * kTrials * V * tsize_, stream_));
   var_alloc_.reset(V);
   cls_alloc_.reset(C);
@@ -443,6 +429,15 @@ void Pack::retire(void* p) {
 // Small records travel as kernel arguments: stream-ordered, no host staging, no wait.
 __global__ void k_put_desc(InstDesc* dst, InstDesc d) { *dst = d; }
 __global__ void k_put_ctrl(InstCtrl* dst, InstCtrl c) { *dst = c; }
+// The control record of a restarted formula; one that was not running is counted again.
+__global__ void k_restart(InstCtrl* dst, InstCtrl c, int keep_best, int32_t* active) {
+  if (dst->done != 0) atomicAdd(active, 1);
+  if (keep_best) {
+    c.best_loc = dst->best_loc;
+    c.best_t = dst->best_t;
+  }
+  *dst = c;
+}
 
 // Signs of V on the device (the control record says which candidate holds it), so that
 // one byte per variable crosses to the host: pre from the solving step's V (0 for V == 0;
@@ -714,7 +709,7 @@ dmm_status Pack::stage_add(const InstDesc& I, int32_t idx, const int32_t* lits,
   R.idx = idx;
   int64_t at = head + A.used;
   R.lit = at;
-  std::memcpy(A.host + at, lits, (size_t)L * 4);
+  unsigned char* const lit_at = A.host + at;
   at += b_lit;
   R.coff = R.unit = -1;
   if (!I.k3) {
@@ -735,13 +730,22 @@ dmm_status Pack::stage_add(const InstDesc& I, int32_t idx, const int32_t* lits,
     at += b_unit;
   }
   R.x = at;
-  if (prec_ == DMM_FP64) {
-    std::memcpy(A.host + at, x0, (size_t)(n + 2 * m) * 8);
-  } else {
-    float* o = reinterpret_cast<float*>(A.host + at);
-    for (int64_t i = 0; i < n + 2 * m; i++) o[i] = (float)x0[i];
-  }
+  unsigned char* const x_at = A.host + at;
   at += b_x;
+  // literals and state, in parts of both
+  const int parts = pool_parts(4 * L + 8 * (n + 2 * m));
+  pool_run(parts, [&](int i) {
+    const int64_t N = n + 2 * m;
+    const int64_t l0 = L * i / parts, l1 = L * (i + 1) / parts, e0 = N * i / parts,
+                  e1 = N * (i + 1) / parts;
+    std::memcpy(lit_at + 4 * l0, lits + l0, (size_t)(l1 - l0) * 4);
+    if (prec_ == DMM_FP64) {
+      std::memcpy(x_at + 8 * e0, x0 + e0, (size_t)(e1 - e0) * 8);
+    } else {
+      float* o = reinterpret_cast<float*>(x_at);
+      for (int64_t e = e0; e < e1; e++) o[e] = (float)x0[e];
+    }
+  });
   std::memcpy(A.host + (int64_t)A.count * sizeof(AdmitRec), &R, sizeof R);
   A.count++;
   A.used = at - head;
@@ -989,23 +993,55 @@ dmm_status Pack::set_state_at(int32_t idx, const double* x, double t, int32_t st
     return DMM_ERR_ARG;
   }
   const InstDesc& I = inst_h_[idx];
-  InstCtrl old;
-  DMM_TRY(read_ctrl(idx, &old));
+  DMM_TRY(flush_adds());
   DMM_TRY(upload_state(I, x));
-  InstCtrl c = running_ctrl(I, t, step);
-  if (keep_best) {
-    c.best_loc = old.best_loc;
-    c.best_t = old.best_t;
-  }
-  if (old.done != 0) DMM_TRY(add_active(+1));
-  DMM_TRY(write_ctrl(idx, c));
+  k_restart<<<1, 1, 0, stream_>>>(ctrl_d_ + idx, running_ctrl(I, t, step), keep_best ? 1 : 0,
+                                  active_d_);
+  DMM_CUDA(cudaGetLastError());
   if (page_locked(x)) DMM_CUDA(cudaStreamSynchronize(stream_));
   return DMM_OK;
 }
 
+dmm_status Pack::pinned() {
+  if (!pinned_) DMM_CUDA(pinned_alloc(&pinned_, 4096));
+  return DMM_OK;
+}
+
+dmm_status Pack::upload_doubles(double* dst, const double* src, int64_t count) {
+  if (count <= kDirectCopy || page_locked(src))
+    DMM_CUDA(cudaMemcpyAsync(dst, src, count * sizeof(double), cudaMemcpyHostToDevice, stream_));
+  else
+    DMM_CUDA(XferLease()->upload<double>(dst, src, count, stream_));
+  return DMM_OK;
+}
+
+template <class T>
+dmm_status Pack::download_state(double* dst, const T* src, int64_t count) {
+  if (sizeof(T) == 8 && (count <= kDirectCopy || page_locked(dst))) {
+    DMM_CUDA(cudaMemcpyAsync(dst, src, count * sizeof(T), cudaMemcpyDeviceToHost, stream_));
+    DMM_CUDA(cudaStreamSynchronize(stream_));
+  } else {
+    DMM_CUDA(XferLease()->download<T>(dst, src, count, stream_));
+  }
+  return DMM_OK;
+}
+
 dmm_status Pack::upload_state(const InstDesc& I, const double* x) {
-  const int64_t N = (int64_t)I.n + 2 * (int64_t)I.m;
-  DMM_TRY(ensure_stage(3 * N));
+  const int64_t n = I.n, m = I.m, N = n + 2 * m;
+  if (N > kDirectCopy && !page_locked(x)) {  // rounded on the host, straight to its place
+    XferLease xfer;
+    if (prec_ == DMM_FP64) {
+      DMM_CUDA(xfer->upload<double>(static_cast<double*>(cand_) + I.var0, x, n, stream_));
+      DMM_CUDA(xfer->upload<double>(static_cast<double*>(Xs_) + I.cls0, x + n, m, stream_));
+      DMM_CUDA(xfer->upload<double>(static_cast<double*>(Xl_) + I.cls0, x + n + m, m, stream_));
+    } else {
+      DMM_CUDA(xfer->upload<float>(static_cast<float*>(cand_) + I.var0, x, n, stream_));
+      DMM_CUDA(xfer->upload<float>(static_cast<float*>(Xs_) + I.cls0, x + n, m, stream_));
+      DMM_CUDA(xfer->upload<float>(static_cast<float*>(Xl_) + I.cls0, x + n + m, m, stream_));
+    }
+    return DMM_OK;
+  }
+  DMM_TRY(ensure_stage(N));
   DMM_CUDA(cudaMemcpyAsync(stage_, x, N * sizeof(double), cudaMemcpyHostToDevice, stream_));
   if (prec_ == DMM_FP64) {
     double* V = static_cast<double*>(cand_) + I.var0;
@@ -1039,24 +1075,26 @@ dmm_status Pack::get_state(int32_t idx, double* x, double* t) {
   DMM_TRY(flush_adds());
   const InstDesc& I = inst_h_[idx];
   const int64_t N = (int64_t)I.n + 2 * (int64_t)I.m;
-  DMM_TRY(ensure_stage(3 * N));
+  DMM_TRY(ensure_stage(N));
+  DMM_TRY(pinned());
+  InstCtrl* c = reinterpret_cast<InstCtrl*>(pinned_ + 64);
+  if (t) DMM_CUDA(cudaMemcpyAsync(c, ctrl_d_ + idx, sizeof(InstCtrl), cudaMemcpyDeviceToHost, stream_));
   if (prec_ == DMM_FP64) {
     k_get_state<double><<<blocks_for(N), kThreads, 0, stream_>>>(
         inst_d_, ctrl_d_, idx, static_cast<double*>(cand_), caps_.vars, static_cast<double*>(Xs_),
         static_cast<double*>(Xl_), static_cast<double*>(Cp_), static_cast<double*>(alpha_cm_), stage_);
+    DMM_CUDA(cudaGetLastError());
+    if (x) DMM_TRY(download_state(x, stage_, N));
   } else {
+    float* out = reinterpret_cast<float*>(stage_);
     k_get_state<float><<<blocks_for(N), kThreads, 0, stream_>>>(
         inst_d_, ctrl_d_, idx, static_cast<float*>(cand_), caps_.vars, static_cast<float*>(Xs_),
-        static_cast<float*>(Xl_), static_cast<float*>(Cp_), static_cast<float*>(alpha_cm_), stage_);
+        static_cast<float*>(Xl_), static_cast<float*>(Cp_), static_cast<float*>(alpha_cm_), out);
+    DMM_CUDA(cudaGetLastError());
+    if (x) DMM_TRY(download_state(x, out, N));
   }
-  DMM_CUDA(cudaGetLastError());
-  if (x) DMM_CUDA(cudaMemcpyAsync(x, stage_, N * sizeof(double), cudaMemcpyDeviceToHost, stream_));
-  DMM_CUDA(cudaStreamSynchronize(stream_));
-  if (t) {
-    InstCtrl c;
-    DMM_TRY(read_ctrl(idx, &c));
-    *t = c.t;
-  }
+  if (!x) DMM_CUDA(cudaStreamSynchronize(stream_));
+  if (t) *t = c->t;
   return DMM_OK;
 }
 
@@ -1502,7 +1540,7 @@ dmm_status Pack::launch_grid(int32_t nsteps) {
   const void* groups = gbuf_[kGrGroups];
   const void* blk = gbuf_[kGrBlk];
   void* epart = gbuf_[kGrEpart];
-  int* err = misc_d_ + 1;
+  int* err = error_d_;
   void* args[] = {view, &gr_tables_, &groups, &blk, &gr_layout_, &nsteps, &sync, &epart, &err};
   DMM_CUDA(cudaLaunchCooperativeKernel(fn, dim3((unsigned)gr_blocks_),
                                        dim3(fp64 ? kGridThreads64 : kGridThreads), args,
@@ -1853,7 +1891,7 @@ dmm_status Pack::launch_persist(int32_t nsteps) {
   static_assert(kMiscAcc2 * 4 + 2 * sizeof(StepAcc) <= kMiscInts * 4, "misc area");
   static_assert(kMiscInts - kMiscLaunch == kLaunchAreaInts, "launch area");
   unsigned int* bar = reinterpret_cast<unsigned int*>(misc_d_ + kMiscLaunch);
-  int* err = misc_d_ + 1;
+  int* err = error_d_;
   // a completed launch leaves its area zeroed (leave_launch); after an error or before the
   // first launch it is zeroed here
   if (!launch_area_clean_)
@@ -2064,12 +2102,12 @@ dmm_status Pack::launch_inst(int32_t nsteps) {
 
 dmm_status Pack::check_error() {
   int32_t e = 0;
-  DMM_CUDA(cudaMemcpyAsync(&e, misc_d_ + 1, sizeof(int32_t), cudaMemcpyDeviceToHost, stream_));
+  DMM_CUDA(cudaMemcpyAsync(&e, error_d_, sizeof(int32_t), cudaMemcpyDeviceToHost, stream_));
   DMM_CUDA(cudaStreamSynchronize(stream_));
   if (e) {
     launch_area_clean_ = false;
     gr_clean_ = false;
-    DMM_CUDA(cudaMemsetAsync(misc_d_ + 1, 0, sizeof(int32_t), stream_));  // reported once
+    DMM_CUDA(cudaMemsetAsync(error_d_, 0, sizeof(int32_t), stream_));  // reported once
     DMM_CUDA(cudaStreamSynchronize(stream_));
     set_error("grid barrier wait gave up in the cooperative step kernel");
     return DMM_ERR_CUDA;
@@ -2377,24 +2415,27 @@ dmm_status Pack::run(double wall_s, int64_t* steps_launched, bool* timed_out,
   DMM_CUDA(cudaSetDevice(dev_));
   *timed_out = false;
   if (steps_launched) *steps_launched = 0;
-  if (!pinned_) DMM_CUDA(pinned_alloc(&pinned_, 4 * sizeof(int32_t)));
+  DMM_TRY(pinned());
+  DMM_TRY(flush_adds());
   const auto t0 = std::chrono::steady_clock::now();
   auto elapsed = [&]() {
     return std::chrono::duration<double>(std::chrono::steady_clock::now() - t0).count();
   };
-  int32_t active = 0, tail0 = 0;
-  DMM_TRY(read_active(&active));
-  DMM_CUDA(cudaMemcpyAsync(&tail0, ring_tail_d_, sizeof(int32_t), cudaMemcpyDeviceToHost, stream_));
+  // status words before the run and after each chunk of steps (two in turn)
+  auto status = [&](int slot) { return pinned_ + 8 * slot; };
+  auto fetch = [&](int slot) -> dmm_status {
+    DMM_CUDA(cudaMemcpyAsync(status(slot), ring_tail_d_, kStatusInts * sizeof(int32_t),
+                             cudaMemcpyDeviceToHost, stream_));
+    return DMM_OK;
+  };
+  DMM_TRY(fetch(2));
   DMM_CUDA(cudaStreamSynchronize(stream_));
-  if (active <= 0) return DMM_OK;
+  const int32_t tail0 = status(2)[0];
+  if (status(2)[4] <= 0) return DMM_OK;
   const int32_t S = tun_.steps_per_graph * (cluster_only() ? kClusterChunk : 1);
-  // chunk k: S steps, then copies of the running count and the finished-ring tail
   auto chunk = [&](int slot) -> dmm_status {
     DMM_TRY(launch_steps(S));
-    DMM_CUDA(cudaMemcpyAsync(pinned_ + slot, active_d_, sizeof(int32_t), cudaMemcpyDeviceToHost,
-                             stream_));
-    DMM_CUDA(cudaMemcpyAsync(pinned_ + 2 + slot, ring_tail_d_, sizeof(int32_t),
-                             cudaMemcpyDeviceToHost, stream_));
+    DMM_TRY(fetch(slot));
     DMM_CUDA(cudaEventRecord(ev_[slot], stream_));
     if (steps_launched) *steps_launched += S;
     return DMM_OK;
@@ -2405,8 +2446,8 @@ dmm_status Pack::run(double wall_s, int64_t* steps_launched, bool* timed_out,
     const int nxt = cur ^ 1;
     DMM_TRY(chunk(nxt));
     DMM_CUDA(cudaEventSynchronize(ev_[cur]));
-    if (pinned_[cur] <= 0) break;
-    if (stop_after > 0 && pinned_[2 + cur] - tail0 >= stop_after) break;
+    if (status(cur)[4] <= 0 || status(cur)[5] != 0) break;
+    if (stop_after > 0 && status(cur)[0] - tail0 >= stop_after) break;
     if (wall_s > 0 && elapsed() > wall_s) {
       *timed_out = true;
       break;
@@ -2414,7 +2455,7 @@ dmm_status Pack::run(double wall_s, int64_t* steps_launched, bool* timed_out,
     cur = nxt;
   }
   DMM_CUDA(cudaStreamSynchronize(stream_));
-  return check_error();
+  return status(cur ^ 1)[5] ? check_error() : DMM_OK;
 }
 
 dmm_status Pack::resume(int32_t idx) {
@@ -2461,6 +2502,7 @@ dmm_status Pack::rhs(int32_t idx, const double* x, double* dxdt, int32_t* loc, d
   DMM_TRY(set_state(idx, x));
   const InstDesc& I = inst_h_[idx];
   const int64_t N = (int64_t)I.n + 2 * (int64_t)I.m;
+  DMM_TRY(ensure_stage(N));
   // tiles of this instance only
   std::vector<Tile> ct, vt;
   // the right-hand side runs the kernel-per-phase form with its own fixed tiles
@@ -2509,9 +2551,12 @@ dmm_status Pack::rhs(int32_t idx, const double* x, double* dxdt, int32_t* loc, d
   k_rhs_finish<<<1, kThreads, 0, stream_>>>(inst_d_, ctrl_d_, idx, epart_);
   DMM_CUDA(cudaGetLastError());
   DMM_TRY(upload_desc(idx));
-  DMM_CUDA(cudaMemcpyAsync(dxdt, stage_, N * sizeof(double), cudaMemcpyDeviceToHost, stream_));
   InstCtrl c;
-  DMM_TRY(read_ctrl(idx, &c));
+  DMM_TRY(pinned());
+  DMM_CUDA(cudaMemcpyAsync(pinned_ + 64, ctrl_d_ + idx, sizeof(InstCtrl), cudaMemcpyDeviceToHost,
+                           stream_));
+  DMM_TRY(download_state(dxdt, stage_, N));
+  std::memcpy(&c, pinned_ + 64, sizeof c);
   if (loc) *loc = c.loc;
   if (energy) *energy = c.energy;
   return DMM_OK;
@@ -2523,8 +2568,8 @@ dmm_status Pack::dostep(int32_t idx, const double* x, const double* dxdt, double
   const InstDesc& I = inst_h_[idx];
   const int64_t N = (int64_t)I.n + 2 * (int64_t)I.m;
   DMM_TRY(ensure_stage(3 * N));
-  DMM_CUDA(cudaMemcpyAsync(stage_, x, N * sizeof(double), cudaMemcpyHostToDevice, stream_));
-  DMM_CUDA(cudaMemcpyAsync(stage_ + N, dxdt, N * sizeof(double), cudaMemcpyHostToDevice, stream_));
+  DMM_TRY(upload_doubles(stage_, x, N));
+  DMM_TRY(upload_doubles(stage_ + N, dxdt, N));
   if (prec_ == DMM_FP64)
     k_dostep<double><<<blocks_for(N), kThreads, 0, stream_>>>(inst_d_, idx, unit_, stage_,
                                                               stage_ + N, h, stage_ + 2 * N);
@@ -2532,9 +2577,7 @@ dmm_status Pack::dostep(int32_t idx, const double* x, const double* dxdt, double
     k_dostep<float><<<blocks_for(N), kThreads, 0, stream_>>>(inst_d_, idx, unit_, stage_,
                                                              stage_ + N, h, stage_ + 2 * N);
   DMM_CUDA(cudaGetLastError());
-  DMM_CUDA(cudaMemcpyAsync(xo, stage_ + 2 * N, N * sizeof(double), cudaMemcpyDeviceToHost, stream_));
-  DMM_CUDA(cudaStreamSynchronize(stream_));
-  return DMM_OK;
+  return download_state(xo, stage_ + 2 * N, N);
 }
 
 dmm_status Pack::assignments(const std::vector<int32_t>& idx, std::vector<int8_t>* out) {

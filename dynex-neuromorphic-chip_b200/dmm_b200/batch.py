@@ -62,7 +62,7 @@ class Batch:
 
     def result(self, index: int):
         r = Report()
-        post = np.zeros(self.formulas[index].n, dtype=np.int8)
+        post = np.empty(self.formulas[index].n, dtype=np.int8)
         check(lib().dmm_batch_result(self._h, int(index), ctypes.byref(r),
                                      ptr(post, ctypes.c_int8)))
         return Result.from_report(r), post
@@ -79,7 +79,7 @@ class Batch:
 
     def state(self, index: int):
         f = self.formulas[index]
-        x = np.zeros(f.state_size(), dtype=np.float64)
+        x = np.empty(f.state_size(), dtype=np.float64)  # every entry is written
         t = ctypes.c_double()
         check(lib().dmm_batch_state(self._h, int(index), ptr(x, ctypes.c_double), ctypes.byref(t)))
         return x, t.value

@@ -109,7 +109,7 @@ class Instance:
                                               int(step)))
 
     def get_state(self):
-        x = np.zeros(self.n + 2 * self.m, dtype=np.float64)
+        x = np.empty(self.n + 2 * self.m, dtype=np.float64)  # every entry is written
         t = ctypes.c_double()
         check(lib().dmm_instance_get_state(self._h, ptr(x, ctypes.c_double), ctypes.byref(t)))
         return x, t.value
@@ -118,7 +118,7 @@ class Instance:
     def generate_dxdt(self, x):
         """dmm_generate_dxdt (dynex.cc:332): (dxdt, loc, energy).  Leaves the instance at x."""
         x = np.ascontiguousarray(x, dtype=np.float64)
-        d = np.zeros_like(x)
+        d = np.empty_like(x)
         loc = ctypes.c_int32()
         e = ctypes.c_double()
         check(lib().dmm_instance_rhs(self._h, ptr(x, ctypes.c_double), ptr(d, ctypes.c_double),
@@ -129,7 +129,7 @@ class Instance:
         """dmm_dostep (dynex.cc:301): x + h*dxdt with unit pin and clamps."""
         x = np.ascontiguousarray(x, dtype=np.float64)
         dxdt = np.ascontiguousarray(dxdt, dtype=np.float64)
-        o = np.zeros_like(x)
+        o = np.empty_like(x)
         check(lib().dmm_instance_dostep(self._h, ptr(x, ctypes.c_double),
                                         ptr(dxdt, ctypes.c_double), float(h),
                                         ptr(o, ctypes.c_double)))
@@ -156,7 +156,7 @@ class Instance:
     def assignment(self, pre: bool = True):
         """(pre, post): sign of V when the solution was found (0 for V == 0) and the
         reported assignment after the final step (+1/-1).  pre is None when unsolved."""
-        post = np.zeros(self.n, dtype=np.int8)
+        post = np.empty(self.n, dtype=np.int8)
         if pre:
             p = np.zeros(self.n, dtype=np.int8)
             st = lib().dmm_instance_assignment(self._h, ptr(p, ctypes.c_int8),
