@@ -26,8 +26,8 @@ LIB = os.path.join(LIB_DIR, "libdmm.so")
 CLI = os.path.join(BIN_DIR, "dynex")
 
 SOURCES = ["pack.cu", "cnf.cpp", "capi.cpp", "server.cpp", "noalloc.cu", "devmem.cpp", "cluster.cu",
-           "grid.cu", "hostpool.cpp"]
-HEADERS = ["hostpool.h", "dmm_admit.cuh", "dmm_device.cuh", "dmm_kernels.cuh", "dmm_step.cuh", "dmm_inst.cuh", "dmm_xpose.cuh", "dmm_xprep.cuh",
+           "grid.cu", "hostpool.cpp", "stream.cu"]
+HEADERS = ["dmm_stream.cuh", "hostpool.h", "dmm_admit.cuh", "dmm_device.cuh", "dmm_kernels.cuh", "dmm_step.cuh", "dmm_inst.cuh", "dmm_xpose.cuh", "dmm_xprep.cuh",
            "dmm_cluster.cuh", "dmm_cluster.h", "dmm_grid.cuh",
            "dmm_grid.h", "dmm_gridprep.cuh",
            "dmm_pack.h", "devmem.h"]

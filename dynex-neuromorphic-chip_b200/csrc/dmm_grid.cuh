@@ -58,7 +58,6 @@ inline GridLayout grid_layout(const GridCaps& c, int tsize, bool general,
   L.dv = take(tsize * c.tv);
   L.vend = take(4 * (c.tv + 1));
   L.unit = take(general ? c.tv : 0);
-  L.pinfo = take(4 * c.B);
   L.rank = take(tsize == 8 ? 16 * kRankMax * (kGridThreads64 / 32) : 0);
   L.xs = L.xl = L.cp = L.lit = L.spos = L.off = L.wdst = L.row = L.csr = L.snd = 0;
   if (resident >= 1) {
@@ -73,7 +72,7 @@ inline GridLayout grid_layout(const GridCaps& c, int tsize, bool general,
     L.spos = take(2 * c.ts);
     L.off = take(general ? 4 * (c.tc + 1) : 0);
     L.wdst = take(4 * c.wd);
-    L.snd = take(4 * c.snd);
+    L.snd = take((4 + 2 * (16 / tsize)) * c.snd);
   }
   L.total = o;
   return L;
@@ -126,16 +125,16 @@ __device__ __forceinline__ void st_relaxed(float* p, float v) {
 __device__ __forceinline__ void st_relaxed(double* p, double v) {
   asm volatile("st.relaxed.gpu.global.f64 [%0], %1;" ::"l"(p), "d"(v));
 }
-// Whether the first `used` entries (of 16 / sizeof(T)) of a word are set.
+// Whether all entries of a word are set.
 template <class T>
-__device__ __forceinline__ bool word_set(const int4& v, int used) {
+__device__ __forceinline__ bool word_set(const int4& v) {
   if constexpr (sizeof(T) == 4) {
     const int u = (int)Unset<unsigned int>::bits();
-    return v.x != u && (v.y != u || used < 2) && (v.z != u || used < 3) && (v.w != u || used < 4);
+    return v.x != u && v.y != u && v.z != u && v.w != u;
   } else {
     const int lo = (int)(unsigned int)Unset<unsigned long long>::bits();
     const int hi = (int)(Unset<unsigned long long>::bits() >> 32);
-    return (v.x != lo || v.y != hi) && (v.z != lo || v.w != hi || used < 2);
+    return (v.x != lo || v.y != hi) && (v.z != lo || v.w != hi);
   }
 }
 template <class T>
@@ -152,13 +151,11 @@ __device__ __forceinline__ int4 unset_word() {
 
 constexpr int kGridPollLimit = 1 << 21;  // polls of an exchange word (about a second)
 
-// Takes up to N words of p[q0 + r step], r < N (those below n; the last one holds `last`
-// entries): polls all of them together until their entries are set, then unsets them.
-// Clears ok when the limit runs out (and does not poll on once it is clear).
+// Takes up to N words of p[q0 + r step], r < N (those below n): polls all of them together until
+// their entries are set, then unsets them.  Clears ok when the limit runs out (and does not
+// poll on once it is clear).
 template <class T, int N>
-__device__ __forceinline__ void take_words(int4* p, int q0, int step, int n, int last, int4 (&v)[N],
-                                           bool& ok) {
-  constexpr int kw = 16 / (int)sizeof(T);
+__device__ __forceinline__ void take_words(int4* p, int q0, int step, int n, int4 (&v)[N], bool& ok) {
   int it = ok ? 0 : kGridPollLimit;
   for (;;) {
     bool set = true;
@@ -167,8 +164,7 @@ __device__ __forceinline__ void take_words(int4* p, int q0, int step, int n, int
       if (q0 + r * step < n) v[r] = ld_relaxed4(p + q0 + r * step);
 #pragma unroll
     for (int r = 0; r < N; r++)
-      if (q0 + r * step < n)
-        set = set && word_set<T>(v[r], q0 + r * step == n - 1 ? last : kw);
+      if (q0 + r * step < n) set = set && word_set<T>(v[r]);
     if (set) break;
     if (++it >= kGridPollLimit) {
       ok = false;
@@ -182,7 +178,7 @@ __device__ __forceinline__ void take_words(int4* p, int q0, int step, int n, int
 
 // A block's copy of the control state of its formula.
 struct GridCtrl {
-  int done, step, set, kcur, pending, best_loc, sol_k;
+  int done, step, set, kcur, pending, best_loc, sol_k, loc, vfail;
   double h, t, t_rhs, best_t, solved_t;
 };
 
@@ -195,7 +191,8 @@ struct GridPtrs {
   const int32_t *woff, *boff, *coff;
   const int16_t* llit;
   const uint16_t *spos, *rows, *idx;
-  const uint32_t *wdst, *snd;
+  const uint16_t* ids;
+  const uint32_t *wdst, *sdst;
   int in_place, dcnt, nsend;
 };
 
@@ -258,7 +255,6 @@ __global__ void __launch_bounds__(sizeof(T) == 8 ? kGridThreads64 : kGridThreads
   T* const s_dv = reinterpret_cast<T*>(gr_smem + LY.dv);
   int* const s_vend = reinterpret_cast<int*>(gr_smem + LY.vend);
   int8_t* const s_unit = reinterpret_cast<int8_t*>(gr_smem + LY.unit);
-  int* const s_to = reinterpret_cast<int*>(gr_smem + LY.pinfo);  // inbox place - send place
   double* const s_rank = reinterpret_cast<double*>(gr_smem + LY.rank);
   const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
 
@@ -292,20 +288,21 @@ __global__ void __launch_bounds__(sizeof(T) == 8 ? kGridThreads64 : kGridThreads
   const int vend0 = v0 > 0 ? vend[v0 - 1] : 0;
   if (tid == 0) {
     const int2 di = tb.dinfo[g.o_blk + b];
-    const int2* const pinfo = tb.pinfo + g.o_bb + (int64_t)b * (B + 1);
+    const int2 si = tb.sinfo[g.o_blk + b];
     const int32_t* const woff = tb.woff + g.o_ct + b * g.kc;
     sp.ux = static_cast<T*>(tb.ux) + g.o_ux;
     sp.inbox = static_cast<T*>(tb.inbox) + g.o_list;
     sp.in_place = di.x;
     sp.dcnt = di.y;
-    sp.nsend = pinfo[B].x - pinfo[0].x;
+    sp.nsend = si.y;
     sp.woff = woff;
     sp.boff = tb.boff + g.o_vt + b * g.kv;
     sp.llit = tb.llit + g.o_slot + s0;
     sp.spos = tb.spos + g.o_slot + s0;
     sp.wdst = tb.wdst + g.o_word + woff[0];
     sp.rows = tb.rows + g.o_row + (int64_t)b * g.kv * g.TVr * 32;
-    sp.snd = tb.sends + g.o_push + pinfo[0].x;
+    sp.sdst = tb.sdst + g.o_push + si.x;
+    sp.ids = tb.ids + (g.o_push + si.x) * kw;
     sp.idx = tb.idx + g.o_slot + vend0;  // from the block's first CSR entry
     sp.Xs = P.Xs + I.cls0 + c0;
     sp.Xl = P.Xl + I.cls0 + c0;
@@ -320,13 +317,11 @@ __global__ void __launch_bounds__(sizeof(T) == 8 ? kGridThreads64 : kGridThreads
     const T* V0 = P.cand + (int64_t)(lc.set * kTrials + lc.kcur) * P.var_cap + I.var0;
     const int32_t* dl = tb.dlist + g.o_list + sp.in_place;
     const int dcnt = sp.dcnt;
-    for (int k = tid; k < dcnt; k += NT) sV[k] = V0[dl[k]];
+    for (int k = tid; k < dcnt; k += NT) sV[k] = dl[k] >= 0 ? V0[dl[k]] : T(0);
     for (int i = tid; i < nv; i += NT) s_cur[i] = V0[v0 + i];
     for (int i = tid; i <= nv; i += NT) s_vend[i] = (i > 0 ? vend[v0 + i - 1] : vend0) - vend0;
     if (GENERAL)
       for (int i = tid; i < nv; i += NT) s_unit[i] = P.unit[I.var0 + v0 + i];
-    const int2* const pinfo = tb.pinfo + g.o_bb + (int64_t)b * (B + 1);
-    for (int c = tid; c < B; c += NT) s_to[c] = pinfo[c].y - (pinfo[c].x - pinfo[0].x);
     // no entry of the areas may look unset (the padding of chunks is sent too)
     for (int q = tid; q < (LY.cur - LY.raw) / 16; q += NT)
       reinterpret_cast<int4*>(gr_smem + LY.raw)[q] = make_int4(0, 0, 0, 0);
@@ -362,7 +357,8 @@ __global__ void __launch_bounds__(sizeof(T) == 8 ? kGridThreads64 : kGridThreads
         bring(LY.lit, sp.llit, ns);
         bring(LY.spos, sp.spos, ns);
         bring(LY.wdst, sp.wdst, sp.woff[g.kc] - sp.woff[0]);
-        bring(LY.snd, sp.snd, sp.nsend);
+        bring(LY.snd, sp.sdst, sp.nsend);
+        bring(LY.snd + 4 * sp.nsend, sp.ids, kw * sp.nsend);
         if (GENERAL)
           for (int c = tid; c <= c1 - c0; c += NT) off_s[c] = grid_slot(g, P.coff, c0 + c) - s0;
       }
@@ -594,7 +590,7 @@ __global__ void __launch_bounds__(sizeof(T) == 8 ? kGridThreads64 : kGridThreads
         bool ok = true;
         for (int q0 = tid; q0 < nw; q0 += 4 * NT) {
           int4 v[4];
-          take_words<T>(src, q0, NT, nw, kw, v, ok);
+          take_words<T>(src, q0, NT, nw, v, ok);
 #pragma unroll
           for (int r = 0; r < 4; r++)
             if (q0 + r * NT < nw) dst[q0 + r * NT] = v[r];
@@ -720,18 +716,37 @@ __global__ void __launch_bounds__(sizeof(T) == 8 ? kGridThreads64 : kGridThreads
     }
     // dV to the inboxes of the blocks that read it
     {
-      const uint32_t* const snd = RES == 2 ? reinterpret_cast<const uint32_t*>(gr_smem + LY.snd) : sp.snd;
-      T* const in = sp.inbox + (s & 1) * tb.inbox_len;
       const int nsend = sp.nsend;
+      const uint32_t* const sdst =
+          RES == 2 ? reinterpret_cast<const uint32_t*>(gr_smem + LY.snd) : sp.sdst;
+      const uint16_t* const ids =
+          RES == 2 ? reinterpret_cast<const uint16_t*>(gr_smem + LY.snd + 4 * nsend) : sp.ids;
+      int4* const in = reinterpret_cast<int4*>(sp.inbox + (s & 1) * tb.inbox_len);
       for (int q0 = tid; q0 < nsend; q0 += 4 * NT) {
-        uint32_t e[4];
+        uint32_t at[4], e[4][kw / 2];  // two 16-bit variables per word
+#pragma unroll
+        for (int r = 0; r < 4; r++) {
+          const int q = q0 + r * NT;
+          if (q < nsend) {
+            at[r] = sdst[q];
+            // (4-byte loads: with RES the lists start at any multiple of 4 bytes)
+#pragma unroll
+            for (int k = 0; k < kw / 2; k++)
+              e[r][k] = reinterpret_cast<const uint32_t*>(ids)[q * (kw / 2) + k];
+          }
+        }
 #pragma unroll
         for (int r = 0; r < 4; r++)
-          if (q0 + r * NT < nsend) e[r] = snd[q0 + r * NT];
+          if (q0 + r * NT < nsend) {
+            union {
+              T v[kw];
+              int4 q;
+            } u;
 #pragma unroll
-        for (int r = 0; r < 4; r++)
-          if (q0 + r * NT < nsend)
-            st_relaxed(in + s_to[e[r] >> 16] + q0 + r * NT, s_dv[e[r] & 0xffffu]);
+            for (int k = 0; k < kw; k++)
+              u.v[k] = s_dv[(e[r][k >> 1] >> (16 * (k & 1))) & 0xffffu];
+            st_relaxed4(in + at[r], u.q);
+          }
       }
     }
     trace_stamp(P, s, 7);
@@ -739,12 +754,12 @@ __global__ void __launch_bounds__(sizeof(T) == 8 ? kGridThreads64 : kGridThreads
     // ---- F: the last warp waits for the reports of all blocks, the others take the words of
     // the inbox meanwhile
     constexpr int kHeld = 4, NI = NT - 32;
-    const int dcnt = sp.dcnt, nin = (dcnt + kw - 1) / kw, last = dcnt - kw * (nin - 1);
+    const int nin = sp.dcnt / kw;  // whole words
     int4 held[kHeld];
     int4* const in_w = reinterpret_cast<int4*>(sp.inbox + (s & 1) * tb.inbox_len + sp.in_place);
     bool in_ok = true;
     if (w != W - 1) {
-      if (tid < nin) take_words<T>(in_w, tid, NI, nin, last, held, in_ok);
+      if (tid < nin) take_words<T>(in_w, tid, NI, nin, held, in_ok);
     } else if (lane == 0) {
       unsigned long long a;
       int ok = 1;
@@ -795,7 +810,7 @@ __global__ void __launch_bounds__(sizeof(T) == 8 ? kGridThreads64 : kGridThreads
       for (int r = 0; r < kHeld; r++)
         if (tid + r * NI < nin) apply(tid + r * NI, held[r]);
       for (int q0 = tid + kHeld * NI; q0 < nin; q0 += kHeld * NI) {
-        take_words<T>(in_w, q0, NI, nin, last, held, in_ok);
+        take_words<T>(in_w, q0, NI, nin, held, in_ok);
 #pragma unroll
         for (int r = 0; r < kHeld; r++)
           if (q0 + r * NI < nin) apply(q0 + r * NI, held[r]);

@@ -21,6 +21,8 @@ constexpr int kGridMaxDistinct = 32767;   // 16-bit tile-local literals
 struct GridGroup {
   int32_t inst, blk0, B, kc, kv, TC, TV, TVr;  // TVr: TV rounded up to 32 (table rows)
   int32_t nct, nvt;                            // B * kc, B * kv
+  int32_t lt, NL, list0;                       // clause tiles per variable list, lists, first one
+  int32_t pad;                                 // entries that chunks of ux are padded to
   int32_t n, m, L, k3;
   int64_t var0, cls0, slot0;
   int64_t o_pair, o_blk, o_ct, o_vt, o_list, o_slot, o_ux, o_word, o_row, o_push, o_bb;
@@ -29,17 +31,19 @@ struct GridGroup {
 // Table arrays of all groups.
 struct GridTables {
   // built at commit, read by the steps
-  int32_t* dlist;   // [o_list] distinct variables of each block's clauses, ascending
-  int2* dinfo;      // [o_blk + b] start and count in dlist and in the inbox
-  int16_t* llit;    // [o_slot + s] block-local literal, +-(1 + place in the list)
+  int32_t* dlist;   // [o_list] distinct variables of each list, ascending; the part of every
+                    // owning block is padded to whole 16-byte words of voltages (with -1)
+  int2* dinfo;      // [o_blk + l] start and count of list l in dlist and in the inbox
+  int16_t* llit;    // [o_slot + s] list-local literal, +-(1 + place in the list)
   uint16_t* spos;   // [o_slot + s] place in the tile's staging area
   uint32_t* wdst;   // [o_word + w] 16-byte word of ux each staging word goes to
   int32_t* woff;    // [o_ct + t] first staging word of each clause tile (nct + 1 of them)
   int32_t* boff;    // [o_vt + v] start of each variable tile's bucket in ux (nvt + 1)
   uint16_t* rows;   // [o_row] bucket places of each variable's first 32 contributions
   uint16_t* idx;    // [o_slot + j] bucket place of the contribution in CSR position j
-  int2* pinfo;      // [o_bb + b (B + 1) + c] start in sends and inbox place of block c's chunk
-  uint32_t* sends;  // [o_push] block-local variable, destination block << 16
+  int2* sinfo;      // [o_blk + b] start and count of block b's send words
+  uint16_t* ids;    // [(o_push + word) kw] block-local variables of a send word
+  uint32_t* sdst;   // [o_push + word] inbox word it goes to
   // exchanged within a step, each twice (steps of even and odd number): unset entries hold a
   // value no arithmetic gives
   void* ux;         // [2 o_ux] contributions, bucket after bucket
@@ -47,12 +51,14 @@ struct GridTables {
   int64_t ux_len, inbox_len;  // elements of one copy
   // scratch of the build
   int32_t *cnt, *sb, *bt;       // [o_pair]
-  int32_t *st, *dcnt, *dlo;     // [o_ct], [o_blk], [o_bb]
+  int32_t *st, *dcnt;           // [o_ct], [o_blk]
+  int32_t *dlo, *dlp, *poff;    // [o_bb]: variables below a block, padded; chunk's send words
+  int32_t *btot, *ptot;         // [o_vt], [o_blk]
   int32_t* out;                 // [8 x group]
 };
 
 // Results of the build, per group: [0] 0 ok, else which limit failed; [1] largest distinct
-// list, [2] largest staging area, [3] largest bucket, [4] largest send list (entries), [5]
+// list, [2] largest staging area, [3] largest bucket, [4] largest send list (words), [5]
 // largest literal-slot count of a block.
 constexpr int kGridOut = 8;
 
@@ -81,10 +87,23 @@ inline int grid_smem(const GridCaps& c, bool fp64, bool general, int resident) {
 const void* grid_kernel(bool fp64, bool general, int resident);
 // Queues the marking of all exchange entries as unset.
 cudaError_t grid_unset(const GridTables& t, bool fp64, cudaStream_t s);
-// Queues the table build of all groups (blk_group: group of every block of the grid).
-cudaError_t grid_build(const GridGroup* groups, const int32_t* blk_group, int ngroups,
-                       int nblocks, int max_n, int max_nvt, const int32_t* lit,
+// Queues the table build of all groups (list_group: group of every list).
+cudaError_t grid_build(const GridGroup* groups, const int32_t* list_group, int ngroups,
+                       int nlists, int max_n, int max_nvt, int max_rows, const int32_t* lit,
                        const int32_t* upos, const int32_t* vend, const int32_t* coff,
                        const GridTables& t, bool fp64, cudaStream_t s);
+
+// ---- streaming form (dmm_stream.cuh)
+constexpr int kStreamThreads = 1024;   // block size
+constexpr int kStreamThreads64 = 512;  // ... in FP64
+constexpr int kStreamSmemMax = 222 * 1024;
+struct StreamLayout {
+  int v0, v1, stage;  // A: two voltage lists (one in use, one arriving), staging area
+  int b0, b1;         // B: two buckets, each behind one padding word
+  int rank;           // FP64: ranking areas
+  int total;          // C: the block's voltages, from 0
+};
+StreamLayout stream_shape(int dl, int st, int bk, int tv, bool fp64);
+const void* stream_kernel(bool fp64, bool general);
 
 }  // namespace dmm

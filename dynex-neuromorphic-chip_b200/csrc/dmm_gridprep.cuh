@@ -1,11 +1,14 @@
 // Device construction of the resident grid form's tables (dmm_grid.cuh), all groups at once.
 //
-//   k_grid_count  (one block per block of the grid) rank of every slot within its chunk
-//                 (clause tile t, variable tile v), chunk sizes, staging offsets; the block's
-//                 number of distinct variables and how many lie below each block's variables.
-//   k_grid_scan   (one block per group) offsets over tiles and blocks, the limits.
-//   k_grid_fill   (one block per block of the grid) variable lists, local literals, staging
-//                 places and destinations, bucket places in variable-major order, send lists.
+//   k_grid_count  (one block per variable list, i.e. per block of the grid form or clause tile
+//                 of the streaming form) rank of every slot within its chunk (clause tile t,
+//                 variable tile v), chunk sizes, staging offsets; the list's number of distinct
+//                 variables and how many lie below each block's variables.
+//   k_grid_rows   (one block per variable tile and per sending block) offsets of the chunks
+//                 inside a bucket and inside a send list.
+//   k_grid_scan   (one block per group) offsets over tiles, lists and blocks, the limits.
+//   k_grid_fill   (as k_grid_count) variable lists, local literals, staging places and
+//                 destinations, bucket places in variable-major order, send lists.
 //
 // Slot order inside a chunk is arbitrary: both sides use the same rank, and a variable's
 // contributions are summed in CSR order through their bucket places.
@@ -24,23 +27,40 @@ __device__ __forceinline__ int grid_slot(const GridGroup& g, const int32_t* coff
   return g.k3 ? 3 * c : c < g.m ? coff[g.cls0 + c] : g.L;
 }
 
+// Exclusive prefix sums over i < count by the block: put(i, sum of get(0..i-1)); returns the
+// total.
+template <int NT, class Get, class Put>
+__device__ int block_prefix(int count, int* wsum, Get get, Put put) {
+  int at = 0;
+  for (int i0 = 0; i0 < count; i0 += NT) {
+    const int i = i0 + threadIdx.x;
+    const int v = i < count ? get(i) : 0;
+    int tot;
+    const int ex = block_exscan<NT>(v, wsum, &tot);
+    if (i < count) put(i, at + ex);
+    at += tot;
+  }
+  return at;
+}
+
 __global__ void __launch_bounds__(kGridPrepThreads)
-    k_grid_count(const GridGroup* __restrict__ groups, const int32_t* __restrict__ blk_group,
+    k_grid_count(const GridGroup* __restrict__ groups, const int32_t* __restrict__ list_group,
                  const int32_t* __restrict__ lit_all, const int32_t* __restrict__ coff, GridTables t,
                  int RW, int kw) {
   constexpr int NT = kGridPrepThreads;
   extern __shared__ __align__(16) int gp_smem[];
   __shared__ int wsum[32];
-  const GridGroup g = groups[blk_group[blockIdx.x]];
-  const int b = blockIdx.x - g.blk0, nvt = g.nvt;
+  const GridGroup g = groups[list_group[blockIdx.x]];
+  const int b = blockIdx.x - g.list0, nvt = g.nvt;
   const int32_t* lit = lit_all + g.slot0;
   int* c_s = gp_smem;
   unsigned* bits = reinterpret_cast<unsigned*>(gp_smem + nvt);
   int* wpre = gp_smem + nvt + RW;
-  for (int i = 0; i < g.kc; i++) {
-    const int ct = b * g.kc + i;
+  for (int i = 0; i < g.lt; i++) {
+    const int ct = b * g.lt + i;
     const int s_lo = grid_slot(g, coff, min(g.m, ct * g.TC)),
               s_hi = grid_slot(g, coff, min(g.m, (ct + 1) * g.TC));
+    __syncthreads();
     for (int v = threadIdx.x; v < nvt; v += NT) c_s[v] = 0;
     __syncthreads();
     for (int s = s_lo + threadIdx.x; s < s_hi; s += NT)
@@ -49,7 +69,7 @@ __global__ void __launch_bounds__(kGridPrepThreads)
     int at = 0;
     for (int v0 = 0; v0 < nvt; v0 += NT) {
       const int v = v0 + threadIdx.x;
-      const int c = v < nvt ? c_s[v] : 0, p = (c + kw - 1) / kw * kw;
+      const int c = v < nvt ? c_s[v] : 0, p = (c + g.pad - 1) / g.pad * g.pad;
       int tot;
       const int ex = block_exscan<NT>(p, wsum, &tot);
       if (v < nvt) {
@@ -61,8 +81,8 @@ __global__ void __launch_bounds__(kGridPrepThreads)
     if (threadIdx.x == 0) t.st[g.o_ct + ct] = at;
   }
   // distinct variables, and those below each block's first variable
-  const int s_lo = grid_slot(g, coff, min(g.m, b * g.kc * g.TC)),
-            s_hi = grid_slot(g, coff, min(g.m, (b + 1) * g.kc * g.TC));
+  const int s_lo = grid_slot(g, coff, min(g.m, b * g.lt * g.TC)),
+            s_hi = grid_slot(g, coff, min(g.m, (b + 1) * g.lt * g.TC));
   const int TVb = g.TV * g.kv;
   int32_t* dlo = t.dlo + g.o_bb + (int64_t)b * (g.B + 1);
   int before = 0;
@@ -79,71 +99,86 @@ __global__ void __launch_bounds__(kGridPrepThreads)
   for (int c = threadIdx.x; c <= g.B; c += NT)
     if (c == g.B || (int64_t)c * TVb >= ((int64_t)(g.n + 32 * RW - 1) / (32 * RW)) * 32 * RW)
       dlo[c] = before;
-  if (threadIdx.x == 0) t.dcnt[g.o_blk + b] = before;
+  __syncthreads();
+  // places: each owning block's variables padded to whole words
+  int32_t* dlp = t.dlp + g.o_bb + (int64_t)b * (g.B + 1);
+  const int padded = block_prefix<NT>(
+      g.B, wsum, [&](int c) { return (dlo[c + 1] - dlo[c] + kw - 1) / kw * kw; },
+      [&](int c, int at) { dlp[c] = at; });
+  if (threadIdx.x == 0) {
+    dlp[g.B] = padded;
+    t.dcnt[g.o_blk + b] = padded;
+  }
+}
+
+constexpr int kGridRowThreads = 256;
+__global__ void __launch_bounds__(kGridRowThreads)
+    k_grid_rows(const GridGroup* __restrict__ groups, GridTables t, int kw) {
+  __shared__ int wsum[32];
+  const GridGroup& g = groups[blockIdx.y];
+  const int nct = g.nct, nvt = g.nvt, r = blockIdx.x;
+  if (r < nvt) {
+    const int tot = block_prefix<kGridRowThreads>(
+        nct, wsum,
+        [&](int c) { return (t.cnt[g.o_pair + (int64_t)c * nvt + r] + g.pad - 1) / g.pad * g.pad; },
+        [&](int c, int at) { t.bt[g.o_pair + (int64_t)r * nct + c] = at; });
+    if (threadIdx.x == 0) t.btot[g.o_vt + r] = tot;
+  } else if (r < nvt + g.B) {
+    const int b = r - nvt;
+    const int tot = block_prefix<kGridRowThreads>(
+        g.NL, wsum,
+        [&](int l) {
+          const int32_t* dlp = t.dlp + g.o_bb + (int64_t)l * (g.B + 1) + b;
+          return (dlp[1] - dlp[0]) / kw;
+        },
+        [&](int l, int at) { t.poff[g.o_bb + (int64_t)l * (g.B + 1) + b] = at; });
+    if (threadIdx.x == 0) t.ptot[g.o_blk + b] = tot;
+  }
 }
 
 __global__ void __launch_bounds__(kGridPrepThreads)
     k_grid_scan(const GridGroup* __restrict__ groups, const int32_t* __restrict__ coff,
                 const int32_t* __restrict__ vend, GridTables t, int kw) {
   constexpr int NT = kGridPrepThreads;
-  __shared__ int s_bad, s_max[8], s_tot[1024];
+  __shared__ int wsum[32], s_bad, s_max[8];
   const GridGroup g = groups[blockIdx.x];
-  const int nct = g.nct, nvt = g.nvt, B = g.B;
+  const int nct = g.nct, nvt = g.nvt, B = g.B, NL = g.NL;
   if (threadIdx.x < 8) s_max[threadIdx.x] = 0;
   if (threadIdx.x == 0) s_bad = 0;
   __syncthreads();
+  block_prefix<NT>(
+      NL, wsum, [&](int l) { return (t.dcnt[g.o_blk + l] + 3) & ~3; },
+      [&](int l, int at) {
+        const int d = t.dcnt[g.o_blk + l];
+        t.dinfo[g.o_blk + l] = make_int2(at, d);
+        atomicMax(&s_max[1], (d + 3) & ~3);
+      });
+  const int words = block_prefix<NT>(
+      nct, wsum, [&](int c) { return t.st[g.o_ct + c] / kw; },
+      [&](int c, int at) {
+        t.woff[g.o_ct + c] = at;
+        atomicMax(&s_max[2], t.st[g.o_ct + c]);
+      });
+  const int uxn = block_prefix<NT>(
+      nvt, wsum, [&](int v) { return t.btot[g.o_vt + v]; },
+      [&](int v, int at) {
+        t.boff[g.o_vt + v] = at;
+        atomicMax(&s_max[3], t.btot[g.o_vt + v]);
+      });
   if (threadIdx.x == 0) {
-    int at = 0;
-    for (int b = 0; b < B; b++) {
-      const int d = t.dcnt[g.o_blk + b];
-      t.dinfo[g.o_blk + b] = make_int2(at, d);
-      at += (d + 3) & ~3;
-      s_max[1] = max(s_max[1], (d + 3) & ~3);
-    }
-    if (s_max[1] > kGridMaxDistinct) atomicExch(&s_bad, 1);
-  } else if (threadIdx.x == 32) {
-    int at = 0, mx = 0;
-    for (int c = 0; c < nct; c++) {
-      const int st = t.st[g.o_ct + c];
-      t.woff[g.o_ct + c] = at;
-      at += st / kw;
-      mx = max(mx, st);
-    }
-    t.woff[g.o_ct + nct] = at;
-    s_max[2] = mx;
-    if (mx > 65535) atomicExch(&s_bad, 2);
+    t.woff[g.o_ct + nct] = words;
+    t.boff[g.o_vt + nvt] = uxn;
+    if (s_max[1] > kGridMaxDistinct) s_bad = 1;
+    else if (s_max[2] > 65535) s_bad = 2;
+    else if (s_max[3] + kw > 65535) s_bad = 3;
   }
-  // chunk offsets inside each bucket: one thread per variable tile; send lists: one per block
-  for (int v = threadIdx.x; v < nvt; v += NT) {
-    int at = 0;
-    for (int c = 0; c < nct; c++) {
-      t.bt[g.o_pair + (int64_t)v * nct + c] = at;
-      at += (t.cnt[g.o_pair + (int64_t)c * nvt + v] + kw - 1) / kw * kw;
-    }
-    s_tot[v] = at;
-    atomicMax(&s_max[3], at);
-    if (at + kw > 65535) atomicExch(&s_bad, 3);
-  }
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    int at = 0;
-    for (int v = 0; v < nvt; v++) {
-      t.boff[g.o_vt + v] = at;
-      at += s_tot[v];
-    }
-    t.boff[g.o_vt + nvt] = at;
-  }
+  // send words of all blocks, one block after another
+  block_prefix<NT>(
+      B, wsum, [&](int b) { return t.ptot[g.o_blk + b]; },
+      [&](int b, int at) { t.sinfo[g.o_blk + b] = make_int2(at, t.ptot[g.o_blk + b]); });
   __syncthreads();
   for (int b = threadIdx.x; b < B; b += NT) {
-    int at = 0;
-    for (int c = 0; c < B; c++) {
-      const int32_t* dlo = t.dlo + g.o_bb + (int64_t)c * (B + 1);
-      t.pinfo[g.o_bb + (int64_t)b * (B + 1) + c] = make_int2(at, t.dinfo[g.o_blk + c].x + dlo[b]);
-      at += dlo[b + 1] - dlo[b];
-    }
-    t.pinfo[g.o_bb + (int64_t)b * (B + 1) + B] = make_int2(at, 0);
-    s_tot[b] = at;
-    atomicMax(&s_max[4], at);
+    atomicMax(&s_max[4], t.ptot[g.o_blk + b]);
     const int TVb = g.TV * g.kv, v0 = min(g.n, b * TVb), v1 = min(g.n, v0 + TVb);
     atomicMax(&s_max[7], (v1 > 0 ? vend[g.var0 + v1 - 1] : 0) - (v0 > 0 ? vend[g.var0 + v0 - 1] : 0));
     const int TCb = g.TC * g.kc;
@@ -152,41 +187,31 @@ __global__ void __launch_bounds__(kGridPrepThreads)
     atomicMax(&s_max[6], t.woff[g.o_ct + (b + 1) * g.kc] - t.woff[g.o_ct + b * g.kc]);
   }
   __syncthreads();
-  if (threadIdx.x == 0) {  // the send lists of all blocks, one after another
-    int base = 0;
-    for (int b = 0; b < B; b++) {
-      t.st[g.o_ct + b] = base;  // (the staging sizes are no longer needed)
-      base += s_tot[b];
-    }
-  }
-  __syncthreads();
-  for (int q = threadIdx.x; q < B * (B + 1); q += NT)
-    t.pinfo[g.o_bb + q].x += t.st[g.o_ct + q / (B + 1)];
   if (threadIdx.x < 8) t.out[kGridOut * blockIdx.x + threadIdx.x] = threadIdx.x == 0 ? s_bad : s_max[threadIdx.x];
 }
 
 // ROW64: rows as the FP64 sums read them (32 variables side by side), else as the FP32 sums do.
 template <bool ROW64>
 __global__ void __launch_bounds__(kGridPrepThreads)
-    k_grid_fill(const GridGroup* __restrict__ groups, const int32_t* __restrict__ blk_group,
+    k_grid_fill(const GridGroup* __restrict__ groups, const int32_t* __restrict__ list_group,
                 const int32_t* __restrict__ lit_all, const int32_t* __restrict__ upos_all,
                 const int32_t* __restrict__ vend_all, const int32_t* __restrict__ coff, GridTables t,
                 int RW, int kw) {
   constexpr int NT = kGridPrepThreads;
   extern __shared__ __align__(16) int gp_smem[];
   __shared__ int wsum[32];
-  const int gi = blk_group[blockIdx.x];
+  const int gi = list_group[blockIdx.x];
   const GridGroup g = groups[gi];
   if (t.out[kGridOut * gi] != 0) return;  // a limit failed: the tables are not used
-  const int b = blockIdx.x - g.blk0, nvt = g.nvt, nct = g.nct;
+  const int b = blockIdx.x - g.list0, nvt = g.nvt, nct = g.nct;
   const int32_t* lit = lit_all + g.slot0;
   const int32_t* upos = upos_all + g.slot0;
   const int32_t* vend = vend_all + g.var0;
   int* s_sb = gp_smem;  // [nvt] staging offset, then the bucket offset of this tile's chunk
   unsigned* bits = reinterpret_cast<unsigned*>(gp_smem + nvt);
   int* wpre = gp_smem + nvt + RW;
-  for (int i = 0; i < g.kc; i++) {
-    const int ct = b * g.kc + i;
+  for (int i = 0; i < g.lt; i++) {
+    const int ct = b * g.lt + i;
     const int s_lo = grid_slot(g, coff, min(g.m, ct * g.TC)),
               s_hi = grid_slot(g, coff, min(g.m, (ct + 1) * g.TC));
     __syncthreads();
@@ -209,7 +234,7 @@ __global__ void __launch_bounds__(kGridPrepThreads)
     // destinations of the staging area's words
     const int w0 = t.woff[g.o_ct + ct];
     for (int v = threadIdx.x >> 5; v < nvt; v += NT / 32) {
-      const int nw = (t.cnt[g.o_pair + (int64_t)ct * nvt + v] + kw - 1) / kw;
+      const int nw = (t.cnt[g.o_pair + (int64_t)ct * nvt + v] + g.pad - 1) / g.pad * g.pad / kw;
       const int d0 = (t.boff[g.o_vt + v] + t.bt[g.o_pair + (int64_t)v * nct + ct]) / kw;
       for (int q = threadIdx.x & 31; q < nw; q += 32)
         t.wdst[g.o_word + w0 + s_sb[v] / kw + q] = (uint32_t)(d0 + q);
@@ -218,10 +243,24 @@ __global__ void __launch_bounds__(kGridPrepThreads)
   __syncthreads();
   // the block's variable list (ascending), local literals and entries of the send lists,
   // range by range
-  const int s_lo = grid_slot(g, coff, min(g.m, b * g.kc * g.TC)),
-            s_hi = grid_slot(g, coff, min(g.m, (b + 1) * g.kc * g.TC));
+  const int s_lo = grid_slot(g, coff, min(g.m, b * g.lt * g.TC)),
+            s_hi = grid_slot(g, coff, min(g.m, (b + 1) * g.lt * g.TC));
   const int TVb = g.TV * g.kv, d0 = t.dinfo[g.o_blk + b].x;
   const int32_t* dlo = t.dlo + g.o_bb + (int64_t)b * (g.B + 1);
+  const int32_t* dlp = t.dlp + g.o_bb + (int64_t)b * (g.B + 1);
+  const int32_t* poff = t.poff + g.o_bb + (int64_t)b * (g.B + 1);
+  // the words of the owning blocks' chunks
+  for (int c = threadIdx.x >> 5; c < g.B; c += NT / 32) {
+    const int nw = (dlp[c + 1] - dlp[c]) / kw;
+    const int64_t w0 = g.o_push + t.sinfo[g.o_blk + c].x + poff[c];
+    for (int q = threadIdx.x & 31; q < nw; q += 32)
+      t.sdst[w0 + q] = (uint32_t)((d0 + dlp[c]) / kw + q);
+    if ((threadIdx.x & 31) == 0)
+      for (int k = dlp[c] + dlo[c + 1] - dlo[c]; k < dlp[c + 1]; k++) {  // padding
+        t.dlist[g.o_list + d0 + k] = -1;
+        t.ids[w0 * kw + k - dlp[c]] = 0;
+      }
+  }
   int before = 0;
   for (int r0 = 0; r0 < g.n; r0 += 32 * RW) {
     const int nr = xp_bitmap<NT>(lit, s_lo, s_hi, bits, wpre, r0, RW, wsum);
@@ -231,10 +270,10 @@ __global__ void __launch_bounds__(kGridPrepThreads)
       while (x) {
         const int v = r0 + 32 * w + __ffs(x) - 1;
         x &= x - 1;
-        t.dlist[g.o_list + d0 + k] = v;
-        const int c = v / TVb;  // the block that owns v sends its dV here
-        t.sends[g.o_push + t.pinfo[g.o_bb + (int64_t)c * (g.B + 1) + b].x + k - dlo[c]] =
-            (uint32_t)(v - c * TVb) | ((uint32_t)b << 16);
+        const int c = v / TVb, at = dlp[c] + k - dlo[c];  // the block that owns v sends it here
+        t.dlist[g.o_list + d0 + at] = v;
+        t.ids[(g.o_push + t.sinfo[g.o_blk + c].x + poff[c]) * kw + at - dlp[c]] =
+            (uint16_t)(v - c * TVb);
         k++;
       }
     }
@@ -242,7 +281,8 @@ __global__ void __launch_bounds__(kGridPrepThreads)
       const int l = __ldg(lit + s);
       const int v = abs(l) - 1 - r0;
       if (v < 0 || v >= 32 * RW) continue;
-      const int loc = before + wpre[v >> 5] + __popc(bits[v >> 5] & ((1u << (v & 31)) - 1u));
+      const int k = before + wpre[v >> 5] + __popc(bits[v >> 5] & ((1u << (v & 31)) - 1u));
+      const int c = (abs(l) - 1) / TVb, loc = dlp[c] + k - dlo[c];
       t.llit[g.o_slot + s] = (int16_t)(l > 0 ? loc + 1 : -(loc + 1));
     }
     before += nr;

@@ -214,6 +214,23 @@ class Pack {
   // in *taken those it runs
   dmm_status plan_grid(const std::vector<int32_t>& cand, std::vector<int32_t>* taken);
   dmm_status launch_grid(int32_t nsteps);
+  // streaming form: builds the tables of formula idx over the whole grid
+  dmm_status plan_stream(int32_t idx, bool* ok);
+  dmm_status launch_stream(int32_t nsteps);
+  // cooperative launch over the tiles, by whichever form was planned
+  dmm_status launch_tiles(int32_t nsteps) {
+    return stream_active_ ? launch_stream(nsteps) : launch_persist(nsteps);
+  }
+  // space for, and pointers to, the tables of `groups`
+  struct GridSizes {
+    int64_t pair = 0, blks = 0, ct = 0, vt = 0, lst = 0, slot = 0, ux = 0, word = 0, row = 0,
+            push = 0, bb = 0;
+    int max_n = 0, max_nvt = 0, max_rows = 0;
+  };
+  void grid_place(GridGroup* g, GridSizes* z) const;
+  dmm_status grid_tables(const std::vector<GridGroup>& groups, const std::vector<int32_t>& map,
+                         int nblocks, const GridSizes& z, bool stream, GridTables* t,
+                         std::vector<int32_t>* out);
   double cluster_step_us() const;
   double grid_step_us(const std::vector<int32_t>& list) const;
   dmm_status grid_buffer(int which, int64_t bytes);
@@ -348,13 +365,16 @@ class Pack {
   int32_t gr_blocks_ = 0;
   bool gr_general_ = false;
   int gr_resident_ = 0;
+  bool stream_active_ = false;
+  bool stream_general_ = false;
+  StreamLayout stream_layout_{};
   bool gr_clean_ = false;  // group counters zeroed (every launch leaves them so)
   bool no_grid_ = false;
   GridLayout gr_layout_{};
   GridTables gr_tables_{};
   enum { kGrGroups, kGrBlk, kGrDlist, kGrDinfo, kGrLlit, kGrSpos, kGrWdst, kGrWoff, kGrBoff,
-         kGrRows, kGrIdx, kGrPinfo, kGrSends, kGrUx, kGrInbox, kGrCnt, kGrSb, kGrBt, kGrSt, kGrDcnt,
-         kGrDlo, kGrOut, kGrSync, kGrEpart, kGrBufs };
+         kGrRows, kGrIdx, kGrSinfo, kGrSdst, kGrDlp, kGrPoff, kGrUx, kGrInbox, kGrCnt, kGrSb, kGrBt, kGrSt, kGrDcnt,
+         kGrDlo, kGrOut, kGrSync, kGrEpart, kGrIds, kGrBtot, kGrPtot, kGrDv, kGrBufs };
   void* gbuf_[kGrBufs] = {};
   int64_t gbuf_cap_[kGrBufs] = {};
   // blocks of formulas laid aside (two, filled in turn) and their device copies

@@ -43,8 +43,8 @@ cudaError_t grid_unset(const GridTables& t, bool fp64, cudaStream_t s) {
   return cudaGetLastError();
 }
 
-cudaError_t grid_build(const GridGroup* groups, const int32_t* blk_group, int ngroups,
-                       int nblocks, int max_n, int max_nvt, const int32_t* lit,
+cudaError_t grid_build(const GridGroup* groups, const int32_t* list_group, int ngroups,
+                       int nlists, int max_n, int max_nvt, int max_rows, const int32_t* lit,
                        const int32_t* upos, const int32_t* vend, const int32_t* coff,
                        const GridTables& t, bool fp64, cudaStream_t s) {
   const int RW = std::min((max_n + 31) / 32, kXpRangeWords), kw = fp64 ? 2 : 4;
@@ -55,14 +55,15 @@ cudaError_t grid_build(const GridGroup* groups, const int32_t* blk_group, int ng
     if (e == cudaSuccess) e = cudaFuncSetAttribute(fill, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
     if (e != cudaSuccess) return e;
   }
-  k_grid_count<<<nblocks, kGridPrepThreads, smem, s>>>(groups, blk_group, lit, coff, t, RW, kw);
+  k_grid_count<<<nlists, kGridPrepThreads, smem, s>>>(groups, list_group, lit, coff, t, RW, kw);
+  k_grid_rows<<<dim3((unsigned)max_rows, (unsigned)ngroups), kGridRowThreads, 0, s>>>(groups, t, kw);
   k_grid_scan<<<ngroups, kGridPrepThreads, 0, s>>>(groups, coff, vend, t, kw);
   if (fp64)
-    k_grid_fill<true><<<nblocks, kGridPrepThreads, smem, s>>>(groups, blk_group, lit, upos, vend,
-                                                              coff, t, RW, kw);
+    k_grid_fill<true><<<nlists, kGridPrepThreads, smem, s>>>(groups, list_group, lit, upos, vend,
+                                                             coff, t, RW, kw);
   else
-    k_grid_fill<false><<<nblocks, kGridPrepThreads, smem, s>>>(groups, blk_group, lit, upos, vend,
-                                                               coff, t, RW, kw);
+    k_grid_fill<false><<<nlists, kGridPrepThreads, smem, s>>>(groups, list_group, lit, upos, vend,
+                                                              coff, t, RW, kw);
   return cudaGetLastError();
 }
 

@@ -213,6 +213,7 @@ constexpr int kXpSmemMax = 220 * 1024;  // dynamic shared memory of the staged f
 // variables: every tiling above the cap ran 8-30 % slower than the best one below it)
 constexpr int kXpSmemMaxMT = 193 * 1024;  // with the form's ~1.4 KB of static shared memory
 constexpr int kClusterChunk = 8;        // launches of steps_per_graph steps run() makes one of
+constexpr int kStreamSlots = 9000000;   // literals from which the streaming form runs a formula
 constexpr int kXpMaxTiles = 1 << 14;    // clause or variable tiles of the staged form, at most
 constexpr int kStatusInts = 8;           // ring_tail_d_
 constexpr int64_t kDirectCopy = 1 << 13; // doubles the driver's own pageable copies move
@@ -1287,6 +1288,234 @@ dmm_status Pack::grid_buffer(int which, int64_t bytes) {
   return DMM_OK;
 }
 
+// Places a group's part of each table array.
+void Pack::grid_place(GridGroup* g, GridSizes* z) const {
+  const int kw = 16 / (int)tsize_;
+  g->o_pair = z->pair;
+  g->o_blk = z->blks;
+  g->o_ct = z->ct;
+  g->o_vt = z->vt;
+  g->o_list = z->lst;
+  g->o_slot = z->slot;
+  g->o_ux = z->ux;
+  g->o_word = z->word;
+  g->o_row = z->row;
+  g->o_push = z->push;
+  g->o_bb = z->bb;
+  const int64_t pairs = (int64_t)g->nct * g->nvt, Ls = RangeAlloc::round(g->L);
+  const int64_t uxn = RangeAlloc::round(g->L + (g->pad - 1) * pairs + 32);
+  z->pair += pairs;
+  z->blks += std::max(g->NL, g->B) + 1;
+  z->ct += std::max(g->nct, g->B) + 1;
+  z->vt += g->nvt + 1;
+  const int64_t chunks = (int64_t)g->NL * g->B;  // each padded to whole words
+  const int64_t ent = RangeAlloc::round(std::min<int64_t>(g->L, (int64_t)g->NL * g->n) +
+                                        (kw - 1) * chunks + 4 * g->NL);
+  z->lst += ent;
+  z->slot += Ls;
+  z->ux += uxn;
+  z->word += uxn / kw;
+  z->row += (int64_t)g->nvt * g->TVr * 32;
+  z->push += ent / kw + 32;
+  z->bb += (int64_t)g->NL * (g->B + 1);
+  z->max_n = std::max(z->max_n, g->n);
+  z->max_nvt = std::max(z->max_nvt, g->nvt);
+  z->max_rows = std::max(z->max_rows, g->nvt + g->B);
+}
+
+// Allocates and builds the tables (map: group of every variable list; nblocks: blocks of the
+// launch); out: what grid_build reports per group.
+dmm_status Pack::grid_tables(const std::vector<GridGroup>& groups, const std::vector<int32_t>& map,
+                             int nblocks, const GridSizes& z, bool stream, GridTables* tables,
+                             std::vector<int32_t>* out) {
+  const int T = (int)tsize_, copies = stream ? 1 : 2;
+  const int64_t G = (int64_t)groups.size();
+  int64_t bytes[kGrBufs] = {};
+  bytes[kGrGroups] = G * (int64_t)sizeof(GridGroup);
+  bytes[kGrBlk] = (int64_t)map.size() * 4;
+  bytes[kGrDlist] = z.lst * 4;
+  bytes[kGrDinfo] = z.blks * 8;
+  bytes[kGrLlit] = z.slot * 2;
+  bytes[kGrSpos] = z.slot * 2;
+  bytes[kGrWdst] = z.word * 4;
+  bytes[kGrWoff] = z.ct * 4;
+  bytes[kGrBoff] = z.vt * 4;
+  bytes[kGrRows] = z.row * 2;
+  bytes[kGrIdx] = z.slot * 2;
+  const int kw = 16 / T;
+  bytes[kGrSinfo] = z.blks * 8;
+  bytes[kGrIds] = z.push * kw * 2;
+  bytes[kGrSdst] = z.push * 4;
+  bytes[kGrDlp] = bytes[kGrPoff] = z.bb * 4;
+  bytes[kGrUx] = copies * z.ux * T;
+  bytes[kGrInbox] = copies * z.lst * T;
+  bytes[kGrCnt] = bytes[kGrSb] = bytes[kGrBt] = z.pair * 4;
+  bytes[kGrSt] = z.ct * 4;
+  bytes[kGrDcnt] = z.blks * 4;
+  bytes[kGrDlo] = z.bb * 4;
+  bytes[kGrOut] = G * kGridOut * 4;
+  bytes[kGrSync] = G * kGridSyncBytes;
+  bytes[kGrEpart] = (int64_t)nblocks * 8;
+  bytes[kGrBtot] = z.vt * 4;
+  bytes[kGrPtot] = z.blks * 4;
+  if (stream) bytes[kGrDv] = caps_.vars * T;
+  for (int q = 0; q < kGrBufs; q++)
+    if (bytes[q] > 0) DMM_TRY(grid_buffer(q, bytes[q]));
+  GridTables t{};
+  t.dlist = static_cast<int32_t*>(gbuf_[kGrDlist]);
+  t.dinfo = static_cast<int2*>(gbuf_[kGrDinfo]);
+  t.llit = static_cast<int16_t*>(gbuf_[kGrLlit]);
+  t.spos = static_cast<uint16_t*>(gbuf_[kGrSpos]);
+  t.wdst = static_cast<uint32_t*>(gbuf_[kGrWdst]);
+  t.woff = static_cast<int32_t*>(gbuf_[kGrWoff]);
+  t.boff = static_cast<int32_t*>(gbuf_[kGrBoff]);
+  t.rows = static_cast<uint16_t*>(gbuf_[kGrRows]);
+  t.idx = static_cast<uint16_t*>(gbuf_[kGrIdx]);
+  t.sinfo = static_cast<int2*>(gbuf_[kGrSinfo]);
+  t.ids = static_cast<uint16_t*>(gbuf_[kGrIds]);
+  t.sdst = static_cast<uint32_t*>(gbuf_[kGrSdst]);
+  t.dlp = static_cast<int32_t*>(gbuf_[kGrDlp]);
+  t.poff = static_cast<int32_t*>(gbuf_[kGrPoff]);
+  t.ux = gbuf_[kGrUx];
+  t.inbox = gbuf_[kGrInbox];
+  t.ux_len = z.ux;
+  t.inbox_len = z.lst;
+  t.cnt = static_cast<int32_t*>(gbuf_[kGrCnt]);
+  t.sb = static_cast<int32_t*>(gbuf_[kGrSb]);
+  t.bt = static_cast<int32_t*>(gbuf_[kGrBt]);
+  t.st = static_cast<int32_t*>(gbuf_[kGrSt]);
+  t.dcnt = static_cast<int32_t*>(gbuf_[kGrDcnt]);
+  t.dlo = static_cast<int32_t*>(gbuf_[kGrDlo]);
+  t.btot = static_cast<int32_t*>(gbuf_[kGrBtot]);
+  t.ptot = static_cast<int32_t*>(gbuf_[kGrPtot]);
+  t.out = static_cast<int32_t*>(gbuf_[kGrOut]);
+  DMM_CUDA(cudaMemcpyAsync(gbuf_[kGrGroups], groups.data(), (size_t)bytes[kGrGroups],
+                           cudaMemcpyHostToDevice, stream_));
+  DMM_CUDA(cudaMemcpyAsync(gbuf_[kGrBlk], map.data(), (size_t)bytes[kGrBlk], cudaMemcpyHostToDevice,
+                           stream_));
+  DMM_CUDA(cudaMemsetAsync(t.rows, 0, (size_t)bytes[kGrRows], stream_));
+  DMM_CUDA(grid_build(static_cast<const GridGroup*>(gbuf_[kGrGroups]),
+                      static_cast<const int32_t*>(gbuf_[kGrBlk]), (int)G, (int)map.size(), z.max_n,
+                      z.max_nvt, z.max_rows, lit_, upos_, vend_, coff_, t, prec_ == DMM_FP64, stream_));
+  out->resize((size_t)(G * kGridOut));
+  DMM_CUDA(cudaMemcpyAsync(out->data(), t.out, (size_t)bytes[kGrOut], cudaMemcpyDeviceToHost, stream_));
+  DMM_CUDA(cudaStreamSynchronize(stream_));
+  *tables = t;
+  return DMM_OK;
+}
+
+dmm_status Pack::plan_stream(int32_t idx, bool* ok) {
+  *ok = false;
+  const InstDesc& I = inst_h_[idx];
+  const bool fp64 = prec_ == DMM_FP64;
+  // chunks of whole 32-byte sectors: a sector written by two blocks in halves is filled from
+  // memory when the buckets exceed the L2
+  const int T = (int)tsize_, kw = 16 / T, B = sms_, pad = 32 / T;
+  if (I.m <= 0 || I.nslots <= 0) return DMM_OK;
+  int kc_min = 1, kv_min = 1;
+  for (int round = 0; round < 4; round++) {
+    // fewest tiles per block whose lists, areas and buckets fit
+    const double n = I.n, L = I.nslots;
+    int kc = 0, kv = 0;
+    for (int sum = kc_min + kv_min; sum <= 128 && !kc; sum++)
+      for (int c = kc_min; c <= sum - kv_min && !kc; c++) {
+        const int v = sum - c;
+        const double Lt = L / ((double)B * c);
+        const double dl = n * (1.0 - std::exp(-Lt / n)) * 1.02 + 0.5 * kw * B + 16;
+        const double st = Lt * 1.02 + 0.5 * pad * B * v + 64;
+        const double bk = L / ((double)B * v) * 1.06 + 0.5 * pad * B * c + 64;
+        const double tv = n / B + 8 * v;
+        if (dl > kGridMaxDistinct || st > 65000 || bk > 65000 || tv > 65000) continue;
+        if (stream_shape((int)dl, (int)st, (int)bk, (int)tv, fp64).total > kStreamSmemMax) continue;
+        kc = c;
+        kv = v;
+      }
+    if (!kc) return DMM_OK;
+    GridGroup g{};
+    g.inst = idx;
+    g.B = B;
+    g.kc = kc;
+    g.kv = kv;
+    g.n = I.n;
+    g.m = I.m;
+    g.L = I.nslots;
+    g.k3 = I.k3;
+    g.var0 = I.var0;
+    g.cls0 = I.cls0;
+    g.slot0 = I.slot0;
+    g.TC = ((I.m + B * kc - 1) / (B * kc) + 3) & ~3;
+    g.TV = ((I.n + B * kv - 1) / (B * kv) + 3) & ~3;
+    g.TVr = (g.TV + 31) & ~31;
+    g.nct = B * kc;
+    g.nvt = B * kv;
+    g.lt = 1;
+    g.pad = pad;
+    g.NL = g.nct;
+    GridSizes z;
+    grid_place(&g, &z);
+    if (z.ux > INT32_MAX / 2 || z.row > INT32_MAX || z.pair > (int64_t(1) << 26)) return DMM_OK;
+    const std::vector<uint64_t> key{~0ull, add_serial_[idx], ((uint64_t)kc << 32) | (uint64_t)kv};
+    if (key == gr_key_) {
+      *ok = true;
+      return DMM_OK;
+    }
+    gr_key_.clear();
+    const std::vector<GridGroup> groups{g};
+    const std::vector<int32_t> map((size_t)g.NL, 0);
+    GridTables t{};
+    std::vector<int32_t> out;
+    DMM_TRY(grid_tables(groups, map, B, z, true, &t, &out));
+    const StreamLayout lay = stream_shape(out[1], out[2], out[3], g.TV * g.kv, fp64);
+    if (out[0] == 3 || (out[0] == 0 && lay.total > kStreamSmemMax && out[3] > out[2])) {
+      kv_min = kv + 1;
+      continue;
+    }
+    if (out[0] != 0 || lay.total > kStreamSmemMax) {
+      kc_min = kc + 1;
+      continue;
+    }
+    stream_general_ = I.k3 == 0;
+    if (occupancy_blocks(stream_kernel(fp64, stream_general_), fp64 ? kStreamThreads64 : kStreamThreads,
+                         lay.total) < 1)
+      return DMM_OK;
+    stream_layout_ = lay;
+    gr_tables_ = t;
+    gr_key_ = key;
+    *ok = true;
+    return DMM_OK;
+  }
+  return DMM_OK;
+}
+
+dmm_status Pack::launch_stream(int32_t nsteps) {
+  const bool fp64 = prec_ == DMM_FP64;
+  PackView<float> vf;
+  PackView<double> vd;
+  void* view;
+  if (fp64) {
+    fill_view<double>(&vd);
+    view = &vd;
+  } else {
+    fill_view<float>(&vf);
+    view = &vf;
+  }
+  unsigned int* bar = reinterpret_cast<unsigned int*>(misc_d_ + kMiscLaunch);
+  if (!launch_area_clean_)
+    DMM_CUDA(cudaMemsetAsync(bar, 0, kLaunchAreaInts * sizeof(int32_t), stream_));
+  launch_area_clean_ = true;
+  const void* fn = stream_kernel(fp64, stream_general_);
+  DMM_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, stream_layout_.total));
+  const void* groups = gbuf_[kGrGroups];
+  void* dv = gbuf_[kGrDv];
+  void* epart = gbuf_[kGrEpart];
+  int* err = error_d_;
+  void* args[] = {view, &gr_tables_, &groups, &stream_layout_, &dv, &nsteps, &bar, &epart, &err};
+  DMM_CUDA(cudaLaunchCooperativeKernel(fn, dim3((unsigned)sms_),
+                                       dim3(fp64 ? kStreamThreads64 : kStreamThreads), args,
+                                       (size_t)stream_layout_.total, stream_));
+  return DMM_OK;
+}
+
 dmm_status Pack::plan_grid(const std::vector<int32_t>& cand, std::vector<int32_t>* taken) {
   taken->clear();
   gr_groups_.clear();
@@ -1321,10 +1550,8 @@ dmm_status Pack::plan_grid(const std::vector<int32_t>& cand, std::vector<int32_t
     }
     std::vector<GridGroup> groups;
     std::vector<int32_t> blk, next;
-    int64_t pair = 0, blks = 0, ct = 0, vt = 0, lst = 0, slot = 0, ux = 0, word = 0, row = 0,
-            push = 0, bb = 0;
+    GridSizes z;
     bool general = false;
-    int max_n = 0, max_nvt = 0;
     for (size_t k = 0; k < list.size(); k++) {
       const InstDesc& I = inst_h_[list[k]];
       GridGroup g{};
@@ -1340,7 +1567,7 @@ dmm_status Pack::plan_grid(const std::vector<int32_t>& cand, std::vector<int32_t
       g.slot0 = I.slot0;
       // fewest tiles per block whose areas fit beside the block's voltages
       const double n = I.n, L = I.nslots;
-      const double distinct = n * (1.0 - std::exp(-L / (B[k] * n))) * 1.02 + 16;
+      const double distinct = n * (1.0 - std::exp(-L / (B[k] * n))) * 1.02 + 0.5 * kw * B[k] + 16;
       bool fits = false;
       for (int sum = 2; sum <= kGridMaxTiles && !fits; sum++)
         for (int kc = (sum + 1) / 2; kc < sum && !fits; kc++) {
@@ -1369,33 +1596,12 @@ dmm_status Pack::plan_grid(const std::vector<int32_t>& cand, std::vector<int32_t
       g.TVr = (g.TV + 31) & ~31;
       g.nct = g.B * g.kc;
       g.nvt = g.B * g.kv;
-      g.o_pair = pair;
-      g.o_blk = blks;
-      g.o_ct = ct;
-      g.o_vt = vt;
-      g.o_list = lst;
-      g.o_slot = slot;
-      g.o_ux = ux;
-      g.o_word = word;
-      g.o_row = row;
-      g.o_push = push;
-      g.o_bb = bb;
-      const int64_t pairs = (int64_t)g.nct * g.nvt, Ls = RangeAlloc::round(I.nslots);
-      const int64_t uxn = RangeAlloc::round(I.nslots + (kw - 1) * pairs + 32);
-      pair += pairs;
-      blks += g.B + 1;
-      ct += g.nct + 1;
-      vt += g.nvt + 1;
-      lst += RangeAlloc::round(I.nslots + 4 * g.B);
-      slot += Ls;
-      ux += uxn;
-      word += uxn / kw;
-      row += (int64_t)g.nvt * g.TVr * 32;
-      push += Ls;
-      bb += (int64_t)g.B * (g.B + 1);
+      g.lt = g.kc;
+      g.pad = kw;
+      g.NL = g.B;
+      g.list0 = g.blk0;
+      grid_place(&g, &z);
       general |= I.k3 == 0;
-      max_n = std::max(max_n, I.n);
-      max_nvt = std::max(max_nvt, g.nvt);
       for (int b = 0; b < g.B; b++) blk.push_back((int32_t)groups.size());
       groups.push_back(g);
       next.push_back(list[k]);
@@ -1404,7 +1610,7 @@ dmm_status Pack::plan_grid(const std::vector<int32_t>& cand, std::vector<int32_t
       list = next;
       continue;
     }
-    if (ux > INT32_MAX / 2 || row > INT32_MAX / 2) return DMM_OK;
+    if (z.ux > INT32_MAX / 2 || z.row > INT32_MAX / 2) return DMM_OK;
     // (the tables of the same formulas in the same tiles are still valid: only this function
     // writes them, and a live formula's device arrays do not change)
     std::vector<uint64_t> key;
@@ -1418,48 +1624,9 @@ dmm_status Pack::plan_grid(const std::vector<int32_t>& cand, std::vector<int32_t
       return DMM_OK;
     }
     gr_key_.clear();
-    const int64_t bytes[kGrBufs] = {
-        (int64_t)(groups.size() * sizeof(GridGroup)), (int64_t)blk.size() * 4, lst * 4, blks * 8,
-        slot * 2, slot * 2, word * 4, ct * 4, vt * 4, row * 2, slot * 2, bb * 8, push * 4,
-        2 * ux * T, 2 * lst * T, pair * 4, pair * 4, pair * 4, ct * 4, blks * 4, bb * 4,
-        (int64_t)groups.size() * kGridOut * 4, (int64_t)groups.size() * kGridSyncBytes,
-        (int64_t)blk.size() * 8};
-    for (int q = 0; q < kGrBufs; q++) DMM_TRY(grid_buffer(q, bytes[q]));
     GridTables t{};
-    t.dlist = static_cast<int32_t*>(gbuf_[kGrDlist]);
-    t.dinfo = static_cast<int2*>(gbuf_[kGrDinfo]);
-    t.llit = static_cast<int16_t*>(gbuf_[kGrLlit]);
-    t.spos = static_cast<uint16_t*>(gbuf_[kGrSpos]);
-    t.wdst = static_cast<uint32_t*>(gbuf_[kGrWdst]);
-    t.woff = static_cast<int32_t*>(gbuf_[kGrWoff]);
-    t.boff = static_cast<int32_t*>(gbuf_[kGrBoff]);
-    t.rows = static_cast<uint16_t*>(gbuf_[kGrRows]);
-    t.idx = static_cast<uint16_t*>(gbuf_[kGrIdx]);
-    t.pinfo = static_cast<int2*>(gbuf_[kGrPinfo]);
-    t.sends = static_cast<uint32_t*>(gbuf_[kGrSends]);
-    t.ux_len = ux;
-    t.inbox_len = lst;
-    t.ux = gbuf_[kGrUx];
-    t.inbox = gbuf_[kGrInbox];
-    t.cnt = static_cast<int32_t*>(gbuf_[kGrCnt]);
-    t.sb = static_cast<int32_t*>(gbuf_[kGrSb]);
-    t.bt = static_cast<int32_t*>(gbuf_[kGrBt]);
-    t.st = static_cast<int32_t*>(gbuf_[kGrSt]);
-    t.dcnt = static_cast<int32_t*>(gbuf_[kGrDcnt]);
-    t.dlo = static_cast<int32_t*>(gbuf_[kGrDlo]);
-    t.out = static_cast<int32_t*>(gbuf_[kGrOut]);
-    DMM_CUDA(cudaMemcpyAsync(gbuf_[kGrGroups], groups.data(), bytes[kGrGroups],
-                             cudaMemcpyHostToDevice, stream_));
-    DMM_CUDA(cudaMemcpyAsync(gbuf_[kGrBlk], blk.data(), bytes[kGrBlk], cudaMemcpyHostToDevice,
-                             stream_));
-    DMM_CUDA(cudaMemsetAsync(t.rows, 0, (size_t)bytes[kGrRows], stream_));
-    DMM_CUDA(grid_build(static_cast<const GridGroup*>(gbuf_[kGrGroups]),
-                        static_cast<const int32_t*>(gbuf_[kGrBlk]), (int)groups.size(),
-                        (int)blk.size(), max_n, max_nvt, lit_, upos_, vend_, coff_, t, fp64,
-                        stream_));
-    std::vector<int32_t> out(groups.size() * kGridOut);
-    DMM_CUDA(cudaMemcpyAsync(out.data(), t.out, bytes[kGrOut], cudaMemcpyDeviceToHost, stream_));
-    DMM_CUDA(cudaStreamSynchronize(stream_));
+    std::vector<int32_t> out;
+    DMM_TRY(grid_tables(groups, blk, (int)blk.size(), z, false, &t, &out));
     // what the tables need; a formula whose tiles came out too large gets more of them
     GridCaps caps{};
     bool again = false;
@@ -1731,6 +1898,7 @@ dmm_status Pack::commit_tiles() {
   DMM_TRY(resolve_long_lists());
   xp_active_ = false;
   one_active_ = false;
+  stream_active_ = false;
   ctiles_h_.clear();
   vtiles_h_.clear();
   std::vector<int32_t> live_list;
@@ -1843,13 +2011,19 @@ dmm_status Pack::commit_tiles() {
   // one formula on the cooperative path: two grid barriers per step; FP32 with the
   // default layout and tiles: the staged form when it fits
   one_active_ = coop && live_list.size() == 1 && small_list.empty();
-  if (one_active_ && prec_ == DMM_FP32 && tun_.u_layout == 0 && tun_.clause_tile == 0 &&
-      tun_.var_tile == 0) {
-    DMM_TRY(prepare_xpose(live_list[0], TC, TV, false, &xp_active_));
-    // too large for one tile per block: several tiles per block, else the tiles above
-    if (!xp_active_) {
-      DMM_TRY(prepare_xpose_mt(live_list[0], &xp_active_));
-      if (!xp_active_) DMM_TRY(set_tiles(live_list[0], TC, TV));
+  if (one_active_ && tun_.u_layout == 0 && tun_.clause_tile == 0 && tun_.var_tile == 0) {
+    const int32_t one = live_list[0];
+    if (prec_ == DMM_FP32) DMM_TRY(prepare_xpose(one, TC, TV, false, &xp_active_));
+    // too large for one tile per block: the streaming form (tiles in turn), else several staged
+    // tiles per block, else the tiles above
+    // (FP32 from 9 million literals on: below, and in FP64, where the sorted sums bound the
+    // step, its third barrier costs more than the gathers it saves; dmm_stream.cuh)
+    if (!xp_active_ && tun_.launch_mode == 0 && !fixed_grid_ && !no_grid_ && prec_ == DMM_FP32 &&
+        inst_h_[one].nslots >= kStreamSlots)
+      DMM_TRY(plan_stream(one, &stream_active_));
+    if (!xp_active_ && !stream_active_ && prec_ == DMM_FP32) {
+      DMM_TRY(prepare_xpose_mt(one, &xp_active_));
+      if (!xp_active_) DMM_TRY(set_tiles(one, TC, TV));
     }
   }
   if (!ctiles_h_.empty())
@@ -2143,7 +2317,7 @@ dmm_status Pack::test_barrier_timeout() {
     return DMM_ERR_STATE;
   }
   barrier_extra_ = 1;
-  const dmm_status st = gr_groups_.empty() ? launch_persist(1) : launch_grid(1);
+  const dmm_status st = gr_groups_.empty() ? launch_tiles(1) : launch_grid(1);
   barrier_extra_ = 0;
   DMM_TRY(st);
   DMM_CUDA(cudaStreamSynchronize(stream_));
@@ -2188,7 +2362,7 @@ dmm_status Pack::launch_steps(int32_t nsteps) {
     const bool clusters_only = cluster_only();
     while (nsteps > 0) {
       const int32_t k = clusters_only ? nsteps : std::min(nsteps, S);
-      if (!ctiles_h_.empty() || !vtiles_h_.empty()) DMM_TRY(launch_persist(k));
+      if (!ctiles_h_.empty() || !vtiles_h_.empty()) DMM_TRY(launch_tiles(k));
       if (n_small_ > 0) DMM_TRY(launch_inst(k));
       if (!gr_groups_.empty()) DMM_TRY(launch_grid(k));
       if (!clusters_.empty()) DMM_TRY(launch_cluster(k));
@@ -2285,6 +2459,7 @@ int Pack::launch_form() const {
   if (ctiles_h_.empty() && vtiles_h_.empty() && gr_groups_.size() == 1)
     return prec_ == DMM_FP32 && !gr_general_ ? 4 : 3;
   if (xp_active_) return xp_mt_ ? 6 : 4;
+  if (stream_active_) return prec_ == DMM_FP32 && !stream_general_ ? 6 : 3;
   if (one_active_) return 3;
   return 2;
 }
@@ -2299,7 +2474,7 @@ dmm_status Pack::trace_phases(int32_t nsteps, double* out) {
   }
   constexpr int K = kTraceK;
   const bool grid = !gr_groups_.empty();
-  const int G = grid ? gr_blocks_ : grid_p_;
+  const int G = grid ? gr_blocks_ : stream_active_ ? sms_ : grid_p_;
   const int64_t half = (int64_t)nsteps * K * G;
   // timer stamps, clock counts, then every block's entry and exit times (trace_launch)
   const int64_t need = 2 * half + 2 * G;
@@ -2312,7 +2487,7 @@ dmm_status Pack::trace_phases(int32_t nsteps, double* out) {
   DMM_CUDA(cudaMemsetAsync(trace_, 0, need * sizeof(long long), stream_));
   trace_on_ = true;
   trace_steps_ = nsteps;
-  dmm_status st = grid ? launch_grid(nsteps) : launch_persist(nsteps);  // one launch: trace step s = launch step s
+  dmm_status st = grid ? launch_grid(nsteps) : launch_tiles(nsteps);  // one launch: trace step s = launch step s
   trace_on_ = false;
   DMM_TRY(st);
   std::vector<long long> h(need);
