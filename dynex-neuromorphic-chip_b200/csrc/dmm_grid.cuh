@@ -32,6 +32,15 @@
 // RES 1: the tables of the variable phase live in shared memory for the launch; RES 2: so do
 // the clause memories and all other tables (formulas up to about 40,000 variables in FP32).
 //
+// FP64: the variables of a tile are kept by falling list length, the order being made with the
+// tables.  The lists that whole warps sum come first and need no queue, and a warp of the others
+// holds lists of like length; every per-variable array of the block is in that order, the
+// global ones are not.  Step with variables in their own order / by length, us: n = 5,000 8.9 /
+// 8.4, 10,000 10.8 / 10.2, 30,000 16.1 / 15.6, 50,000 23.0 / 21.8; clauses of mixed lengths
+// n = 10,000 12.5 / 11.8, 30,000 21.2 / 20.7.  FP32 sums take four lanes a list and gain nothing.
+// Splitting the network over two or four lanes was slower (n = 10,000 10.6 and 11.5): the
+// exchanges across lanes cost more than the shorter code saves.
+//
 // Every clause value and per-variable sum is computed from the same operands in the same order
 // as in the other forms: the states are identical.
 #pragma once
@@ -56,7 +65,7 @@ inline GridLayout grid_layout(const GridCaps& c, int tsize, bool general,
   L.raw = take((tsize * c.st > 16 + tsize * c.bk ? tsize * c.st : 16 + tsize * c.bk));
   L.cur = take(tsize * c.tv);
   L.dv = take(tsize * c.tv);
-  L.vend = take(4 * (c.tv + 1));
+  L.vend = take(8 * c.tv);
   L.unit = take(general ? c.tv : 0);
   L.rank = take(tsize == 8 ? 16 * kRankMax * (kGridThreads64 / 32) : 0);
   L.xs = L.xl = L.cp = L.lit = L.spos = L.off = L.wdst = L.row = L.csr = L.snd = 0;
@@ -240,9 +249,8 @@ __global__ void __launch_bounds__(sizeof(T) == 8 ? kGridThreads64 : kGridThreads
   __shared__ ClauseConsts<T> s_kc;
   __shared__ int cnt[3][W];
   __shared__ double red[W];
-  __shared__ int s_ok, s_last, s_nlong, s_unsat, s_next;
-  __shared__ int s_qend[kGridMaxTiles];  // end of each variable tile's part of s_long
-  __shared__ int32_t s_long[kLongQueue];
+  __shared__ int s_ok, s_last, s_unsat, s_next;
+  __shared__ int s_nq[kGridMaxTiles];  // lists of each variable tile that whole warps sum
   {
     unsigned have;
     asm volatile("mov.u32 %0, %%dynamic_smem_size;" : "=r"(have));
@@ -253,7 +261,7 @@ __global__ void __launch_bounds__(sizeof(T) == 8 ? kGridThreads64 : kGridThreads
   T* const raw = stage;
   T* const s_cur = reinterpret_cast<T*>(gr_smem + LY.cur);
   T* const s_dv = reinterpret_cast<T*>(gr_smem + LY.dv);
-  int* const s_vend = reinterpret_cast<int*>(gr_smem + LY.vend);
+  int2* const s_list = reinterpret_cast<int2*>(gr_smem + LY.vend);  // start and length of each list
   int8_t* const s_unit = reinterpret_cast<int8_t*>(gr_smem + LY.unit);
   double* const s_rank = reinterpret_cast<double*>(gr_smem + LY.rank);
   const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
@@ -273,7 +281,6 @@ __global__ void __launch_bounds__(sizeof(T) == 8 ? kGridThreads64 : kGridThreads
     lc.h = S->h_state;
     lc.t = S->t;
     lc.best_t = S->best_t;
-    s_nlong = 0;
     s_kc = make_consts<T>(I, lc.h);
   }
   __syncthreads();
@@ -313,32 +320,39 @@ __global__ void __launch_bounds__(sizeof(T) == 8 ? kGridThreads64 : kGridThreads
   }
   __syncthreads();
   int32_t* const off_s = reinterpret_cast<int32_t*>(gr_smem + LY.off);
+  // variable (from the block's first) at place i of the block: FP64 tiles keep their variables
+  // by falling list length, so that a warp's lists have similar lengths
+  auto var_at = [&](int i) {
+    if constexpr (sizeof(T) == 4) {
+      return i;
+    } else {
+      const int t0 = i / g.TV * g.TV;
+      return t0 + (int)tb.perm[g.o_var + v0 + i];
+    }
+  };
   if (lc.done == 0) {
     const T* V0 = P.cand + (int64_t)(lc.set * kTrials + lc.kcur) * P.var_cap + I.var0;
     const int32_t* dl = tb.dlist + g.o_list + sp.in_place;
     const int dcnt = sp.dcnt;
     for (int k = tid; k < dcnt; k += NT) sV[k] = dl[k] >= 0 ? V0[dl[k]] : T(0);
-    for (int i = tid; i < nv; i += NT) s_cur[i] = V0[v0 + i];
-    for (int i = tid; i <= nv; i += NT) s_vend[i] = (i > 0 ? vend[v0 + i - 1] : vend0) - vend0;
-    if (GENERAL)
-      for (int i = tid; i < nv; i += NT) s_unit[i] = P.unit[I.var0 + v0 + i];
+    for (int i = tid; i < nv; i += NT) {
+      const int v = v0 + var_at(i);
+      s_cur[i] = V0[v];
+      const int e0 = v > 0 ? vend[v - 1] : 0;
+      s_list[i] = make_int2(e0 - vend0, vend[v] - e0);
+      if (GENERAL) s_unit[i] = P.unit[I.var0 + v];
+    }
     // no entry of the areas may look unset (the padding of chunks is sent too)
     for (int q = tid; q < (LY.cur - LY.raw) / 16; q += NT)
       reinterpret_cast<int4*>(gr_smem + LY.raw)[q] = make_int4(0, 0, 0, 0);
     if constexpr (sizeof(T) == 8) {
-      // variables with lists past one thread's network, tile by tile: summed by warps
-      for (int j = 0; j < g.kv; j++) {
-        const int i0 = min(nv, j * g.TV), i1 = min(nv, i0 + g.TV);
-        for (int i = i0 + tid; i < i1; i += NT) {
-          const int e1 = vend[v0 + i], e0 = v0 + i > 0 ? vend[v0 + i - 1] : 0;
-          if (e1 - e0 > 32) {
-            const int q = atomicAdd(&s_nlong, 1);
-            if (q < kLongQueue) s_long[q] = i;
-          }
-        }
-        __syncthreads();
-        if (tid == 0) s_qend[j] = min(s_nlong, kLongQueue);
-        __syncthreads();
+      // how many of a tile's first lists whole warps sum: the ones past one thread's network
+      for (int j = tid; j < kGridMaxTiles; j += NT) s_nq[j] = 0;
+      __syncthreads();
+      for (int i = tid; i < nv; i += NT) {
+        const int j = i / g.TV;
+        const bool last = i + 1 == nv || (i + 1) % g.TV == 0;
+        if (s_list[i].y > 32 && (last || s_list[i + 1].y <= 32)) s_nq[j] = i + 1 - j * g.TV;
       }
     }
     if constexpr (RES >= 1) {
@@ -440,33 +454,38 @@ __global__ void __launch_bounds__(sizeof(T) == 8 ? kGridThreads64 : kGridThreads
       } else {
         // pairs of clauses: 4-byte words of literals and places, 2-wide loads of the memories
         // (the tile starts at a multiple of 4 clauses of a 32-aligned range)
-        auto pair = [&](int c) {
-          const int* L3 = reinterpret_cast<const int*>(llit + 3 * c);
-          const unsigned* Q3 = reinterpret_cast<const unsigned*>(spos + 3 * c);
+        using T2 = typename std::conditional<sizeof(T) == 8, double2, float2>::type;
+        struct Pair {
           int lw[3];
           unsigned qw[3];
+          T2 xs, xl, cp;
+        };
+        auto load_pair = [&](Pair& p, int c) {
+          const int* L3 = reinterpret_cast<const int*>(llit + 3 * c);
+          const unsigned* Q3 = reinterpret_cast<const unsigned*>(spos + 3 * c);
 #pragma unroll
           for (int r = 0; r < 3; r++) {
-            lw[r] = __ldg(L3 + r);
-            qw[r] = __ldg(Q3 + r);
+            p.lw[r] = __ldg(L3 + r);
+            p.qw[r] = __ldg(Q3 + r);
           }
+          p.xs = *reinterpret_cast<const T2*>(Xs + c);
+          p.xl = *reinterpret_cast<const T2*>(Xl + c);
+          p.cp.x = p.cp.y = T(0);
+          if (pending) p.cp = *reinterpret_cast<const T2*>(Cp + c);
+        };
+        auto do_pair = [&](const Pair& p, int c) {
           auto lit = [&](int k) {
-            return (k & 1) ? (lw[k >> 1] >> 16) : (int)(short)(lw[k >> 1] & 0xffff);
+            return (k & 1) ? (p.lw[k >> 1] >> 16) : (int)(short)(p.lw[k >> 1] & 0xffff);
           };
           auto pos = [&](int k) {
-            return (int)((k & 1) ? (qw[k >> 1] >> 16) : (qw[k >> 1] & 0xffffu));
+            return (int)((k & 1) ? (p.qw[k >> 1] >> 16) : (p.qw[k >> 1] & 0xffffu));
           };
-          using T2 = typename std::conditional<sizeof(T) == 8, double2, float2>::type;
-          const T2 xs2 = *reinterpret_cast<const T2*>(Xs + c);
-          const T2 xl2 = *reinterpret_cast<const T2*>(Xl + c);
-          T2 cp2, al2;
-          cp2.x = cp2.y = T(0);
+          T2 al2;
           al2.x = al2.y = kc.alpha;
-          if (pending) cp2 = *reinterpret_cast<const T2*>(Cp + c);
           if (acm) al2 = *reinterpret_cast<const T2*>(acm + c);
-          T xs[2] = {xs2.x, xs2.y}, xl[2] = {xl2.x, xl2.y}, cc[2];
-          cc[0] = one(lit(0), lit(1), lit(2), pos(0), pos(1), pos(2), xs[0], xl[0], cp2.x, al2.x);
-          cc[1] = one(lit(3), lit(4), lit(5), pos(3), pos(4), pos(5), xs[1], xl[1], cp2.y, al2.y);
+          T xs[2] = {p.xs.x, p.xs.y}, xl[2] = {p.xl.x, p.xl.y}, cc[2];
+          cc[0] = one(lit(0), lit(1), lit(2), pos(0), pos(1), pos(2), xs[0], xl[0], p.cp.x, al2.x);
+          cc[1] = one(lit(3), lit(4), lit(5), pos(3), pos(4), pos(5), xs[1], xl[1], p.cp.y, al2.y);
           T2 o;
           o.x = xs[0];
           o.y = xs[1];
@@ -511,15 +530,25 @@ __global__ void __launch_bounds__(sizeof(T) == 8 ? kGridThreads64 : kGridThreads
           }
           if (pairs) {
             const int c = full_end + 2 * tid;
-            if (c + 2 <= t1) pair(c);
-            else if (c < t1) single(c);
+            if (c + 2 <= t1) {
+              Pair p;
+              load_pair(p, c);
+              do_pair(p, c);
+            } else if (c < t1) {
+              single(c);
+            }
           } else if (g_end + tid < t1) {
             single(g_end + tid);  // fewer than 4 clauses
           }
         } else {
           for (int c = t0 + 2 * tid; c < t1; c += 2 * NT) {
-            if (c + 2 <= t1) pair(c);
-            else single(c);
+            if (c + 2 <= t1) {
+              Pair p;
+              load_pair(p, c);
+              do_pair(p, c);
+            } else {
+              single(c);
+            }
           }
         }
       }
@@ -599,7 +628,7 @@ __global__ void __launch_bounds__(sizeof(T) == 8 ? kGridThreads64 : kGridThreads
       }
       if (tid == 0) {
         raw[0] = sizeof(T) == 4 ? T(0) : inf_val<T>();
-        s_next = j > 0 ? s_qend[j - 1] : 0;
+        s_next = 0;
       }
       const uint16_t* const rt =
           (RES >= 1 ? reinterpret_cast<const uint16_t*>(gr_smem + LY.row) : sp.rows) + j * g.TVr * 32;
@@ -618,8 +647,9 @@ __global__ void __launch_bounds__(sizeof(T) == 8 ? kGridThreads64 : kGridThreads
             q = reinterpret_cast<const uint4*>(rt)[4 * (i + VPP - i0) + gl];
           int d = 0, e0 = 0;
           if (valid) {
-            e0 = s_vend[i];
-            d = s_vend[i + 1] - e0;
+            const int2 list = s_list[i];
+            e0 = list.x;
+            d = list.y;
           }
           const T dv = row_sum4<RES == 0>(reinterpret_cast<const float*>(raw), qc, idx + e0, d, gl);
           bool acc_k = false;
@@ -659,44 +689,30 @@ __global__ void __launch_bounds__(sizeof(T) == 8 ? kGridThreads64 : kGridThreads
         };
         // the last four warps start with the lists that whole warps sum, the others with the
         // rest, and all of them end with what is left of the former
-        const int q1 = s_qend[j];
-        auto warp_sum = [&](int i) {
-          const int e0 = s_vend[i], d = s_vend[i + 1] - e0;
-          const double dv = d <= kRankMax
-                                ? rank_sum<RES == 0>(ud, idx + e0, d, s_rank + 2 * kRankMax * w, lane)
-                                : sorted_sum<false, uint16_t, RES == 0>(ud, idx + e0, d, lane);
-          if (lane == 0) finish(i, T(dv));
-        };
+        const int q1 = s_nq[j];
         auto queue = [&]() {
           for (;;) {
             int q = 0;
             if (lane == 0) q = atomicAdd(&s_next, 1);
             q = __shfl_sync(0xffffffffu, q, 0);
             if (q >= q1) break;
-            warp_sum(s_long[q]);
+            const int2 list = s_list[i0 + q];
+            const double dv =
+                list.y <= kRankMax
+                    ? rank_sum<RES == 0>(ud, idx + list.x, list.y, s_rank + 2 * kRankMax * w, lane)
+                    : sorted_sum<false, uint16_t, RES == 0>(ud, idx + list.x, list.y, lane);
+            if (lane == 0) finish(i0 + q, T(dv));
           }
         };
         if (w >= W - 4) queue();
-        for (int vb = i0 + 32 * w; vb < i1; vb += NT) {
-          const int i = vb + lane;
-          const int d = i < i1 ? s_vend[i + 1] - s_vend[i] : 0;
-          const bool small = i < i1 && d <= 32;
-          const int ds = small ? d : 0;
-          const int dm = redux_max(ds);
-          const uint4* row = reinterpret_cast<const uint4*>(rt) + 4 * (vb - i0) + lane;
-          const double dv = dm <= 16   ? row_net_sum<16>(ud, row, ds)
-                            : dm <= 24 ? row_net_sum<24>(ud, row, ds)
-                                       : row_net_sum<32>(ud, row, ds);
-          if (small) finish(i, T(dv));
+        for (int vb = i0 + q1 + 32 * w; vb < i1; vb += NT) {
+          const int i = min(vb + lane, i1 - 1), r = i - i0;
+          const int2 list = s_list[i];
+          const uint4* row = reinterpret_cast<const uint4*>(rt) + (r >> 5) * 128 + (r & 31);
+          const double dv = row_net_sum<32>(ud, row, list.y);
+          if (vb + lane < i1) finish(i, T(dv));
         }
         queue();
-        if (s_nlong > kLongQueue)  // lists past the queue's end
-          for (int i = i0 + w; i < i1; i += W) {
-            if (s_vend[i + 1] - s_vend[i] <= 32) continue;
-            bool queued = false;
-            for (int q = lane; q < kLongQueue; q += 32) queued |= s_long[q] == i;
-            if (!__any_sync(0xffffffffu, queued)) warp_sum(i);
-          }
       }
     }
     kmax = redux_max(kmax);
@@ -819,7 +835,7 @@ __global__ void __launch_bounds__(sizeof(T) == 8 ? kGridThreads64 : kGridThreads
     if (!in_ok) s_ok = 0;
     if (lc.done == 1) {  // V(step) for the solution report
       T* sol = sp.cand + (int64_t)(set * kTrials + kcur) * P.var_cap;
-      for (int i = tid; i < nv; i += NT) sol[i] = s_cur[i];
+      for (int i = tid; i < nv; i += NT) sol[var_at(i)] = s_cur[i];
     }
     for (int i = tid; i < nv; i += NT) {
       T c = add(s_cur[i], mul(h, s_dv[i]));
@@ -848,7 +864,7 @@ __global__ void __launch_bounds__(sizeof(T) == 8 ? kGridThreads64 : kGridThreads
   // ---- end of the launch: state, energy of the last right-hand side, control record
   if (!gave_up && steps_run > 0) {
     T* cur = sp.cand + (int64_t)(lc.set * kTrials + lc.kcur) * P.var_cap;
-    for (int i = tid; i < nv; i += NT) cur[i] = s_cur[i];
+    for (int i = tid; i < nv; i += NT) cur[var_at(i)] = s_cur[i];
     double e = 0.0;
     for (int c = tid; c < c1 - c0; c += NT) {
       T C;

@@ -25,7 +25,7 @@ struct GridGroup {
   int32_t pad;                                 // entries that chunks of ux are padded to
   int32_t n, m, L, k3;
   int64_t var0, cls0, slot0;
-  int64_t o_pair, o_blk, o_ct, o_vt, o_list, o_slot, o_ux, o_word, o_row, o_push, o_bb;
+  int64_t o_pair, o_blk, o_ct, o_vt, o_list, o_slot, o_ux, o_word, o_row, o_push, o_bb, o_var;
 };
 
 // Table arrays of all groups.
@@ -41,6 +41,9 @@ struct GridTables {
   int32_t* boff;    // [o_vt + v] start of each variable tile's bucket in ux (nvt + 1)
   uint16_t* rows;   // [o_row] bucket places of each variable's first 32 contributions
   uint16_t* idx;    // [o_slot + j] bucket place of the contribution in CSR position j
+  // FP64: variables of a tile in order of falling list length (null: in their own order)
+  uint16_t* pos;    // [o_var + v] place of variable v in its tile
+  uint16_t* perm;   // [o_var + tile TV + place] variable of the tile
   int2* sinfo;      // [o_blk + b] start and count of block b's send words
   uint16_t* ids;    // [(o_push + word) kw] block-local variables of a send word
   uint32_t* sdst;   // [o_push + word] inbox word it goes to

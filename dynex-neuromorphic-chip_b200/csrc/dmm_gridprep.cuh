@@ -112,6 +112,34 @@ __global__ void __launch_bounds__(kGridPrepThreads)
 }
 
 constexpr int kGridRowThreads = 256;
+
+// Places of every variable tile's variables by falling list length (a counting sort over
+// lengths up to 255; longer ones first, in any order among equals: sums do not depend on it).
+__global__ void __launch_bounds__(kGridRowThreads)
+    k_grid_order(const GridGroup* __restrict__ groups, const int32_t* __restrict__ vend_all,
+                 GridTables t) {
+  __shared__ int bin[256], wsum[32];
+  const GridGroup& g = groups[blockIdx.y];
+  const int vt = blockIdx.x;
+  if (vt >= g.nvt) return;
+  const int v0 = min(g.n, vt * g.TV), v1 = min(g.n, v0 + g.TV);
+  const int32_t* vend = vend_all + g.var0;
+  auto key = [&](int v) { return 255 - min(255, vend[v] - (v > 0 ? vend[v - 1] : 0)); };
+  bin[threadIdx.x] = 0;
+  __syncthreads();
+  for (int v = v0 + threadIdx.x; v < v1; v += kGridRowThreads) atomicAdd(&bin[key(v)], 1);
+  __syncthreads();
+  int tot;
+  const int ex = block_exscan<kGridRowThreads>(bin[threadIdx.x], wsum, &tot);
+  bin[threadIdx.x] = ex;
+  __syncthreads();
+  for (int v = v0 + threadIdx.x; v < v1; v += kGridRowThreads) {
+    const int p = atomicAdd(&bin[key(v)], 1);
+    t.pos[g.o_var + v] = (uint16_t)p;
+    t.perm[g.o_var + v0 + p] = (uint16_t)(v - v0);
+  }
+}
+
 __global__ void __launch_bounds__(kGridRowThreads)
     k_grid_rows(const GridGroup* __restrict__ groups, GridTables t, int kw) {
   __shared__ int wsum[32];
@@ -225,7 +253,7 @@ __global__ void __launch_bounds__(kGridPrepThreads)
       const uint16_t at = (uint16_t)(kw + t.bt[g.o_pair + (int64_t)vt * nct + ct] + r);
       const int p = __ldg(upos + s), j = p - (v > 0 ? __ldg(vend + v - 1) : 0);
       t.idx[g.o_slot + p] = at;
-      const int vi = v - vt * g.TV;
+      const int vi = t.pos ? t.pos[g.o_var + v] : v - vt * g.TV;
       uint16_t* row = t.rows + g.o_row + (int64_t)vt * g.TVr * 32;
       if (j < 32)
         row[ROW64 ? ((vi >> 5) * 128 + (j >> 3) * 32 + (vi & 31)) * 8 + (j & 7)
@@ -273,7 +301,7 @@ __global__ void __launch_bounds__(kGridPrepThreads)
         const int c = v / TVb, at = dlp[c] + k - dlo[c];  // the block that owns v sends it here
         t.dlist[g.o_list + d0 + at] = v;
         t.ids[(g.o_push + t.sinfo[g.o_blk + c].x + poff[c]) * kw + at - dlp[c]] =
-            (uint16_t)(v - c * TVb);
+            (uint16_t)(t.pos ? v / g.TV * g.TV - c * TVb + t.pos[g.o_var + v] : v - c * TVb);
         k++;
       }
     }

@@ -55,6 +55,8 @@ cudaError_t grid_build(const GridGroup* groups, const int32_t* list_group, int n
     if (e == cudaSuccess) e = cudaFuncSetAttribute(fill, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
     if (e != cudaSuccess) return e;
   }
+  if (t.pos)
+    k_grid_order<<<dim3((unsigned)max_nvt, (unsigned)ngroups), kGridRowThreads, 0, s>>>(groups, vend, t);
   k_grid_count<<<nlists, kGridPrepThreads, smem, s>>>(groups, list_group, lit, coff, t, RW, kw);
   k_grid_rows<<<dim3((unsigned)max_rows, (unsigned)ngroups), kGridRowThreads, 0, s>>>(groups, t, kw);
   k_grid_scan<<<ngroups, kGridPrepThreads, 0, s>>>(groups, coff, vend, t, kw);

@@ -1302,6 +1302,7 @@ void Pack::grid_place(GridGroup* g, GridSizes* z) const {
   g->o_row = z->row;
   g->o_push = z->push;
   g->o_bb = z->bb;
+  g->o_var = z->var;
   const int64_t pairs = (int64_t)g->nct * g->nvt, Ls = RangeAlloc::round(g->L);
   const int64_t uxn = RangeAlloc::round(g->L + (g->pad - 1) * pairs + 32);
   z->pair += pairs;
@@ -1318,6 +1319,7 @@ void Pack::grid_place(GridGroup* g, GridSizes* z) const {
   z->row += (int64_t)g->nvt * g->TVr * 32;
   z->push += ent / kw + 32;
   z->bb += (int64_t)g->NL * (g->B + 1);
+  z->var += RangeAlloc::round(g->n);
   z->max_n = std::max(z->max_n, g->n);
   z->max_nvt = std::max(z->max_nvt, g->nvt);
   z->max_rows = std::max(z->max_rows, g->nvt + g->B);
@@ -1347,6 +1349,8 @@ dmm_status Pack::grid_tables(const std::vector<GridGroup>& groups, const std::ve
   bytes[kGrIds] = z.push * kw * 2;
   bytes[kGrSdst] = z.push * 4;
   bytes[kGrDlp] = bytes[kGrPoff] = z.bb * 4;
+  const bool ordered = prec_ == DMM_FP64 && !stream;
+  if (ordered) bytes[kGrPos] = bytes[kGrPerm] = z.var * 2;
   bytes[kGrUx] = copies * z.ux * T;
   bytes[kGrInbox] = copies * z.lst * T;
   bytes[kGrCnt] = bytes[kGrSb] = bytes[kGrBt] = z.pair * 4;
@@ -1374,6 +1378,8 @@ dmm_status Pack::grid_tables(const std::vector<GridGroup>& groups, const std::ve
   t.sinfo = static_cast<int2*>(gbuf_[kGrSinfo]);
   t.ids = static_cast<uint16_t*>(gbuf_[kGrIds]);
   t.sdst = static_cast<uint32_t*>(gbuf_[kGrSdst]);
+  t.pos = ordered ? static_cast<uint16_t*>(gbuf_[kGrPos]) : nullptr;
+  t.perm = ordered ? static_cast<uint16_t*>(gbuf_[kGrPerm]) : nullptr;
   t.dlp = static_cast<int32_t*>(gbuf_[kGrDlp]);
   t.poff = static_cast<int32_t*>(gbuf_[kGrPoff]);
   t.ux = gbuf_[kGrUx];
@@ -1576,7 +1582,7 @@ dmm_status Pack::plan_grid(const std::vector<int32_t>& cand, std::vector<int32_t
           const double stage = L / (B[k] * kc) * 1.02 + 0.5 * kw * B[k] * kv + 64;
           const double bucket = L / (B[k] * kv) * 1.06 + 0.5 * kw * B[k] * kc + 64;
           const double tvb = n / B[k] + 8 * kv;
-          const double smem = T * distinct + T * std::max(stage, bucket) + tvb * (2 * T + 5) +
+          const double smem = T * distinct + T * std::max(stage, bucket) + tvb * (2 * T + 9) +
                               8 * B[k] + (fp64 ? 16384 : 0) + 2048;
           if (distinct > kGridMaxDistinct || stage > 65000 || bucket > 65000 ||
               smem > kGridSmemMax || B[k] * kv > 1024 || B[k] * kc > 1024)
