@@ -137,48 +137,72 @@ __device__ __forceinline__ void cluster_sync(unsigned R) {
 
 // General clause (k literals) without a per-thread array: the first pass finds the two
 // smallest a_j, the second forms the contributions from recomputed a_j.  The same values as
-// clause_general.  lit(j): literal; val(j): voltage; put(j, u): contribution.
-template <class T, class Lit, class Val, class Put>
+// clause_general.  lit(j): literal; val(l): its voltage; pos(j): place of the contribution;
+// put(p, u): contribution.
+// Four literals at a time, loaded together: a literal on its own is a chain of two shared-memory
+// loads and the arithmetic, twice, and a warp waits for its longest clause.  Step at 6.6 clauses
+// of 1 to 8 literals per variable, one at a time / four, us: n = 1,000 FP64 7.6 / 7.2; n = 30,000
+// FP32 14.6 / 13.6, FP64 20.8 / 20.4.
+template <class T, class Lit, class Val, class Pos, class Put>
 __device__ __forceinline__ T clause_any(int k, Lit lit, Val val, T Xs, T Xl,
-                                        const ClauseConsts<T>& kc, Put put, bool& strict_sat) {
+                                        const ClauseConsts<T>& kc, Pos pos, Put put,
+                                        bool& strict_sat) {
   const T one = T(1), half = T(0.5), zero = T(0);
   strict_sat = false;
   if (k == 0) return mul(T(2147483647.0), half);
   if (k == 1) {
     const int l = lit(0);
-    const T v = val(0);
+    const T v = val(l);
     strict_sat = (v > zero && l > 0) || (v < zero && l < 0);
-    put(0, zero);
+    put(pos(0), zero);
     return zero;
   }
   T mn = T(2147483647.0), mn2 = T(2147483647.0);
   int arg = -1;
-  for (int j = 0; j < k; j++) {
-    const bool neg = lit(j) < 0;
-    const T v = val(j);
-    strict_sat |= neg ? v < zero : v > zero;
-    const T a = sub(one, neg_if(clampv(v, -one, one), neg));
-    if (a < mn) {
-      mn2 = mn;
-      mn = a;
-      arg = j;
-    } else if (a < mn2) {
-      mn2 = a;
+  for (int j0 = 0; j0 < k; j0 += 4) {
+    int l[4];
+    T v[4];
+#pragma unroll
+    for (int r = 0; r < 4; r++) l[r] = lit(min(j0 + r, k - 1));
+#pragma unroll
+    for (int r = 0; r < 4; r++) v[r] = val(l[r]);
+#pragma unroll
+    for (int r = 0; r < 4; r++) {
+      const bool neg = l[r] < 0, in = j0 + r < k;
+      strict_sat |= neg ? v[r] < zero : v[r] > zero;  // past the end: the last literal again
+      const T a = sub(one, neg_if(clampv(v[r], -one, one), neg));
+      const bool lt = in && a < mn, lt2 = in && a < mn2;
+      mn2 = lt ? mn : lt2 ? a : mn2;
+      mn = lt ? a : mn;
+      arg = lt ? j0 + r : arg;
     }
   }
   const T C = mul(mn, half);
   const T xs = clampv(Xs, zero, one), xl = clampv(Xl, one, kc.xlmax);
   const T xlxs = mul(xl, xs);
   const T rfac = mul(add(one, mul(kc.zeta, xl)), sub(one, xs));
-  for (int j = 0; j < k; j++) {
-    const bool neg = lit(j) < 0;
-    const T q = neg ? -one : one;
-    const T c = clampv(val(j), -one, one);
-    const T a = sub(one, neg_if(c, neg));
-    const T others = (j == arg) ? mn2 : mn;
-    const T g = mul(mul(q, others), half);
-    const T r = (C == mul(a, half)) ? mul(sub(q, c), half) : zero;
-    put(j, add(mul(xlxs, g), mul(rfac, r)));
+  for (int j0 = 0; j0 < k; j0 += 4) {
+    int l[4], p[4];
+    T v[4];
+#pragma unroll
+    for (int r = 0; r < 4; r++) {
+      const int j = min(j0 + r, k - 1);
+      l[r] = lit(j);
+      p[r] = pos(j);
+    }
+#pragma unroll
+    for (int r = 0; r < 4; r++) v[r] = val(l[r]);
+#pragma unroll
+    for (int r = 0; r < 4; r++) {
+      const bool neg = l[r] < 0;
+      const T q = neg ? -one : one;
+      const T c = clampv(v[r], -one, one);
+      const T a = sub(one, neg_if(c, neg));
+      const T others = (j0 + r == arg) ? mn2 : mn;
+      const T g = mul(mul(q, others), half);
+      const T rr = (C == mul(a, half)) ? mul(sub(q, c), half) : zero;
+      if (j0 + r < k) put(p[r], add(mul(xlxs, g), mul(rfac, rr)));
+    }
   }
   return C;
 }
@@ -476,8 +500,8 @@ __global__ void __launch_bounds__(sizeof(T) == 8 ? kClusterThreads64 : kClusterT
         const int o = off_s[c];
         C = clause_any<T>(
             off_s[c + 1] - o, [&](int j) { return (int)lit_s[o + j]; },
-            [&](int j) { return sV[abs((int)lit_s[o + j]) - 1]; }, xs, xl, kc,
-            [&](int j, T u) { stage[spos[o + j]] = u; }, ss);
+            [&](int l) { return sV[abs(l) - 1]; }, xs, xl, kc,
+            [&](int j) { return (int)spos[o + j]; }, [&](int p, T u) { stage[p] = u; }, ss);
       }
       cp_s[c] = C;
       unsat += !(C < T(0.5));

@@ -36,10 +36,17 @@
 // tables.  The lists that whole warps sum come first and need no queue, and a warp of the others
 // holds lists of like length; every per-variable array of the block is in that order, the
 // global ones are not.  Step with variables in their own order / by length, us: n = 5,000 8.9 /
-// 8.4, 10,000 10.8 / 10.2, 30,000 16.1 / 15.6, 50,000 23.0 / 21.8; clauses of mixed lengths
-// n = 10,000 12.5 / 11.8, 30,000 21.2 / 20.7.  FP32 sums take four lanes a list and gain nothing.
+// 8.4, 10,000 10.8 / 10.2, 30,000 16.1 / 15.6, 50,000 23.0 / 21.8.  FP32 sums take four lanes a list and gain nothing.
 // Splitting the network over two or four lanes was slower (n = 10,000 10.6 and 11.5): the
 // exchanges across lanes cost more than the shorter code saves.
+//
+// Clauses of other lengths than three: a block goes through a tile's clauses by falling length
+// (a table, with equal ones in their own order), so that a warp's clauses take alike many
+// iterations, and the clauses of three literals among them take the unrolled path.  The clause
+// phase is bound by instructions there: at 6.6 clauses of 1 to 8 literals per variable, in their
+// own order / by length, us: n = 30,000 FP32 13.6 / 11.7, FP64 20.4 / 17.0 (of which the clause
+// phase 8.8 / 5.4); n = 10,000 FP32 8.0 / 7.6, FP64 11.8 / 11.2; n = 60,000, where the clause
+// memories are read from L2 in that order, FP32 25.9 / 22.1, FP64 38.4 / 38.3.
 //
 // Every clause value and per-variable sum is computed from the same operands in the same order
 // as in the other forms: the states are identical.
@@ -68,7 +75,7 @@ inline GridLayout grid_layout(const GridCaps& c, int tsize, bool general,
   L.vend = take(8 * c.tv);
   L.unit = take(general ? c.tv : 0);
   L.rank = take(tsize == 8 ? 16 * kRankMax * (kGridThreads64 / 32) : 0);
-  L.xs = L.xl = L.cp = L.lit = L.spos = L.off = L.wdst = L.row = L.csr = L.snd = 0;
+  L.xs = L.xl = L.cp = L.lit = L.spos = L.off = L.ord = L.wdst = L.row = L.csr = L.snd = 0;
   if (resident >= 1) {
     L.row = take(2 * c.row);
     L.csr = take(2 * c.csr);
@@ -80,6 +87,7 @@ inline GridLayout grid_layout(const GridCaps& c, int tsize, bool general,
     L.lit = take(2 * c.ts);
     L.spos = take(2 * c.ts);
     L.off = take(general ? 4 * (c.tc + 1) : 0);
+    L.ord = take(general ? 2 * c.tc : 0);
     L.wdst = take(4 * c.wd);
     L.snd = take((4 + 2 * (16 / tsize)) * c.snd);
   }
@@ -199,7 +207,7 @@ struct GridPtrs {
   const T* acm;
   const int32_t *woff, *boff, *coff;
   const int16_t* llit;
-  const uint16_t *spos, *rows, *idx;
+  const uint16_t *spos, *rows, *idx, *ord;
   const uint16_t* ids;
   const uint32_t *wdst, *sdst;
   int in_place, dcnt, nsend;
@@ -316,6 +324,7 @@ __global__ void __launch_bounds__(sizeof(T) == 8 ? kGridThreads64 : kGridThreads
     sp.Cp = P.Cp + I.cls0 + c0;
     sp.acm = I.has_alpha_cm ? P.alpha_cm + I.cls0 + c0 : nullptr;
     sp.coff = P.coff + I.cls0 + c0;
+    sp.ord = tb.cord + g.o_cls + c0;
     sp.cand = P.cand + I.var0 + v0;
   }
   __syncthreads();
@@ -373,8 +382,10 @@ __global__ void __launch_bounds__(sizeof(T) == 8 ? kGridThreads64 : kGridThreads
         bring(LY.wdst, sp.wdst, sp.woff[g.kc] - sp.woff[0]);
         bring(LY.snd, sp.sdst, sp.nsend);
         bring(LY.snd + 4 * sp.nsend, sp.ids, kw * sp.nsend);
-        if (GENERAL)
+        if (GENERAL) {
           for (int c = tid; c <= c1 - c0; c += NT) off_s[c] = grid_slot(g, P.coff, c0 + c) - s0;
+          bring(LY.ord, sp.ord, c1 - c0);
+        }
       }
     }
   }
@@ -419,7 +430,11 @@ __global__ void __launch_bounds__(sizeof(T) == 8 ? kGridThreads64 : kGridThreads
     for (int i = 0; i < g.kc; i++) {
       const int t0 = min(c1 - c0, i * g.TC), t1 = min(c1 - c0, t0 + g.TC);
       if constexpr (GENERAL) {
-        for (int c = t0 + tid; c < t1; c += NT) {
+        // longest clauses first
+        const uint16_t* const ord =
+            RES == 2 ? reinterpret_cast<const uint16_t*>(gr_smem + LY.ord) : sp.ord;
+        for (int q = t0 + tid; q < t1; q += NT) {
+          const int c = t0 + ord[q];
           int o, o1;
           if constexpr (RES == 2) {
             o = off_s[c];
@@ -428,19 +443,24 @@ __global__ void __launch_bounds__(sizeof(T) == 8 ? kGridThreads64 : kGridThreads
             o = g.k3 ? 3 * c : __ldg(sp.coff + c) - s0;
             o1 = g.k3 ? 3 * c + 3 : c0 + c + 1 < m ? __ldg(sp.coff + c + 1) - s0 : g.L - s0;
           }
-          T xs = Xs[c], xl = Xl[c];
+          T xs = Xs[c], xl = Xl[c], C;
           const T al = acm ? acm[c] : kc.alpha;
-          if (pending) advance_memory(xs, xl, Cp[c], al, kc);
-          bool ss;
-          const T C = clause_any<T>(
-              o1 - o, [&](int j) { return (int)llit[o + j]; },
-              [&](int j) { return sV[abs((int)llit[o + j]) - 1]; }, xs, xl, kc,
-              [&](int j, T u) { stage[spos[o + j]] = u; }, ss);
+          if (o1 - o == 3) {
+            C = one(llit[o], llit[o + 1], llit[o + 2], spos[o], spos[o + 1], spos[o + 2], xs, xl,
+                    Cp[c], al);
+          } else {
+            if (pending) advance_memory(xs, xl, Cp[c], al, kc);
+            bool ss;
+            C = clause_any<T>(
+                o1 - o, [&](int j) { return (int)llit[o + j]; },
+                [&](int l) { return sV[abs(l) - 1]; }, xs, xl, kc,
+                [&](int j) { return (int)spos[o + j]; }, [&](int p, T u) { stage[p] = u; }, ss);
+            unsat += !(C < T(0.5));
+            vf += !ss;
+          }
           Xs[c] = xs;
           Xl[c] = xl;
           Cp[c] = C;
-          unsat += !(C < T(0.5));
-          vf += !ss;
         }
       } else if constexpr (RES == 2) {
         for (int c = t0 + tid; c < t1; c += NT) {

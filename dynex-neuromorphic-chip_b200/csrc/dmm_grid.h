@@ -25,7 +25,8 @@ struct GridGroup {
   int32_t pad;                                 // entries that chunks of ux are padded to
   int32_t n, m, L, k3;
   int64_t var0, cls0, slot0;
-  int64_t o_pair, o_blk, o_ct, o_vt, o_list, o_slot, o_ux, o_word, o_row, o_push, o_bb, o_var;
+  int64_t o_pair, o_blk, o_ct, o_vt, o_list, o_slot, o_ux, o_word, o_row, o_push, o_bb, o_var,
+      o_cls;
 };
 
 // Table arrays of all groups.
@@ -44,6 +45,8 @@ struct GridTables {
   // FP64: variables of a tile in order of falling list length (null: in their own order)
   uint16_t* pos;    // [o_var + v] place of variable v in its tile
   uint16_t* perm;   // [o_var + tile TV + place] variable of the tile
+  // general clauses: those of a tile in order of falling length (null: all have three literals)
+  uint16_t* cord;   // [o_cls + tile TC + place] clause of the tile
   int2* sinfo;      // [o_blk + b] start and count of block b's send words
   uint16_t* ids;    // [(o_push + word) kw] block-local variables of a send word
   uint32_t* sdst;   // [o_push + word] inbox word it goes to
@@ -78,7 +81,7 @@ constexpr int kGridSyncBytes = 256;  // per group
 // Byte offsets of a block's dynamic shared memory.
 struct GridLayout {
   int sv, raw, cur, dv, vend, unit, pinfo, rank;
-  int xs, xl, cp, lit, spos, off, wdst, row, csr, snd, total;
+  int xs, xl, cp, lit, spos, off, ord, wdst, row, csr, snd, total;
 };
 
 // resident: 0 no tables in shared memory, 1 those of the variable phase, 2 all and the clause
@@ -92,7 +95,7 @@ const void* grid_kernel(bool fp64, bool general, int resident);
 cudaError_t grid_unset(const GridTables& t, bool fp64, cudaStream_t s);
 // Queues the table build of all groups (list_group: group of every list).
 cudaError_t grid_build(const GridGroup* groups, const int32_t* list_group, int ngroups,
-                       int nlists, int max_n, int max_nvt, int max_rows, const int32_t* lit,
+                       int nlists, int max_n, int max_nct, int max_nvt, int max_rows, const int32_t* lit,
                        const int32_t* upos, const int32_t* vend, const int32_t* coff,
                        const GridTables& t, bool fp64, cudaStream_t s);
 

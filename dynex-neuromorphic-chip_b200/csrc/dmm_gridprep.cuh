@@ -140,6 +140,38 @@ __global__ void __launch_bounds__(kGridRowThreads)
   }
 }
 
+// Places of every clause tile's clauses by falling length, in their own order among equals (so
+// that neighbours stay close): counts per thread's range and length, one scan over them.
+__global__ void __launch_bounds__(kGridRowThreads)
+    k_grid_clauses(const GridGroup* __restrict__ groups, const int32_t* __restrict__ coff,
+                   GridTables t) {
+  constexpr int K = 16;  // lengths 0 .. 14, and longer ones
+  __shared__ int at[K * kGridRowThreads], wsum[32];
+  const GridGroup& g = groups[blockIdx.y];
+  const int ct = blockIdx.x, tid = threadIdx.x;
+  if (ct >= g.nct) return;
+  const int c0 = min(g.m, ct * g.TC), n = min(g.m, c0 + g.TC) - c0;
+  const int per = (n + kGridRowThreads - 1) / kGridRowThreads;
+  const int i0 = min(n, tid * per), i1 = min(n, i0 + per);
+  auto key = [&](int i) {
+    return K - 1 - min(K - 1, grid_slot(g, coff, c0 + i + 1) - grid_slot(g, coff, c0 + i));
+  };
+  for (int k = 0; k < K; k++) at[k * kGridRowThreads + tid] = 0;
+  for (int i = i0; i < i1; i++) at[key(i) * kGridRowThreads + tid]++;
+  __syncthreads();
+  int own = 0, tot;
+  for (int k = 0; k < K; k++) own += at[tid * K + k];
+  int sum = block_exscan<kGridRowThreads>(own, wsum, &tot);
+  for (int k = 0; k < K; k++) {
+    const int v = at[tid * K + k];
+    at[tid * K + k] = sum;
+    sum += v;
+  }
+  __syncthreads();
+  for (int i = i0; i < i1; i++)
+    t.cord[g.o_cls + c0 + at[key(i) * kGridRowThreads + tid]++] = (uint16_t)i;
+}
+
 __global__ void __launch_bounds__(kGridRowThreads)
     k_grid_rows(const GridGroup* __restrict__ groups, GridTables t, int kw) {
   __shared__ int wsum[32];

@@ -224,8 +224,8 @@ class Pack {
   // space for, and pointers to, the tables of `groups`
   struct GridSizes {
     int64_t pair = 0, blks = 0, ct = 0, vt = 0, lst = 0, slot = 0, ux = 0, word = 0, row = 0,
-            push = 0, bb = 0, var = 0;
-    int max_n = 0, max_nvt = 0, max_rows = 0;
+            push = 0, bb = 0, var = 0, cls = 0;
+    int max_n = 0, max_nct = 0, max_nvt = 0, max_rows = 0;
   };
   void grid_place(GridGroup* g, GridSizes* z) const;
   dmm_status grid_tables(const std::vector<GridGroup>& groups, const std::vector<int32_t>& map,
@@ -373,7 +373,7 @@ class Pack {
   GridLayout gr_layout_{};
   GridTables gr_tables_{};
   enum { kGrGroups, kGrBlk, kGrDlist, kGrDinfo, kGrLlit, kGrSpos, kGrWdst, kGrWoff, kGrBoff,
-         kGrRows, kGrIdx, kGrSinfo, kGrSdst, kGrDlp, kGrPoff, kGrPos, kGrPerm, kGrUx, kGrInbox, kGrCnt, kGrSb, kGrBt, kGrSt, kGrDcnt,
+         kGrRows, kGrIdx, kGrSinfo, kGrSdst, kGrDlp, kGrPoff, kGrPos, kGrPerm, kGrCord, kGrUx, kGrInbox, kGrCnt, kGrSb, kGrBt, kGrSt, kGrDcnt,
          kGrDlo, kGrOut, kGrSync, kGrEpart, kGrIds, kGrBtot, kGrPtot, kGrDv, kGrBufs };
   void* gbuf_[kGrBufs] = {};
   int64_t gbuf_cap_[kGrBufs] = {};

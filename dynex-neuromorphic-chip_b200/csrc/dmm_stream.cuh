@@ -216,8 +216,9 @@ __global__ void __launch_bounds__(sizeof(T) == 8 ? kStreamThreads64 : kStreamThr
           bool ss;
           const T C = clause_any<T>(
               o1 - o, [&](int j) { return (int)__ldg(llit + o + j); },
-              [&](int j) { return sV[abs((int)__ldg(llit + o + j)) - 1]; }, xs, xl, kc,
-              [&](int j, T u) { stage[__ldg(spos + o + j)] = u; }, ss);
+              [&](int l) { return sV[abs(l) - 1]; }, xs, xl, kc,
+              [&](int j) { return (int)__ldg(spos + o + j); }, [&](int p, T u) { stage[p] = u; },
+              ss);
           Xs[c] = xs;
           Xl[c] = xl;
           Cp[c] = C;

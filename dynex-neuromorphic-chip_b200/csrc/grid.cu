@@ -44,7 +44,7 @@ cudaError_t grid_unset(const GridTables& t, bool fp64, cudaStream_t s) {
 }
 
 cudaError_t grid_build(const GridGroup* groups, const int32_t* list_group, int ngroups,
-                       int nlists, int max_n, int max_nvt, int max_rows, const int32_t* lit,
+                       int nlists, int max_n, int max_nct, int max_nvt, int max_rows, const int32_t* lit,
                        const int32_t* upos, const int32_t* vend, const int32_t* coff,
                        const GridTables& t, bool fp64, cudaStream_t s) {
   const int RW = std::min((max_n + 31) / 32, kXpRangeWords), kw = fp64 ? 2 : 4;
@@ -57,6 +57,8 @@ cudaError_t grid_build(const GridGroup* groups, const int32_t* list_group, int n
   }
   if (t.pos)
     k_grid_order<<<dim3((unsigned)max_nvt, (unsigned)ngroups), kGridRowThreads, 0, s>>>(groups, vend, t);
+  if (t.cord)
+    k_grid_clauses<<<dim3((unsigned)max_nct, (unsigned)ngroups), kGridRowThreads, 0, s>>>(groups, coff, t);
   k_grid_count<<<nlists, kGridPrepThreads, smem, s>>>(groups, list_group, lit, coff, t, RW, kw);
   k_grid_rows<<<dim3((unsigned)max_rows, (unsigned)ngroups), kGridRowThreads, 0, s>>>(groups, t, kw);
   k_grid_scan<<<ngroups, kGridPrepThreads, 0, s>>>(groups, coff, vend, t, kw);

@@ -1255,26 +1255,37 @@ static const void* staged_fn(int G, bool mt) {
 // 4.8 at 1,000; FP64 4.7 and 9.9), in waves when the clusters do not all fit at once; the
 // resident grid form by a block's share of the clauses (FP32 5.1 us at 54, 9.8 at 1,600; FP64
 // 7.5 and 15.9).  The two meet at about 18,000 clauses (FP32) and 13,000 (FP64) for one formula.
+// Clauses of other lengths have their own fits, at 3.5 and 6.6 clauses per variable (cluster
+// FP32 4.2 us at 206 and 7.2 at 825, FP64 6.1 and, at 619, 9.5; grid FP32 6.2 at 67 and 11.8 at
+// 1,338, FP64 9.2 and 17.0): a warp of the cluster form waits for its longest clause, the grid
+// form orders them.  These meet at about 10,000 and 9,400 clauses (cluster / grid at 13,200:
+// FP32 7.2 / 6.3; at 10,500: FP64 10.6 / 8.8).
 double Pack::cluster_step_us() const {
+  const bool fp64 = prec_ == DMM_FP64;
   int64_t blocks = 0;
-  int tc = 0;
+  double most = 0;
   for (const ClusterLaunch& L : clusters_) {
     blocks += (int64_t)L.R * L.count;
-    tc = std::max(tc, L.caps.tc);
+    const double us = L.general ? (fp64 ? 4.2 + 8.2e-3 * L.caps.tc : 2.6 + 5.6e-3 * L.caps.tc)
+                                : (fp64 ? 3.6 + 5.0e-3 * L.caps.tc : 2.6 + 2.2e-3 * L.caps.tc);
+    most = std::max(most, us);
   }
-  const double waves = (double)((blocks + sms_ - 1) / sms_);
-  return waves * (prec_ == DMM_FP64 ? 3.6 + 5.0e-3 * tc : 2.6 + 2.2e-3 * tc);
+  return (double)((blocks + sms_ - 1) / sms_) * most;
 }
 
 double Pack::grid_step_us(const std::vector<int32_t>& list) const {
   if ((int)list.size() > sms_) return 1e9;
+  const bool fp64 = prec_ == DMM_FP64;
   double total = 0, most = 0;
+  bool general = false;
   for (int32_t i : list) {
     total += inst_h_[i].m;
     most = std::max(most, (double)inst_h_[i].m);
+    general |= inst_h_[i].k3 == 0;
   }
   const double share = std::max(total / sms_, most / (sms_ - (double)list.size() + 1));
-  return prec_ == DMM_FP64 ? 7.0 + 5.2e-3 * share : 4.9 + 3.2e-3 * share;
+  return general ? (fp64 ? 8.6 + 6.3e-3 * share : 5.9 + 4.3e-3 * share)
+                 : (fp64 ? 7.0 + 5.2e-3 * share : 4.9 + 3.2e-3 * share);
 }
 
 dmm_status Pack::grid_buffer(int which, int64_t bytes) {
@@ -1303,6 +1314,7 @@ void Pack::grid_place(GridGroup* g, GridSizes* z) const {
   g->o_push = z->push;
   g->o_bb = z->bb;
   g->o_var = z->var;
+  g->o_cls = z->cls;
   const int64_t pairs = (int64_t)g->nct * g->nvt, Ls = RangeAlloc::round(g->L);
   const int64_t uxn = RangeAlloc::round(g->L + (g->pad - 1) * pairs + 32);
   z->pair += pairs;
@@ -1320,7 +1332,9 @@ void Pack::grid_place(GridGroup* g, GridSizes* z) const {
   z->push += ent / kw + 32;
   z->bb += (int64_t)g->NL * (g->B + 1);
   z->var += RangeAlloc::round(g->n);
+  z->cls += RangeAlloc::round(g->m);
   z->max_n = std::max(z->max_n, g->n);
+  z->max_nct = std::max(z->max_nct, g->nct);
   z->max_nvt = std::max(z->max_nvt, g->nvt);
   z->max_rows = std::max(z->max_rows, g->nvt + g->B);
 }
@@ -1351,6 +1365,9 @@ dmm_status Pack::grid_tables(const std::vector<GridGroup>& groups, const std::ve
   bytes[kGrDlp] = bytes[kGrPoff] = z.bb * 4;
   const bool ordered = prec_ == DMM_FP64 && !stream;
   if (ordered) bytes[kGrPos] = bytes[kGrPerm] = z.var * 2;
+  bool general = false;
+  for (const GridGroup& g : groups) general |= !stream && g.k3 == 0;
+  if (general) bytes[kGrCord] = z.cls * 2;
   bytes[kGrUx] = copies * z.ux * T;
   bytes[kGrInbox] = copies * z.lst * T;
   bytes[kGrCnt] = bytes[kGrSb] = bytes[kGrBt] = z.pair * 4;
@@ -1379,6 +1396,7 @@ dmm_status Pack::grid_tables(const std::vector<GridGroup>& groups, const std::ve
   t.ids = static_cast<uint16_t*>(gbuf_[kGrIds]);
   t.sdst = static_cast<uint32_t*>(gbuf_[kGrSdst]);
   t.pos = ordered ? static_cast<uint16_t*>(gbuf_[kGrPos]) : nullptr;
+  t.cord = general ? static_cast<uint16_t*>(gbuf_[kGrCord]) : nullptr;
   t.perm = ordered ? static_cast<uint16_t*>(gbuf_[kGrPerm]) : nullptr;
   t.dlp = static_cast<int32_t*>(gbuf_[kGrDlp]);
   t.poff = static_cast<int32_t*>(gbuf_[kGrPoff]);
@@ -1402,7 +1420,7 @@ dmm_status Pack::grid_tables(const std::vector<GridGroup>& groups, const std::ve
   DMM_CUDA(cudaMemsetAsync(t.rows, 0, (size_t)bytes[kGrRows], stream_));
   DMM_CUDA(grid_build(static_cast<const GridGroup*>(gbuf_[kGrGroups]),
                       static_cast<const int32_t*>(gbuf_[kGrBlk]), (int)G, (int)map.size(), z.max_n,
-                      z.max_nvt, z.max_rows, lit_, upos_, vend_, coff_, t, prec_ == DMM_FP64, stream_));
+                      z.max_nct, z.max_nvt, z.max_rows, lit_, upos_, vend_, coff_, t, prec_ == DMM_FP64, stream_));
   out->resize((size_t)(G * kGridOut));
   DMM_CUDA(cudaMemcpyAsync(out->data(), t.out, (size_t)bytes[kGrOut], cudaMemcpyDeviceToHost, stream_));
   DMM_CUDA(cudaStreamSynchronize(stream_));

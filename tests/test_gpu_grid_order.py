@@ -46,3 +46,27 @@ def test_lists_of_given_lengths(n, lengths):
 def test_unit_clauses_follow_their_variables():
     form = random_formula(5003, 30011, 1, 9, seed=4)
     check(form, uniform_init(form.n, form.m, 6), "fp64", 8, pieces=[1, 7])
+
+
+def formula_of_clause_lengths(n, lengths, m, seed):
+    """m clauses over distinct variables, clause c of lengths[c mod len(lengths)] literals."""
+    rng = np.random.default_rng(seed)
+    lens = np.resize(lengths, m)
+    rng.shuffle(lens)
+    off = np.concatenate([[0], np.cumsum(lens)])
+    lits = np.concatenate([rng.choice(n, k, replace=False) + 1 for k in lens])
+    lits = lits * rng.choice([-1, 1], size=len(lits))
+    return dmm.from_arrays(lits.astype(np.int32), off, n)
+
+
+@pytest.mark.parametrize("prec", ["fp32", "fp64"])
+@pytest.mark.parametrize("n,m,lengths", [
+    (4001, 12345, [2, 3, 4, 5, 8, 9]),           # both sides of whole groups of four literals
+    (3000, 11111, [3] * 200 + [1, 14, 15, 16, 17, 25]),  # around the last class of the ordering
+    (5000, 9001, [4]),                           # all alike, none of three
+    (60000, 330001, [2, 3, 3, 5]),               # clause memories not resident
+])
+def test_clauses_of_given_lengths(prec, n, m, lengths):
+    """Clause tiles are gone through by falling clause length."""
+    form = formula_of_clause_lengths(n, lengths, m, n)
+    check(form, uniform_init(form.n, form.m, 4), prec, 8, pieces=[3, 5])
