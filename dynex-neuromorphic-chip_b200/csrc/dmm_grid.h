@@ -4,6 +4,7 @@
 #include <cuda_runtime.h>
 
 #include <cstdint>
+#include <vector>
 
 #include "dmm_device.cuh"
 
@@ -91,6 +92,8 @@ inline int grid_smem(const GridCaps& c, bool fp64, bool general, int resident) {
   return grid_shape(c, fp64, general, resident).total;
 }
 const void* grid_kernel(bool fp64, bool general, int resident);
+// The kernels of the form in one precision, its table build included.
+void grid_functions(bool fp64, std::vector<const void*>* out);
 // Queues the marking of all exchange entries as unset.
 cudaError_t grid_unset(const GridTables& t, bool fp64, cudaStream_t s);
 // Queues the table build of all groups (list_group: group of every list).

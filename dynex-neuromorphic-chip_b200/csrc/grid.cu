@@ -71,4 +71,14 @@ cudaError_t grid_build(const GridGroup* groups, const int32_t* list_group, int n
   return cudaGetLastError();
 }
 
+void grid_functions(bool fp64, std::vector<const void*>* out) {
+  for (int q = 0; q < 6; q++) out->push_back(grid_kernel(fp64, q & 1, q >> 1));
+  out->push_back(fp64 ? (const void*)k_grid_unset<unsigned long long>
+                      : (const void*)k_grid_unset<unsigned int>);
+  out->push_back(fp64 ? (const void*)k_grid_fill<true> : (const void*)k_grid_fill<false>);
+  out->insert(out->end(), {(const void*)k_grid_order, (const void*)k_grid_clauses,
+                           (const void*)k_grid_count, (const void*)k_grid_rows,
+                           (const void*)k_grid_scan});
+}
+
 }  // namespace dmm

@@ -2446,11 +2446,15 @@ dmm_status Pack::preload_kernels() {
     fns.push_back((const void*)k_set_state<double>);
     fns.push_back((const void*)k_get_state<double>);
     fns.push_back((const void*)k_signs<double>);
+    fns.push_back((const void*)k_signs_all<double>);
+    fns.push_back((const void*)k_admit<double>);
     fns.push_back(persist_fn_x<true>(prec_, G));
   } else {
     fns.push_back((const void*)k_set_state<float>);
     fns.push_back((const void*)k_get_state<float>);
     fns.push_back((const void*)k_signs<float>);
+    fns.push_back((const void*)k_signs_all<float>);
+    fns.push_back((const void*)k_admit<float>);
     fns.push_back(persist_fn_x<true>(prec_, G));
     fns.push_back(staged_fn(G, false));
     fns.push_back(staged_fn(G, true));
@@ -2468,6 +2472,9 @@ dmm_status Pack::preload_kernels() {
   }
   fns.push_back(cluster_kernel(prec_ == DMM_FP64, false));
   fns.push_back(cluster_kernel(prec_ == DMM_FP64, true));
+  grid_functions(prec_ == DMM_FP64, &fns);
+  fns.push_back(stream_kernel(prec_ == DMM_FP64, false));
+  fns.push_back(stream_kernel(prec_ == DMM_FP64, true));
   for (const void* f : fns) {
     cudaFuncAttributes a;
     DMM_CUDA(cudaFuncGetAttributes(&a, f));
