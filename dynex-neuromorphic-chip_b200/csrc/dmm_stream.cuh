@@ -18,7 +18,7 @@
 // of the third barrier (about 3 us).
 //
 // Measured (FP32, 8 clauses per variable, us per step against the staged form's several tiles per
-// block): n = 4 10^5 89 / 96, 6 10^5 138 / 146, 10^6 238 / 267, 1.5 10^6 398 / 416; clauses of
+// block): n = 4 10^5 89 / 96, 6 10^5 138 / 146, 10^6 235 / 267, 1.5 10^6 398 / 416; clauses of
 // 1 to 8 literals, n = 4 10^5 156 / 189 (tile form).  Bound by memory traffic: about 900 MB per step
 // at n = 10^6 (clause memories 192, literal and place words 96, buckets and lists in and out
 // 430, row tables 64, send words 72, destinations 30).  Tried: L2 evict-last for the
@@ -93,8 +93,8 @@ __global__ void __launch_bounds__(sizeof(T) == 8 ? kStreamThreads64 : kStreamThr
   bool ok = true;
 
   // C: voltages of the block's variables at `cur` (their new value when h is given) to the
-  // inboxes
-  auto send = [&](const T* cur, T* nxt, bool step_h, T h) {
+  // inboxes (unless no step of this launch will read them)
+  auto send = [&](const T* cur, T* nxt, bool step_h, T h, bool lists) {
     T* const sv = reinterpret_cast<T*>(st_smem);
     for (int i = tid; i < nv; i += NT) {
       T c = cur[v0 + i];
@@ -110,7 +110,8 @@ __global__ void __launch_bounds__(sizeof(T) == 8 ? kStreamThreads64 : kStreamThr
       sv[i] = c;
     }
     __syncthreads();
-    const int2 si = tb.sinfo[g.o_blk + b];
+    int2 si = tb.sinfo[g.o_blk + b];
+    if (!lists) si.y = 0;
     const uint32_t* const sdst = tb.sdst + g.o_push + si.x;
     using Ids = typename std::conditional<sizeof(T) == 8, unsigned int, uint2>::type;
     const Ids* const ids = reinterpret_cast<const Ids*>(tb.ids + (g.o_push + si.x) * kw);
@@ -141,7 +142,7 @@ __global__ void __launch_bounds__(sizeof(T) == 8 ? kStreamThreads64 : kStreamThr
 
   // the voltages of the first step
   if (lc.done == 0) {
-    send(P.cand + (int64_t)(lc.set * kTrials + lc.kcur) * P.var_cap + I.var0, nullptr, false, T(0));
+    send(P.cand + (int64_t)(lc.set * kTrials + lc.kcur) * P.var_cap + I.var0, nullptr, false, T(0), true);
     target += P.barrier_extra;
     ok = grid_barrier<NT>(bar, target, err, &s_ok);
   }
@@ -463,8 +464,12 @@ __global__ void __launch_bounds__(sizeof(T) == 8 ? kStreamThreads64 : kStreamThr
     __syncthreads();
     steps_run++;
 
-    // ---- C: the accepted voltages, and the inboxes
-    send(cur, P.cand + (int64_t)(lc.set * kTrials + lc.kcur) * P.var_cap + I.var0, true, s_kc.h);
+    // ---- C: the accepted voltages, and the inboxes.  The launch's last step has no reader for
+    // the latter (us per step at n = 10^6 with and without them there: launches of one step
+    // 299 / 256, of 32 steps 236.7 / 235.4; leaving early instead of a loop bound of zero, and
+    // skipping the barrier too, made the step's code slower: 261 / 242)
+    send(cur, P.cand + (int64_t)(lc.set * kTrials + lc.kcur) * P.var_cap + I.var0, true, s_kc.h,
+         s + 1 < nsteps && lc.done == 0);
     trace_stamp(P, s, 8);
     ok = grid_barrier<NT>(bar, target, err, &s_ok);
     trace_stamp(P, s, 9);
