@@ -556,7 +556,7 @@ def large_line(K, W, device, ranks, barrier) -> dict:
     out = {"workload": f"planted 3-SAT n={n} m={m} r=8 p0=0.08 p1=0.46, one formula, FP32",
            "n": n, "m": m}
     with dmm.Instance(f, precision="fp32", device=device) as inst:
-        kern = KERNELS[inst.launch_form]
+        kern = "k_stream (fused step, tables and voltage lists streamed through shared memory)"
         out["launch_form"] = inst.launch_form
         ms, done, _, xs = time_plain(inst, x0, K, W, ranks, barrier)
         rms, rsteps = time_resident(inst, xs, K, W)
@@ -566,7 +566,7 @@ def large_line(K, W, device, ranks, barrier) -> dict:
                 "resident": {"value": m * rsteps / (rms / 1000.0),
                              "ms_per_step": rms / max(1, rsteps)},
                 "roofline": roofline(algo, ms / K, kern,
-                                     traffic=profiled_traffic("k_staged_n1m.md"))})
+                                     traffic=profiled_traffic("k_stream_n1m.md"))})
     return out
 
 

@@ -251,11 +251,13 @@ dmm_status dmm_instance_assignment(dmm_instance* inst, int8_t* pre, int8_t* post
  *   6  the staged kernel with several clause and variable tiles per block (formulas whose
  *      tiles are too large for one of each per block)
  *   5  one block per formula
- * With the default tiles, layout and launch mode a small formula (about 18,000 clauses in FP32,
- * 13,000 in FP64) is run by one thread-block cluster, its data and exchanges in shared memory,
- * and a larger one (up to about 450,000 clauses) by blocks that keep their voltages resident
- * and exchange without grid barriers; both are reported as the form they stand in for: 4 for
- * FP32 with 3-literal clauses, else 3.
+ * With the default tiles, layout and launch mode a small formula (about 18,000 3-literal clauses
+ * in FP32, 13,000 in FP64; 10,000 and 9,400 of other lengths) is run by one thread-block cluster,
+ * its data and exchanges in shared memory, a larger one (up to about 450,000 clauses) by blocks
+ * that keep their voltages resident and exchange without grid barriers, and an FP32 one of
+ * 9,000,000 literals or more by blocks through whose shared memory its tables and voltage lists
+ * stream.  They are reported as the form they stand in for: for FP32 with 3-literal clauses 4,
+ * the streaming ones 6; else 3.
  * A negative dmm_status on error. */
 int32_t dmm_instance_launch_form(const dmm_instance* inst);
 /* No counterpart in the reference.  Test hook for the failure path of the cooperative step
