@@ -124,23 +124,35 @@ struct Unset<unsigned long long> {
 };
 
 // Exchange accesses (ordered among themselves as volatile; each entry is its own flag, so they
-// need no order against other memory and the loads around them may be batched).
-__device__ __forceinline__ int4 ld_relaxed4(const void* p) {
+// need no order against other memory and the loads around them may be batched).  The memory
+// model treats a vector access as one access per element, so the elements are whole entries:
+// with 4-byte elements the two halves of an FP64 entry could be seen one without the other.
+template <class T>
+__device__ __forceinline__ int4 ld_word(const int4* p) {
   int4 v;
-  asm volatile("ld.relaxed.gpu.global.v4.s32 {%0, %1, %2, %3}, [%4];"
-               : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w)
-               : "l"(p));
+  if constexpr (sizeof(T) == 4) {
+    asm volatile("ld.relaxed.gpu.global.v4.b32 {%0, %1, %2, %3}, [%4];"
+                 : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w)
+                 : "l"(p));
+  } else {
+    unsigned long long a, b;
+    asm volatile("ld.relaxed.gpu.global.v2.b64 {%0, %1}, [%2];" : "=l"(a), "=l"(b) : "l"(p));
+    v = make_int4((int)a, (int)(a >> 32), (int)b, (int)(b >> 32));
+  }
   return v;
 }
-__device__ __forceinline__ void st_relaxed4(void* p, int4 v) {
-  asm volatile("st.relaxed.gpu.global.v4.s32 [%0], {%1, %2, %3, %4};" ::"l"(p), "r"(v.x), "r"(v.y),
-               "r"(v.z), "r"(v.w));
+// The entries of an FP64 word.
+__host__ __device__ __forceinline__ unsigned long long entry64(int lo, int hi) {
+  return (unsigned int)lo | (unsigned long long)(unsigned int)hi << 32;
 }
-__device__ __forceinline__ void st_relaxed(float* p, float v) {
-  asm volatile("st.relaxed.gpu.global.f32 [%0], %1;" ::"l"(p), "f"(v));
-}
-__device__ __forceinline__ void st_relaxed(double* p, double v) {
-  asm volatile("st.relaxed.gpu.global.f64 [%0], %1;" ::"l"(p), "d"(v));
+template <class T>
+__device__ __forceinline__ void st_word(int4* p, int4 v) {
+  if constexpr (sizeof(T) == 4)
+    asm volatile("st.relaxed.gpu.global.v4.b32 [%0], {%1, %2, %3, %4};" ::"l"(p), "r"(v.x),
+                 "r"(v.y), "r"(v.z), "r"(v.w));
+  else
+    asm volatile("st.relaxed.gpu.global.v2.b64 [%0], {%1, %2};" ::"l"(p), "l"(entry64(v.x, v.y)),
+                 "l"(entry64(v.z, v.w)));
 }
 // Whether all entries of a word are set.
 template <class T>
@@ -149,9 +161,8 @@ __device__ __forceinline__ bool word_set(const int4& v) {
     const int u = (int)Unset<unsigned int>::bits();
     return v.x != u && v.y != u && v.z != u && v.w != u;
   } else {
-    const int lo = (int)(unsigned int)Unset<unsigned long long>::bits();
-    const int hi = (int)(Unset<unsigned long long>::bits() >> 32);
-    return (v.x != lo || v.y != hi) && (v.z != lo || v.w != hi);
+    const unsigned long long u = Unset<unsigned long long>::bits();
+    return entry64(v.x, v.y) != u && entry64(v.z, v.w) != u;
   }
 }
 template <class T>
@@ -178,7 +189,7 @@ __device__ __forceinline__ void take_words(int4* p, int q0, int step, int n, int
     bool set = true;
 #pragma unroll
     for (int r = 0; r < N; r++)
-      if (q0 + r * step < n) v[r] = ld_relaxed4(p + q0 + r * step);
+      if (q0 + r * step < n) v[r] = ld_word<T>(p + q0 + r * step);
 #pragma unroll
     for (int r = 0; r < N; r++)
       if (q0 + r * step < n) set = set && word_set<T>(v[r]);
@@ -190,7 +201,7 @@ __device__ __forceinline__ void take_words(int4* p, int q0, int step, int n, int
   }
 #pragma unroll
   for (int r = 0; r < N; r++)
-    if (q0 + r * step < n) st_relaxed4(p + q0 + r * step, unset_word<T>());
+    if (q0 + r * step < n) st_word<T>(p + q0 + r * step, unset_word<T>());
 }
 
 // A block's copy of the control state of its formula.
@@ -587,7 +598,7 @@ __global__ void __launch_bounds__(sizeof(T) == 8 ? kGridThreads64 : kGridThreads
             if (q0 + r * NT < nw) at[r] = wdst[w0 + q0 + r * NT];
 #pragma unroll
           for (int r = 0; r < 4; r++)
-            if (q0 + r * NT < nw) st_relaxed4(dst + at[r], src[q0 + r * NT]);
+            if (q0 + r * NT < nw) st_word<T>(dst + at[r], src[q0 + r * NT]);
         }
       }
       if (i + 1 < g.kc) __syncthreads();  // before the next tile reuses the area
@@ -781,7 +792,7 @@ __global__ void __launch_bounds__(sizeof(T) == 8 ? kGridThreads64 : kGridThreads
 #pragma unroll
             for (int k = 0; k < kw; k++)
               u.v[k] = s_dv[(e[r][k >> 1] >> (16 * (k & 1))) & 0xffffu];
-            st_relaxed4(in + at[r], u.q);
+            st_word<T>(in + at[r], u.q);
           }
       }
     }
