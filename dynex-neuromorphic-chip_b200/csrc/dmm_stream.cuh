@@ -71,6 +71,9 @@ __global__ void __launch_bounds__(sizeof(T) == 8 ? kStreamThreads64 : kStreamThr
     I = P.inst[g.inst];
     const volatile InstCtrl* S = P.ctrl + g.inst;
     lc.done = S->done;
+    // a wait of the launch before gave up (the host has not seen it yet): the lists and
+    // buckets are those of the abandoned step, so none is taken
+    if (*reinterpret_cast<volatile int*>(err) != 0) lc.done = -1;
     lc.step = S->step;
     lc.set = S->set;
     lc.kcur = S->kcur;

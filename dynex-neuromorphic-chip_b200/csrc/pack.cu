@@ -2344,6 +2344,10 @@ dmm_status Pack::test_barrier_timeout() {
   const dmm_status st = gr_groups_.empty() ? launch_tiles(1) : launch_grid(1);
   barrier_extra_ = 0;
   DMM_TRY(st);
+  // a run has its next launch queued before it sees the error: the forms that check for one
+  // must leave the state and the control record alone
+  if (!gr_groups_.empty()) DMM_TRY(launch_grid(1));
+  else if (stream_active_) DMM_TRY(launch_stream(1));
   DMM_CUDA(cudaStreamSynchronize(stream_));
   return check_error();
 }

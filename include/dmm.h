@@ -262,7 +262,9 @@ dmm_status dmm_instance_assignment(dmm_instance* inst, int8_t* pre, int8_t* post
 int32_t dmm_instance_launch_form(const dmm_instance* inst);
 /* No counterpart in the reference.  Test hook for the failure path of the cooperative step
  * kernels: one launch whose first grid barrier waits for one arrival more than the grid has,
- * so every block's bounded wait runs out (a few seconds); returns the status the library
+ * so every block's bounded wait runs out (a few seconds), and behind it, where the resident grid
+ * or the streaming kernel runs the formula, an ordinary one, which must take no step (a run
+ * queues a launch before it sees the error of the one before); returns the status the library
  * reports for it (DMM_ERR_CUDA, "grid barrier wait gave up ...").  The device context stays
  * usable; the instance's state is undefined afterwards (set a state before stepping). */
 dmm_status dmm_instance_test_barrier_timeout(dmm_instance* inst);
