@@ -15,6 +15,14 @@
 
 namespace dmm {
 
+// Lets launches of `fn` ask for up to `cap` bytes of dynamic shared memory.  The attribute belongs
+// to the function on the current device and is shared by all handles and threads, so it is always
+// set to the kernel's own cap, never to one launch's size: a thread that set less between another's
+// call here and its launch would have that launch rejected.
+inline cudaError_t allow_smem(const void* fn, int cap) {
+  return cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, cap);
+}
+
 constexpr int kMaxK = 25;          // longest clause (MAX_LITS_SYSTEM, dynex.cc:69)
 constexpr int kThreads = 256;      // block size of every tile kernel (fixed: reductions
                                    // over a block are part of the result definition)

@@ -50,11 +50,9 @@ cudaError_t grid_build(const GridGroup* groups, const int32_t* list_group, int n
   const int RW = std::min((max_n + 31) / 32, kXpRangeWords), kw = fp64 ? 2 : 4;
   const int smem = (max_nvt + 2 * RW) * 4;
   const void* fill = fp64 ? (const void*)k_grid_fill<true> : (const void*)k_grid_fill<false>;
-  if (smem > 48 * 1024) {
-    cudaError_t e = cudaFuncSetAttribute(k_grid_count, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-    if (e == cudaSuccess) e = cudaFuncSetAttribute(fill, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-    if (e != cudaSuccess) return e;
-  }
+  cudaError_t e = allow_smem((const void*)k_grid_count, kGridSmemMax);
+  if (e == cudaSuccess) e = allow_smem(fill, kGridSmemMax);
+  if (e != cudaSuccess) return e;
   if (t.pos)
     k_grid_order<<<dim3((unsigned)max_nvt, (unsigned)ngroups), kGridRowThreads, 0, s>>>(groups, vend, t);
   if (t.cord)

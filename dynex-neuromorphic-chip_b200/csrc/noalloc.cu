@@ -286,7 +286,7 @@ extern "C" dmm_status dmm_rhs3_f32_noalloc(const int32_t* lits, int32_t n, int32
   constexpr int kSmem = (NA_THREADS / 32) * 2 * NA_MAX_OCC * (int)sizeof(int32_t);
   int sms = 0;
   DMM_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-  DMM_CUDA(cudaFuncSetAttribute(k_na_rhs, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmem));
+  DMM_CUDA(allow_smem((const void*)k_na_rhs, kSmem));
   // a thread per slot, a warp per variable in a few rounds; at most a block per SM
   const int want = std::max((L + NA_THREADS - 1) / NA_THREADS, (n + 63) / 64);
   const int grid = std::max(1, std::min(want, sms));

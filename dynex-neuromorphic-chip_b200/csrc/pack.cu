@@ -212,6 +212,7 @@ constexpr int kXpSmemMax = 220 * 1024;  // dynamic shared memory of the staged f
 // shared-memory carve-out, and the L1 left to the gathers shrinks (measured at 0.4-1.5 million
 // variables: every tiling above the cap ran 8-30 % slower than the best one below it)
 constexpr int kXpSmemMaxMT = 193 * 1024;  // with the form's ~1.4 KB of static shared memory
+constexpr int staged_smem_max(bool mt) { return mt ? kXpSmemMaxMT : kXpSmemMax; }
 constexpr int kClusterChunk = 8;        // launches of steps_per_graph steps run() makes one of
 constexpr int kStreamSlots = 9000000;   // literals from which the streaming form runs a formula
 constexpr int kXpMaxTiles = 1 << 14;    // clause or variable tiles of the staged form, at most
@@ -768,13 +769,13 @@ dmm_status Pack::flush_adds() {
   const int smem = (kAdmitVars + (kAdmitThreads / 32) * kSortCap) * 4;
   const AdmitRec* recs = reinterpret_cast<const AdmitRec*>(A.dev);
   if (prec_ == DMM_FP64) {
-    DMM_CUDA(cudaFuncSetAttribute(k_admit<double>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+    DMM_CUDA(allow_smem((const void*)k_admit<double>, smem));
     k_admit<double><<<count, kAdmitThreads, smem, stream_>>>(
         recs, A.dev, inst_d_, ctrl_d_, lit_, vslot_, upos_, vend_, coff_, unit_,
         static_cast<double*>(cand_), static_cast<double*>(Xs_), static_cast<double*>(Xl_), active_d_,
         longv_d_, ring_tail_d_ + 2, longv_cap_);
   } else {
-    DMM_CUDA(cudaFuncSetAttribute(k_admit<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+    DMM_CUDA(allow_smem((const void*)k_admit<float>, smem));
     k_admit<float><<<count, kAdmitThreads, smem, stream_>>>(
         recs, A.dev, inst_d_, ctrl_d_, lit_, vslot_, upos_, vend_, coff_, unit_,
         static_cast<float*>(cand_), static_cast<float*>(Xs_), static_cast<float*>(Xl_), active_d_,
@@ -1205,10 +1206,10 @@ dmm_status Pack::enqueue_step(bool rhs_only, void* dv_out) {
   return DMM_OK;
 }
 
-static int occupancy_blocks(const void* fn, int threads, size_t smem = 0) {
+// cap: the kernel's largest dynamic shared memory (allow_smem)
+static int occupancy_blocks(const void* fn, int threads, size_t smem = 0, int cap = 0) {
   int b = 1;
-  if (smem > 0 &&
-      cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) {
+  if (smem > 0 && allow_smem(fn, cap) != cudaSuccess) {
     cudaGetLastError();
     return 0;
   }
@@ -1500,7 +1501,7 @@ dmm_status Pack::plan_stream(int32_t idx, bool* ok) {
     }
     stream_general_ = I.k3 == 0;
     if (occupancy_blocks(stream_kernel(fp64, stream_general_), fp64 ? kStreamThreads64 : kStreamThreads,
-                         lay.total) < 1)
+                         lay.total, kStreamSmemMax) < 1)
       return DMM_OK;
     stream_layout_ = lay;
     gr_tables_ = t;
@@ -1528,7 +1529,7 @@ dmm_status Pack::launch_stream(int32_t nsteps) {
     DMM_CUDA(cudaMemsetAsync(bar, 0, kLaunchAreaInts * sizeof(int32_t), stream_));
   launch_area_clean_ = true;
   const void* fn = stream_kernel(fp64, stream_general_);
-  DMM_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, stream_layout_.total));
+  DMM_CUDA(allow_smem(fn, kStreamSmemMax));
   const void* groups = gbuf_[kGrGroups];
   void* dv = gbuf_[kGrDv];
   void* epart = gbuf_[kGrEpart];
@@ -1695,7 +1696,8 @@ dmm_status Pack::plan_grid(const std::vector<int32_t>& cand, std::vector<int32_t
       gr_resident_--;
     gr_layout_ = grid_shape(caps, fp64, general, gr_resident_);
     const void* fn = grid_kernel(fp64, general, gr_resident_);
-    if (occupancy_blocks(fn, fp64 ? kGridThreads64 : kGridThreads, gr_layout_.total) < 1) return DMM_OK;
+    if (occupancy_blocks(fn, fp64 ? kGridThreads64 : kGridThreads, gr_layout_.total, kGridSmemMax) < 1)
+      return DMM_OK;
     gr_general_ = general;
     gr_tables_ = t;
     gr_blocks_ = (int32_t)blk.size();
@@ -1727,7 +1729,7 @@ dmm_status Pack::launch_grid(int32_t nsteps) {
   }
   gr_clean_ = true;
   const void* fn = grid_kernel(fp64, gr_general_, gr_resident_);
-  DMM_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, gr_layout_.total));
+  DMM_CUDA(allow_smem(fn, kGridSmemMax));
   const void* groups = gbuf_[kGrGroups];
   const void* blk = gbuf_[kGrBlk];
   void* epart = gbuf_[kGrEpart];
@@ -1817,12 +1819,8 @@ dmm_status Pack::prepare_xpose(int32_t idx, int TC, int TV, bool mt, bool* ok) {
   const int32_t* vend = vend_ + I.var0;
   DMM_CUDA(cudaMemsetAsync(dlist, 0, bytes[kXpDlist], stream_));
   DMM_CUDA(cudaMemsetAsync(dst, 0xFF, bytes[kXpDst], stream_));
-  if (smem_k > 48 * 1024) {
-    DMM_CUDA(cudaFuncSetAttribute(k_xp_count<kXprepThreads>,
-                                  cudaFuncAttributeMaxDynamicSharedMemorySize, smem_k));
-    DMM_CUDA(cudaFuncSetAttribute(k_xp_fill<kXprepThreads>,
-                                  cudaFuncAttributeMaxDynamicSharedMemorySize, smem_k));
-  }
+  DMM_CUDA(allow_smem((const void*)k_xp_count<kXprepThreads>, kXpSmemMax));
+  DMM_CUDA(allow_smem((const void*)k_xp_fill<kXprepThreads>, kXpSmemMax));
   k_xp_count<kXprepThreads><<<nct, kXprepThreads, smem_k, stream_>>>(lit, L, TC, TV, nvt, n, RW,
                                                                      cnt, sb, st, dcnt, spos);
   k_xp_scan<kXprepThreads><<<1, kXprepThreads, 0, stream_>>>(nct, nvt, cnt, st, dcnt, ubase,
@@ -1840,8 +1838,9 @@ dmm_status Pack::prepare_xpose(int32_t idx, int TC, int TV, bool mt, bool* ok) {
   const int bk_cap = mt ? std::max(h[7], 8) : std::max(h[2], 8);
   const int smem = mt ? xp_layout_mt(sv_cap, st_cap, bk_cap, TV).total
                       : xp_layout(sv_cap, bk_cap, TV).total;
-  if (smem > (mt ? kXpSmemMaxMT : kXpSmemMax)) return DMM_OK;
-  if (occupancy_blocks(staged_fn(tun_.var_group, mt), kStagedThreads, smem) * sms_ != grid_p_)
+  if (smem > staged_smem_max(mt)) return DMM_OK;
+  if (occupancy_blocks(staged_fn(tun_.var_group, mt), kStagedThreads, smem, staged_smem_max(mt)) * sms_ !=
+      grid_p_)
     return DMM_OK;
   xsv_cap_ = sv_cap;
   xst_cap_ = st_cap;
@@ -2097,8 +2096,7 @@ dmm_status Pack::launch_persist(int32_t nsteps) {
   launch_area_clean_ = true;
   void* args[] = {view, &nsteps, &bar, &err};
   const size_t smem = xp_active_ ? (size_t)xsmem_ : 0;
-  if (smem)
-    DMM_CUDA(cudaFuncSetAttribute(persist_fn(), cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  if (smem) DMM_CUDA(allow_smem(persist_fn(), staged_smem_max(xp_mt_)));
   const int block = xp_active_ ? kStagedThreads : persist_threads(prec_);
   DMM_CUDA(cudaLaunchCooperativeKernel(persist_fn(), dim3(grid_p_), dim3(block), args, smem,
                                        stream_));
@@ -2203,7 +2201,7 @@ dmm_status Pack::cluster_config(const ClusterLaunch& L, cudaLaunchConfig_t* cfg,
                                 cudaLaunchAttribute* at) {
   const bool fp64 = prec_ == DMM_FP64;
   const void* fn = cluster_kernel(fp64, L.general);
-  DMM_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, L.smem));
+  DMM_CUDA(allow_smem(fn, kClusterSmemMax));
   if (L.R > 8) DMM_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
   *cfg = cudaLaunchConfig_t{};
   *at = cudaLaunchAttribute{};
@@ -2272,8 +2270,7 @@ template <int G>
 static dmm_status launch_inst_g(const PackView<float>& v, const int32_t* order, int count,
                                 int nsteps, int* queue, int grid, cudaStream_t s) {
   // function attributes are per device: set it on the current one (a cheap driver call)
-  DMM_CUDA(cudaFuncSetAttribute(k_inst<G>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                (int)kInstSmem));
+  DMM_CUDA(allow_smem((const void*)k_inst<G>, (int)kInstSmem));
   k_inst<G><<<grid, kInstThreads, kInstSmem, s>>>(v, order, count, nsteps, queue);
   DMM_CUDA(cudaGetLastError());
   return DMM_OK;
