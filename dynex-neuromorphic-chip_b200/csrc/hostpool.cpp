@@ -21,10 +21,6 @@ namespace {
 class Pool {
  public:
   ~Pool() {
-    if (getpid() != pid_) {  // a forked child: the threads are the parent's
-      for (auto& t : threads_) t.detach();
-      return;
-    }
     {
       std::lock_guard<std::mutex> g(mu_);
       stop_ = true;
@@ -32,6 +28,7 @@ class Pool {
     cv_.notify_all();
     for (auto& t : threads_) t.join();
   }
+  bool own_process() const { return getpid() == pid_; }
 
   void run(int parts, const std::function<void(int)>& f) {
     std::unique_lock<std::mutex> user(user_mu_, std::try_to_lock);
@@ -59,7 +56,7 @@ class Pool {
 
  private:
   bool start() {
-    if (getpid() != pid_) return false;
+    if (!own_process()) return false;
     if (!threads_.empty()) return true;
     const int hw = (int)std::thread::hardware_concurrency();
     const int want = std::min(kPoolHelpers, hw - 1);
@@ -115,9 +112,19 @@ class Pool {
   std::atomic<int> taken_{0}, left_{0}, in_{0};
 };
 
+// Ended with the process.  A forked child has none of the threads but a copy of their state, where
+// they still wait: destroying the condition variable there would wait for them for ever, so the
+// child leaves the pool as it is.
+struct PoolOwner {
+  Pool* const p = new Pool;
+  ~PoolOwner() {
+    if (p->own_process()) delete p;
+  }
+};
+
 Pool& pool() {
-  static Pool p;
-  return p;
+  static PoolOwner o;
+  return *o.p;
 }
 
 constexpr int64_t kTouchBytes = int64_t(4) << 20;
