@@ -14,22 +14,28 @@
 // most NA_MAX_OCC literal slots.  The clause memory rate is the scalar alpha of the
 // parameters (no per-clause alpha).
 //
-// One cooperative launch does everything: it checks the literals, evaluates the clauses and
-// counts occurrences, lays out and fills the variables' slot lists, and sums them; a failed
-// check ends it before dxdt or loc is written.  The call then reads the counters (literals out
-// of range, over-long variable lists; written to page-locked host memory), waiting for the
-// caller's stream once, so it blocks the calling thread until the work queued before it and
-// its own finish.
+// Four launches: one checks the literals and counts occurrences, one lays out the variables' slot
+// lists, one evaluates the clauses and fills the lists, one sums them; a failed check keeps the
+// last two from writing dxdt or loc.  The last block of the last launch writes the counters
+// (literals out of range, over-long variable lists) to page-locked host memory and the call waits
+// for the caller's stream once to read them, so it blocks the calling thread until the work
+// queued before it and its own finish.
 //
-// As nine launches and two waits a call took 105 us at n = 8,009, m = 64,007, nearly all of it
-// launch gaps and host round trips; with the one launch it takes 52, about 30 of them the
-// kernel (three grid barriers and the atomics that count and place 192,021 slots).
+// The launches are ordinary ones: a block runs wherever an SM has room.  One cooperative launch
+// with three grid barriers needs room for all its blocks at once, so it would wait for every SM
+// that a kernel on another of the caller's streams holds, and could not run at all beside one that
+// waits for this call's result.  As programmatic dependents (na_wait) they cost no more than the
+// one launch did; what is left is launch and host latency, the atomics that count and place the
+// slots, and the chain of dependent loads of a list.  us per call at (n, m) = (1,000, 8,000) /
+// (8,009, 64,007) / (32,000, 65,536): nine launches with two host waits 67 / 98 / 155; one
+// cooperative launch 30.6 / 43.9 / 44.3; four launches one after another 36.1 / 50.1 / 46.0; as
+// dependents 30.9 / 43.1 / 40.2.
 //
 // Every call uses the same array and leaves its contents behind, but for the parts that must
 // start at zero: it zeroes them at its end and checks them at its start (counts left by calls
-// that raced are cleared and the launch repeated).  Calls whose work overlaps on the GPU (different streams,
-// or different host threads on one device) race on the array and must be serialized by
-// the caller.
+// that raced are cleared and the launches repeated).  Calls whose work overlaps on the GPU
+// (different streams, or different host threads on one device) race on the array and must be
+// serialized by the caller.
 //
 // Host code cannot use g_na_scratch's name as a device address.  On its first call on a
 // device, the entry point looks the address up with cudaGetSymbolAddress while that
@@ -57,10 +63,9 @@ struct NaScratch {
   float C[NA_MAX_CLAUSES];      // C_m of each clause
   int32_t cnt[NA_MAX_VARS];     // occurrences (zero between calls)
   int32_t fill[NA_MAX_VARS];    // list cursors: the lists' ends once filled
-  // [0] unsatisfied clauses, [1] long lists, [2] bad literals, [3] slots handed out (zero
-  // between calls), [4] a grid-barrier wait gave up
+  // [0] unsatisfied clauses, [1] long lists, [2] bad literals, [3] slots handed out, [4] blocks
+  // of the last launch that have left (all zero between calls)
   int32_t counters[8];
-  unsigned int bar[kLaunchAreaInts];  // grid barrier, left zeroed by every call
 };
 static_assert(sizeof(NaScratch) < (size_t(22) << 20) / 10, "about 2.1 MB, as documented");
 
@@ -123,79 +128,94 @@ __device__ __forceinline__ float na_sum(const NaScratch* s, int first, int d, in
   return p;
 }
 
-// flags (host memory): counters [1], [2] and [4] of the call.
-__global__ void __launch_bounds__(NA_THREADS, 1)
-    k_na_rhs(NaScratch* s, const int32_t* __restrict__ lits, int n, int m, const float* x,
-             ClauseConsts<float> kc, float* dxdt, int32_t* loc, volatile int32_t* flags) {
+// The launches after the first are programmatic dependents: their blocks may start once every block
+// of the launch before has started (all of them are on an SM by then, so none waits for room that
+// a later launch holds) and wait here until it has ended and its writes are visible.
+__device__ __forceinline__ void na_next() { asm volatile("griddepcontrol.launch_dependents;"); }
+__device__ __forceinline__ void na_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
+// Literals in range and occurrence counts.
+__global__ void __launch_bounds__(NA_THREADS)
+    k_na_count(NaScratch* s, const int32_t* __restrict__ lits, int n, int m) {
+  na_next();
+  int bad = 0;
+  for (int q = blockIdx.x * NA_THREADS + threadIdx.x; q < 3 * m; q += gridDim.x * NA_THREADS) {
+    const int l = lits[q];
+    if (l == 0 || l > n || l < -n) bad++;
+    else atomicAdd(&s->cnt[abs(l) - 1], 1);
+  }
+  bad = warp_sum_i(bad);
+  if ((threadIdx.x & 31) == 0 && bad) atomicAdd(&s->counters[2], bad);
+}
+
+// A range for every list (their order does not matter); over-long lists.
+__global__ void __launch_bounds__(NA_THREADS) k_na_lists(NaScratch* s, int n) {
+  na_next();
+  na_wait();
+  const int lane = threadIdx.x & 31;
+  const int v = blockIdx.x * NA_THREADS + threadIdx.x;  // (whole warps: the grid covers n)
+  const int c = v < n ? s->cnt[v] : 0;
+  int incl = c;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const int y = __shfl_up_sync(0xffffffffu, incl, o);
+    if (lane >= o) incl += y;
+  }
+  int first = 0;
+  if (lane == 31) first = atomicAdd(&s->counters[3], incl);
+  first = __shfl_sync(0xffffffffu, first, 31);
+  if (v < n) s->fill[v] = first + incl - c;
+  if (c > NA_MAX_OCC) atomicAdd(&s->counters[1], 1);
+}
+
+// What the first two launches found: 0 nothing, 1 a check failed, 2 the counts do not add up (they
+// were not all zero before the call).
+__device__ __forceinline__ int na_fault(const NaScratch* s, int m) {
+  const int longs = s->counters[1], bad = s->counters[2], slots = s->counters[3];
+  return slots + bad != 3 * m ? 2 : bad || longs ? 1 : 0;
+}
+
+__global__ void __launch_bounds__(NA_THREADS)
+    k_na_clause(NaScratch* s, const int32_t* __restrict__ lits, int n, int m,
+                const float* __restrict__ x, ClauseConsts<float> kc) {
+  na_next();
+  na_wait();
+  if (na_fault(s, m)) return;
+  int unsat = 0;
+  for (int c = blockIdx.x * NA_THREADS + threadIdx.x; c < m; c += gridDim.x * NA_THREADS) {
+    const int l0 = lits[3 * c], l1 = lits[3 * c + 1], l2 = lits[3 * c + 2];
+    const int p0 = atomicAdd(&s->fill[abs(l0) - 1], 1), p1 = atomicAdd(&s->fill[abs(l1) - 1], 1),
+              p2 = atomicAdd(&s->fill[abs(l2) - 1], 1);
+    float u0, u1, u2;
+    bool ss;
+    const float C = clause3(l0, l1, l2, x[abs(l0) - 1], x[abs(l1) - 1], x[abs(l2) - 1], x[n + c],
+                            x[n + m + c], kc, u0, u1, u2, ss);
+    s->list[p0] = make_int2(3 * c, __float_as_int(u0));
+    s->list[p1] = make_int2(3 * c + 1, __float_as_int(u1));
+    s->list[p2] = make_int2(3 * c + 2, __float_as_int(u2));
+    s->C[c] = C;
+    unsat += !(C < 0.5f);
+  }
+  unsat = warp_sum_i(unsat);
+  if ((threadIdx.x & 31) == 0 && unsat) atomicAdd(&s->counters[0], unsat);
+}
+
+// dV of every variable, dXs and dXl of every clause (x may be dxdt: an entry is read by the thread
+// that writes it).  The last block to leave reports and clears the counters.  flags (host memory):
+// over-long lists, bad literals, counts that do not add up.
+__global__ void __launch_bounds__(NA_THREADS)
+    k_na_sum(NaScratch* s, int n, int m, const float* x, ClauseConsts<float> kc, float* dxdt,
+             int32_t* loc, volatile int32_t* flags) {
   extern __shared__ int32_t na_smem[];  // 2 NA_MAX_OCC per warp
-  __shared__ int s_ok;
   const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
   const int gt = blockIdx.x * NA_THREADS + tid, GT = gridDim.x * NA_THREADS;
-  unsigned int target = 0;
-  auto counter = [&](int k) { return *reinterpret_cast<volatile int32_t*>(&s->counters[k]); };
-  auto barrier = [&]() {
-    return grid_barrier<NA_THREADS>(s->bar, target, &s->counters[4], &s_ok);
-  };
-  {  // literals and occurrence counts
-    int bad = 0;
-    for (int q = gt; q < 3 * m; q += GT) {
-      const int l = lits[q];
-      if (l == 0 || l > n || l < -n) bad++;
-      else atomicAdd(&s->cnt[abs(l) - 1], 1);
-    }
-    bad = warp_sum_i(bad);
-    if (lane == 0 && bad) atomicAdd(&s->counters[2], bad);
-  }
-  bool ok = barrier();
-  const int bad_all = ok ? counter(2) : 0;  // grid-uniform
-  if (ok) {  // a range for every list (their order does not matter)
-    for (int v0 = blockIdx.x * NA_THREADS + 32 * w; v0 < n; v0 += GT) {
-      const int v = v0 + lane;
-      const int c = v < n ? __ldcg(s->cnt + v) : 0;
-      int incl = c;
-#pragma unroll
-      for (int o = 1; o < 32; o <<= 1) {
-        const int y = __shfl_up_sync(0xffffffffu, incl, o);
-        if (lane >= o) incl += y;
-      }
-      int first = 0;
-      if (lane == 31) first = atomicAdd(&s->counters[3], incl);
-      first = __shfl_sync(0xffffffffu, first, 31);
-      if (v < n) s->fill[v] = first + incl - c;
-      if (c > NA_MAX_OCC) atomicAdd(&s->counters[1], 1);
-    }
-    ok = barrier();
-  }
-  const int long_all = ok ? counter(1) : 0;
-  // the counts must add up: they were not all zero before this call otherwise
-  const bool dirty = ok && counter(3) + bad_all != 3 * m;
-  if (ok && (bad_all || long_all || dirty)) {  // nothing is written to dxdt and loc
-    if (dirty && gt == 0) atomicExch(&s->counters[4], 2);
+  na_wait();
+  const int fault = na_fault(s, m);
+  if (fault) {  // nothing is written to dxdt and loc
     for (int v = gt; v < n; v += GT) s->cnt[v] = 0;
-    ok = false;
-  } else if (ok) {
-    int unsat = 0;
-    for (int c = gt; c < m; c += GT) {
-      const int l0 = lits[3 * c], l1 = lits[3 * c + 1], l2 = lits[3 * c + 2];
-      const int p0 = atomicAdd(&s->fill[abs(l0) - 1], 1), p1 = atomicAdd(&s->fill[abs(l1) - 1], 1),
-                p2 = atomicAdd(&s->fill[abs(l2) - 1], 1);
-      float u0, u1, u2;
-      bool ss;
-      const float C = clause3(l0, l1, l2, x[abs(l0) - 1], x[abs(l1) - 1], x[abs(l2) - 1],
-                              x[n + c], x[n + m + c], kc, u0, u1, u2, ss);
-      s->list[p0] = make_int2(3 * c, __float_as_int(u0));
-      s->list[p1] = make_int2(3 * c + 1, __float_as_int(u1));
-      s->list[p2] = make_int2(3 * c + 2, __float_as_int(u2));
-      s->C[c] = C;
-      unsat += !(C < 0.5f);
-    }
-    unsat = warp_sum_i(unsat);
-    if (lane == 0 && unsat) atomicAdd(&s->counters[0], unsat);
-    ok = barrier();
-  }
-  if (ok) {  // dV of every variable, dXs and dXl of every clause
+  } else {
     for (int v = blockIdx.x * (NA_THREADS / 32) + w; v < n; v += gridDim.x * (NA_THREADS / 32)) {
-      const int d = __ldcg(s->cnt + v), end = __ldcg(s->fill + v);
+      const int d = s->cnt[v], end = s->fill[v];
       const float dv = na_sum(s, end - d, d, na_smem + w * 2 * NA_MAX_OCC, lane);
       if (lane == 0) {
         dxdt[v] = dv;
@@ -204,23 +224,21 @@ __global__ void __launch_bounds__(NA_THREADS, 1)
     }
     for (int c = gt; c < m; c += GT) {
       const float xs = clampv(x[n + c], 0.f, 1.f);
-      const float C = s->C[c];  // this thread's own
+      const float C = s->C[c];
       dxdt[n + c] = mul(mul(kc.beta, add(xs, kc.eps)), sub(C, kc.gamma));
       dxdt[n + m + c] = mul(kc.alpha, sub(C, kc.delta));
     }
-    if (gt == 0) *loc = counter(0);
+    if (gt == 0) *loc = s->counters[0];
   }
-  // the last block to leave reports, and clears what must start at zero
   __syncthreads();
   if (tid == 0) {
     __threadfence();
-    if (atomicAdd(s->bar + 1, 1u) == gridDim.x - 1) {
-      flags[0] = counter(1);
-      flags[1] = counter(2);
-      flags[2] = counter(4);
-      for (int k = 0; k < 8; k++) *reinterpret_cast<volatile int32_t*>(&s->counters[k]) = 0;
-      for (int k = 0; k < kLaunchAreaInts; k++)
-        *reinterpret_cast<volatile unsigned int*>(&s->bar[k]) = 0u;
+    if (atomicAdd(&s->counters[4], 1) == (int)gridDim.x - 1) {
+      __threadfence();
+      flags[0] = s->counters[1];
+      flags[1] = s->counters[2];
+      flags[2] = fault == 2;
+      for (int k = 0; k < 8; k++) s->counters[k] = 0;
       __threadfence_system();
     }
   }
@@ -286,23 +304,42 @@ extern "C" dmm_status dmm_rhs3_f32_noalloc(const int32_t* lits, int32_t n, int32
   constexpr int kSmem = (NA_THREADS / 32) * 2 * NA_MAX_OCC * (int)sizeof(int32_t);
   int sms = 0;
   DMM_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-  DMM_CUDA(allow_smem((const void*)k_na_rhs, kSmem));
-  // a thread per slot, a warp per variable in a few rounds; at most a block per SM
-  const int want = std::max((L + NA_THREADS - 1) / NA_THREADS, (n + 63) / 64);
-  const int grid = std::max(1, std::min(want, sms));
+  DMM_CUDA(allow_smem((const void*)k_na_sum, kSmem));
+  // a thread per slot or clause (at most two blocks per SM), a warp per variable in a few rounds
+  // (the sorters take half an SM's shared memory each)
+  auto blocks = [&](int64_t threads, int most) {
+    return (unsigned)std::max<int64_t>(1, std::min<int64_t>((threads + NA_THREADS - 1) / NA_THREADS, most));
+  };
+  const unsigned g_slots = blocks(L, 2 * sms), g_vars = blocks(n, NA_MAX_VARS / NA_THREADS),
+                 g_clauses = blocks(m, 2 * sms), g_sum = blocks(std::max<int64_t>(m, 8 * (int64_t)n), sms);
   volatile int32_t* hf = flags;
-  void* args[] = {&s, &lits, &n, &m, &x, &kc, &dxdt, &loc, &flags};
+  cudaLaunchAttribute at{};
+  at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at.val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t cfg{};
+  cfg.blockDim = dim3(NA_THREADS);
+  cfg.stream = st;
+  cfg.attrs = &at;
+  cfg.numAttrs = 1;
   for (int attempt = 0; attempt < 2; attempt++) {
     hf[0] = hf[1] = hf[2] = 0;
-    DMM_CUDA(cudaLaunchCooperativeKernel((const void*)k_na_rhs, dim3((unsigned)grid),
-                                         dim3(NA_THREADS), args, (size_t)kSmem, st));
+    k_na_count<<<g_slots, NA_THREADS, 0, st>>>(s, lits, n, m);
+    DMM_CUDA(cudaGetLastError());
+    cfg.gridDim = dim3(g_vars);
+    DMM_CUDA(cudaLaunchKernelEx(&cfg, k_na_lists, s, n));
+    cfg.gridDim = dim3(g_clauses);
+    DMM_CUDA(cudaLaunchKernelEx(&cfg, k_na_clause, s, lits, n, m, x, kc));
+    cfg.gridDim = dim3(g_sum);
+    cfg.dynamicSmemBytes = kSmem;
+    DMM_CUDA(cudaLaunchKernelEx(&cfg, k_na_sum, s, n, m, x, kc, dxdt, loc, hf));
+    cfg.dynamicSmemBytes = 0;
     DMM_CUDA(cudaStreamSynchronize(st));
     if (hf[2] == 0) break;
-    // the scratch was not as a finished call leaves it (2), or a wait gave up (1)
+    // the scratch was not as a finished call leaves it
     DMM_CUDA(cudaMemsetAsync(s, 0, sizeof(NaScratch), st));
     DMM_CUDA(cudaStreamSynchronize(st));
-    if (hf[2] == 1 || attempt == 1) {
-      set_error("dmm_rhs3_f32_noalloc: grid barrier wait gave up");
+    if (attempt == 1) {
+      set_error("dmm_rhs3_f32_noalloc: another call used the scratch at the same time");
       return DMM_ERR_CUDA;
     }
   }

@@ -304,9 +304,9 @@ dmm_status dmm_instance_trace_phases(dmm_instance* inst, int32_t nsteps, double*
  * Intermediates live in one fixed __device__ array (about 2.1 MB per GPU, held until the
  * process exits), so n <= 32768, m <= 65536 and at most 1024 literal slots per variable;
  * larger formulas are rejected with DMM_ERR_ARG, literals outside [-n, n] or zero with
- * DMM_ERR_LITERAL.  These checks run on the device, in the one launch that then evaluates the
+ * DMM_ERR_LITERAL.  These checks run on the device, before the launches that evaluate the
  * right-hand side, and the call waits for the stream to read their result, so it blocks the
- * calling thread.  The first call on a device looks up the array's address.  Calls
+ * calling thread.  Its launches are ordinary ones: they need no SM to themselves.  The first call on a device looks up the array's address.  Calls
  * share the array: calls that overlap on the GPU race and must be serialized by the
  * caller.  Results equal dmm_instance_rhs on an FP32 instance. */
 dmm_status dmm_rhs3_f32_noalloc(const int32_t* lits, int32_t n, int32_t m, const float* x,
