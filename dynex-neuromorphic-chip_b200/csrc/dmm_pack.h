@@ -195,6 +195,7 @@ class Pack {
   // when it does not go there
   dmm_status stage_add(const InstDesc& I, int32_t idx, const int32_t* lits,
                        const int64_t* clause_off, bool units, const double* x0, bool* done);
+  int64_t admit_head() const;
   dmm_status build_csr(const InstDesc& I, const int32_t* lits);
   // sorts the slot lists longer than the device sorter (reported by the CSR builds since
   // the last call); runs before the CSR is first used
@@ -377,7 +378,7 @@ class Pack {
          kGrDlo, kGrOut, kGrSync, kGrEpart, kGrIds, kGrBtot, kGrPtot, kGrDv, kGrBufs };
   void* gbuf_[kGrBufs] = {};
   int64_t gbuf_cap_[kGrBufs] = {};
-  // blocks of formulas laid aside (two, filled in turn) and their device copies
+  // blocks of formulas laid aside (two, filled in turn) and their device copies, at most 16 MB each
   static constexpr int64_t kAdmitBytes = int64_t(16) << 20;
   static constexpr int kAdmitRecs = 1024;
   struct AdmitBlock {
@@ -390,6 +391,7 @@ class Pack {
   };
   AdmitBlock admit_[2];
   int admit_cur_ = 0;
+  bool admit_off_ = false;  // there was no memory for a block
   // largest bucket and slot count of a block for each cluster size, per formula
   struct ClusterNeed {
     uint64_t serial = 0;

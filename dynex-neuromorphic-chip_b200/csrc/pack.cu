@@ -679,6 +679,11 @@ static dmm_status upload_alpha(T* dst, const double* a, int32_t m, cudaStream_t 
   return DMM_OK;
 }
 
+// Bytes of the records at the start of a block.
+int64_t Pack::admit_head() const {
+  return (std::min<int64_t>(kAdmitRecs, caps_.insts) * (int64_t)sizeof(AdmitRec) + 15) & ~int64_t(15);
+}
+
 dmm_status Pack::stage_add(const InstDesc& I, int32_t idx, const int32_t* lits,
                            const int64_t* clause_off, bool units, const double* x0, bool* done) {
   *done = false;
@@ -686,19 +691,31 @@ dmm_status Pack::stage_add(const InstDesc& I, int32_t idx, const int32_t* lits,
   auto al = [](int64_t b) { return (b + 15) & ~int64_t(15); };
   const int64_t b_lit = al(4 * L), b_coff = I.k3 ? 0 : al(4 * m), b_unit = units ? al(n) : 0,
                 b_x = al((n + 2 * m) * (int64_t)tsize_);
-  const int64_t head = (int64_t)kAdmitRecs * sizeof(AdmitRec);
-  if (n > kAdmitVars || L > kAdmitSlots || head + b_lit + b_coff + b_unit + b_x > kAdmitBytes)
+  // a block holds what the pack can, up to kAdmitBytes: a batch of two small formulas takes no
+  // 16 MB of device and page-locked memory for them
+  const int64_t recs = std::min<int64_t>(kAdmitRecs, caps_.insts), head = admit_head();
+  const int64_t cap = std::min<int64_t>(
+      kAdmitBytes, head + 4 * caps_.slots + 4 * caps_.clauses + caps_.vars +
+                       (int64_t)tsize_ * (caps_.vars + 2 * caps_.clauses) + 64 * recs);
+  if (n > kAdmitVars || L > kAdmitSlots || head + b_lit + b_coff + b_unit + b_x > cap)
     return DMM_OK;
-  if (admit_[admit_cur_].count == kAdmitRecs ||
-      head + admit_[admit_cur_].used + b_lit + b_coff + b_unit + b_x > kAdmitBytes)
+  if (admit_[admit_cur_].count == recs ||
+      head + admit_[admit_cur_].used + b_lit + b_coff + b_unit + b_x > cap)
     DMM_TRY(flush_adds());
   AdmitBlock& A = admit_[admit_cur_];
   if (!A.host) {
     void *h = nullptr, *dv = nullptr;
-    DMM_CUDA(pinned_alloc(&h, kAdmitBytes));
+    cudaError_t e = pinned_alloc(&h, cap);
+    if (e == cudaSuccess) e = dev_alloc(&dv, cap);
+    if (e == cudaErrorMemoryAllocation) {  // formulas are added one by one without the blocks
+      cudaGetLastError();
+      pinned_free(h);
+      admit_off_ = true;
+      return DMM_OK;
+    }
     A.host = static_cast<unsigned char*>(h);
-    DMM_CUDA(dev_alloc(&dv, kAdmitBytes));
     A.dev = static_cast<unsigned char*>(dv);
+    DMM_CUDA(e);
     DMM_CUDA(cudaEventCreateWithFlags(&A.sent, cudaEventDisableTiming));
   }
   if (A.busy) {  // its previous contents are still on their way
@@ -758,7 +775,7 @@ dmm_status Pack::stage_add(const InstDesc& I, int32_t idx, const int32_t* lits,
 dmm_status Pack::flush_adds() {
   AdmitBlock& A = admit_[admit_cur_];
   if (A.count == 0) return DMM_OK;
-  const int64_t head = (int64_t)kAdmitRecs * sizeof(AdmitRec);
+  const int64_t head = admit_head();
   const int count = A.count;
   const int64_t used = A.used;
   A.count = 0;
@@ -819,7 +836,7 @@ dmm_status Pack::add(const int32_t* lits, const int64_t* clause_off, int32_t n, 
     return DMM_ERR_BUDGET;
   }
   // small formulas with an initial state are laid aside and unpacked many at a time
-  if (x0 && !alpha_cm && !device_literal_check && n <= kAdmitVars && L <= kAdmitSlots) {
+  if (x0 && !alpha_cm && !device_literal_check && !admit_off_ && n <= kAdmitVars && L <= kAdmitSlots) {
     bool k3 = false, units = true, done = false;
     dmm_status st = validate_formula(lits, clause_off, n, m, &k3, &units, true);
     InstDesc I{};
