@@ -232,6 +232,7 @@ class Pack {
   dmm_status grid_tables(const std::vector<GridGroup>& groups, const std::vector<int32_t>& map,
                          int nblocks, const GridSizes& z, bool stream, GridTables* t,
                          std::vector<int32_t>* out);
+  void drop_grid_tables();
   double cluster_step_us() const;
   double grid_step_us(const std::vector<int32_t>& list) const;
   dmm_status grid_buffer(int which, int64_t bytes);

@@ -1357,6 +1357,18 @@ void Pack::grid_place(GridGroup* g, GridSizes* z) const {
   z->max_rows = std::max(z->max_rows, g->nvt + g->B);
 }
 
+// Gives the tables back after an allocation failed, so that the forms that need none (or less)
+// can run.
+void Pack::drop_grid_tables() {
+  cudaGetLastError();
+  clear_error();
+  for (int q = 0; q < kGrBufs; q++) {
+    if (gbuf_[q]) retire(gbuf_[q]);
+    gbuf_[q] = nullptr;
+    gbuf_cap_[q] = 0;
+  }
+}
+
 // Allocates and builds the tables (map: group of every variable list; nblocks: blocks of the
 // launch); out: what grid_build reports per group.
 dmm_status Pack::grid_tables(const std::vector<GridGroup>& groups, const std::vector<int32_t>& map,
@@ -1506,7 +1518,12 @@ dmm_status Pack::plan_stream(int32_t idx, bool* ok) {
     const std::vector<int32_t> map((size_t)g.NL, 0);
     GridTables t{};
     std::vector<int32_t> out;
-    DMM_TRY(grid_tables(groups, map, B, z, true, &t, &out));
+    const dmm_status st = grid_tables(groups, map, B, z, true, &t, &out);
+    if (st == DMM_ERR_NOMEM) {
+      drop_grid_tables();
+      return DMM_OK;
+    }
+    DMM_TRY(st);
     const StreamLayout lay = stream_shape(out[1], out[2], out[3], g.TV * g.kv, fp64);
     if (out[0] == 3 || (out[0] == 0 && lay.total > kStreamSmemMax && out[3] > out[2])) {
       kv_min = kv + 1;
@@ -1668,7 +1685,12 @@ dmm_status Pack::plan_grid(const std::vector<int32_t>& cand, std::vector<int32_t
     gr_key_.clear();
     GridTables t{};
     std::vector<int32_t> out;
-    DMM_TRY(grid_tables(groups, blk, (int)blk.size(), z, false, &t, &out));
+    const dmm_status st = grid_tables(groups, blk, (int)blk.size(), z, false, &t, &out);
+    if (st == DMM_ERR_NOMEM) {
+      drop_grid_tables();
+      return DMM_OK;
+    }
+    DMM_TRY(st);
     // what the tables need; a formula whose tiles came out too large gets more of them
     GridCaps caps{};
     bool again = false;

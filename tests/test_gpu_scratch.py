@@ -86,3 +86,51 @@ def test_blocks_for_added_formulas_refused():
         got = outcome(b, forms)
     b.close()
     same(got, want)
+
+
+@pytest.mark.parametrize("prec,sizes", [("fp64", [(12000, 96000)] * 8), ("fp32", [(30000, 240000)] * 3)])
+def test_tables_of_the_resident_form_refused(prec, sizes):
+    forms, b = make(prec, sizes)
+    want = outcome(b, forms)
+    b.close()
+    forms, b = make(prec, sizes)
+    with device_filled(48 * MB):
+        got = outcome(b, forms)
+    # with memory again the next run builds the tables after all
+    again = outcome_again(b, forms)
+    b.close()
+    same(got, want)
+    same(again, want)
+
+
+def outcome_again(batch, forms):
+    batch.set_tuning(launch_mode=0)
+    for k, f in enumerate(forms):
+        batch.set_state_at(k, dmm.initial_state_uniform(f, 50 + k), 0.0)
+    batch.run()
+    return [(batch.result(k), batch.state(k)) for k in range(len(forms))]
+
+
+def test_tables_of_the_streaming_form_refused():
+    import torch
+
+    form, _ = dmm.generate_planted(400_000, 3_200_000, 0.08, 0.58, seed=3)
+    x0 = dmm.initial_state_uniform(form, 4)
+
+    def run():
+        with dmm.Instance(form, precision="fp32") as inst:
+            inst.set_state(x0)
+            r = inst.step(6)
+            return r.steps, r.t, r.loc, inst.get_state()[0]
+
+    want = run()
+    # room for the formula and, beside it, for less than the streaming form's tables
+    lib().dmm_release_cached_memory()
+    before = torch.cuda.mem_get_info()[0]
+    inst = dmm.Instance(form, precision="fp32")
+    inst.set_state(x0)
+    whole = before - torch.cuda.mem_get_info()[0]
+    inst.close()
+    with device_filled(whole - 100 * MB):
+        got = run()
+    assert got[:3] == want[:3] and np.array_equal(got[3], want[3])
