@@ -235,7 +235,13 @@ KERNELS = {"staged": "k_staged (fused step, staged form)",
            "staged-multi": "k_staged (fused step, staged form, several tiles per block)",
            "cooperative-single": "k_persist (fused step, single formula)",
            "cooperative": "k_persist (fused step)",
-           "two-kernel": "k_clause + k_var", "one-block-per-formula": "k_inst"}
+           "two-kernel": "k_clause + k_var", "one-block-per-formula": "k_inst",
+           "cluster": "k_cluster (fused step, one thread-block cluster)",
+           "resident-grid": "k_grid (fused step, voltages resident in shared memory)",
+           "streaming": "k_stream (fused step, tables and voltage lists streamed through shared "
+                        "memory)"}
+# committed ncu summary of each kernel on the formula of 10^6 variables
+LARGE_PROFILES = {"streaming": "k_stream_n1m.md", "staged-multi": "k_staged_n1m.md"}
 
 
 def profiled_ratio(summary: str) -> float | None:
@@ -530,7 +536,7 @@ def fp64_line(form, x0, K, W, device, ranks, barrier) -> dict:
 
     n, m = form.n, form.m
     with dmm.Instance(form, precision="fp64", device=device) as inst:
-        kern = KERNELS[inst.launch_form]
+        kern = KERNELS[inst.step_kernel]
         ms, done, _, xs = time_plain(inst, x0, K, W, ranks, barrier)
         rms, rsteps = time_resident(inst, xs, K, W)
     e_t, e_steps, h2d, d2h = time_e2e(form, x0, "fp64", device, barrier, reps=5)
@@ -556,8 +562,8 @@ def large_line(K, W, device, ranks, barrier) -> dict:
     out = {"workload": f"planted 3-SAT n={n} m={m} r=8 p0=0.08 p1=0.46, one formula, FP32",
            "n": n, "m": m}
     with dmm.Instance(f, precision="fp32", device=device) as inst:
-        kern = "k_stream (fused step, tables and voltage lists streamed through shared memory)"
-        out["launch_form"] = inst.launch_form
+        kern = inst.step_kernel
+        out["launch_form"], out["step_kernel"] = inst.launch_form, kern
         ms, done, _, xs = time_plain(inst, x0, K, W, ranks, barrier)
         rms, rsteps = time_resident(inst, xs, K, W)
     algo = 28 * m + 8 * n
@@ -565,8 +571,8 @@ def large_line(K, W, device, ranks, barrier) -> dict:
                 "ms_per_step": ms / K,
                 "resident": {"value": m * rsteps / (rms / 1000.0),
                              "ms_per_step": rms / max(1, rsteps)},
-                "roofline": roofline(algo, ms / K, kern,
-                                     traffic=profiled_traffic("k_stream_n1m.md"))})
+                "roofline": roofline(algo, ms / K, KERNELS[kern],
+                                     traffic=profiled_traffic(LARGE_PROFILES.get(kern, "")))})
     return out
 
 
@@ -603,7 +609,7 @@ def main():
     n, m = form.n, form.m
     K, W = a.steps, max(3, a.warmup)
     inst = dmm.Instance(form, precision="fp32", device=local)
-    form_name = inst.launch_form
+    form_name, kernel_name = inst.launch_form, inst.step_kernel
     step_ms, steps_done, clocks, x0 = time_plain(inst, x0, K, W, ranks, barrier, local)
     t_max = max_over_ranks(step_ms)
     total_updates = sum_over_ranks(m * steps_done)
@@ -669,7 +675,7 @@ def main():
                     "path": f"dmm_instance_create + set_state + {E2E_STEPS} steps + assignment "
                             "readback, pinned host buffers"},
             "gpu_launches": K,
-            "roofline": roofline(algo_bytes, launch_ms, KERNELS[form_name],
+            "roofline": roofline(algo_bytes, launch_ms, KERNELS[kernel_name],
                                  traffic=profiled_traffic("k_staged_n100k.md"),
                                  note="traffic: ncu DRAM bytes of one launch of this kernel on "
                                       "this workload, read from the committed profile summary"),

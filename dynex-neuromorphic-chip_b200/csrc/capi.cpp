@@ -318,6 +318,12 @@ int32_t dmm_instance_launch_form(const dmm_instance* inst) {
   return inst->pack->launch_form();
 }
 
+int32_t dmm_instance_step_kernel(const dmm_instance* inst) {
+  if (!inst) return DMM_ERR_ARG;
+  dmm::DeviceScope device_scope(inst->pack->device());
+  return inst->pack->step_kernel();
+}
+
 dmm_status dmm_instance_trace_phases(dmm_instance* inst, int32_t nsteps, double* out) {
   dmm::clear_error();
   if (!inst || nsteps <= 0 || !out) return DMM_ERR_ARG;

@@ -154,9 +154,11 @@ class Pack {
   // out[2 kTraceK] = SM clock (MHz); out[2 kTraceK + 1], [+ 2] = launch prologue and epilogue
   // (staged kernel).
   dmm_status trace_phases(int32_t nsteps, double* out);
-  // Kernel used by launch_steps: 1 two-kernel, 2 cooperative, 3 cooperative single formula,
-  // 4 staged, 5 one block per formula (dmm_instance_launch_form).
+  // Form of launch_steps: 1 two-kernel, 2 cooperative, 3 cooperative single formula, 4 staged, 5
+  // one block per formula, 6 several staged tiles per block (dmm_instance_launch_form); the
+  // kernel: the same, or 7 cluster, 8 resident grid, 9 streaming (dmm_instance_step_kernel).
   int launch_form() const;
+  int step_kernel() const;
   // Test hook: one cooperative launch whose first grid barrier waits for one arrival more
   // than the grid has; returns what check_error reports (DMM_ERR_CUDA).
   dmm_status test_barrier_timeout();

@@ -2535,6 +2535,14 @@ int Pack::launch_form() const {
   return 2;
 }
 
+int Pack::step_kernel() const {
+  if (tun_.launch_mode != 1 && ctiles_h_.empty() && vtiles_h_.empty() && n_small_ == 0) {
+    if (!clusters_.empty()) return 7;
+    if (!gr_groups_.empty()) return 8;
+  }
+  return tun_.launch_mode != 1 && stream_active_ ? 9 : launch_form();
+}
+
 dmm_status Pack::trace_phases(int32_t nsteps, double* out) {
   DMM_CUDA(cudaSetDevice(dev_));
   TileForms tile_forms(*this, false);

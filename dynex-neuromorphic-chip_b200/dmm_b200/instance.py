@@ -197,11 +197,22 @@ class Instance:
 
     @property
     def launch_form(self) -> str:
-        """Kernel that step/solve launch with the current tuning (see LAUNCH_FORMS)."""
+        """Launch form with the current tuning (see LAUNCH_FORMS).  The cluster, resident grid and
+        streaming kernels are reported as the form they stand in for: `step_kernel` names them."""
         f = lib().dmm_instance_launch_form(self._h)
         if f < 0:
             check(f)
         return self.LAUNCH_FORMS[f]
+
+    STEP_KERNELS = {**LAUNCH_FORMS, 7: "cluster", 8: "resident-grid", 9: "streaming"}
+
+    @property
+    def step_kernel(self) -> str:
+        """Kernel that step/solve launch with the current tuning (see STEP_KERNELS)."""
+        k = lib().dmm_instance_step_kernel(self._h)
+        if k < 0:
+            check(k)
+        return self.STEP_KERNELS[k]
 
     def trace_phases(self, nsteps: int) -> dict:
         """Per-step microseconds (mean, max over blocks) between the cooperative kernel's

@@ -241,8 +241,8 @@ dmm_status dmm_instance_report(dmm_instance* inst, dmm_report* rep);
  *        of dynex.cc:667-670 and the solution file of dynex.cc:693-699),
  *  post: the reported assignment after the final step (+1/-1; `v` lines, dynex.cc:1506-1512). */
 dmm_status dmm_instance_assignment(dmm_instance* inst, int8_t* pre, int8_t* post);
-/* No counterpart in the reference.  The kernel that dmm_instance_step / _solve launch for
- * this instance with its current tuning:
+/* No counterpart in the reference.  The launch form of this instance with its current tuning
+ * (dmm_instance_step_kernel names the kernel itself):
  *   1  two kernels per step (clause tiles, then variable tiles), CUDA graphs
  *   2  one cooperative kernel for several steps, three grid barriers per step
  *   3  the same for a single formula (FP64, or FP32 without the staged tables): two grid
@@ -256,10 +256,17 @@ dmm_status dmm_instance_assignment(dmm_instance* inst, int8_t* pre, int8_t* post
  * its data and exchanges in shared memory, a larger one (up to about 450,000 clauses) by blocks
  * that keep their voltages resident and exchange without grid barriers, and an FP32 one of
  * 9,000,000 literals or more by blocks through whose shared memory its tables and voltage lists
- * stream.  They are reported as the form they stand in for: for FP32 with 3-literal clauses 4,
- * the streaming ones 6; else 3.
+ * stream.  They are reported here as the form they stand in for: for FP32 with 3-literal clauses
+ * 4, the streaming ones 6; else 3.
  * A negative dmm_status on error. */
 int32_t dmm_instance_launch_form(const dmm_instance* inst);
+/* No counterpart in the reference.  The kernel that dmm_instance_step / _solve launch: the codes of
+ * dmm_instance_launch_form, and for the three that these stand in for
+ *   7  one thread-block cluster per formula
+ *   8  blocks of the whole grid with resident voltages
+ *   9  tables and voltage lists streamed through the blocks' shared memory
+ * A negative dmm_status on error. */
+int32_t dmm_instance_step_kernel(const dmm_instance* inst);
 /* No counterpart in the reference.  Test hook for the failure path of the cooperative step
  * kernels: one launch whose first grid barrier waits for one arrival more than the grid has,
  * so every block's bounded wait runs out (a few seconds), and behind it, where the resident grid
