@@ -458,7 +458,13 @@ dmm_status dmm_batch_result(dmm_batch* b, int32_t index, dmm_report* rep, int8_t
   }
   if (!post) return DMM_OK;
   if (b->after.empty() || ++b->reads < 2) return b->pack->assignment(i, nullptr, post);
+  // One copy for all of them saves a wait of about 45 us per formula and costs a second pass over
+  // the signs, which a read by itself has not: at 4 10^5 variables 0.22 ms against 0.08.
+  constexpr int64_t kTogether = 1 << 16;  // signs per formula, on average
   if (b->post_off.empty()) {
+    int64_t signs = 0;
+    for (int32_t k : b->idx) signs += b->pack->desc(k).n;
+    if (signs > kTogether * (int64_t)b->idx.size()) return b->pack->assignment(i, nullptr, post);
     DMM_TRY(b->pack->assignments(b->idx, &b->post));
     b->post_off.resize(b->idx.size() + 1);
     for (size_t k = 0; k < b->idx.size(); k++)

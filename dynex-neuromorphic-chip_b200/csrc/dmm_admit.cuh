@@ -132,7 +132,9 @@ __global__ void __launch_bounds__(kAdmitThreads)
   }
 }
 
-// Reported assignments (signs of the current V) of `count` formulas: out[off[k] ..].
+// Reported assignments (signs of the current V) of `count` formulas: out[off[k] ..], formula k by
+// the blocks (k, y): one block each is enough for the small formulas of a large batch, but a large
+// one among them would be a chain of loads in one block.
 template <class T>
 __global__ void k_signs_all(const InstDesc* __restrict__ inst, const InstCtrl* __restrict__ ctrl,
                             const int32_t* __restrict__ idx, const int64_t* __restrict__ off,
@@ -140,7 +142,9 @@ __global__ void k_signs_all(const InstDesc* __restrict__ inst, const InstCtrl* _
   const int i = idx[blockIdx.x];
   const T* v = cand + (int64_t)(ctrl[i].set * kTrials + ctrl[i].kcur) * var_cap + inst[i].var0;
   int8_t* o = out + off[blockIdx.x];
-  for (int k = threadIdx.x; k < inst[i].n; k += blockDim.x) o[k] = v[k] > T(0) ? 1 : -1;
+  const int n = inst[i].n;
+  for (int k = blockIdx.y * blockDim.x + threadIdx.x; k < n; k += gridDim.y * blockDim.x)
+    o[k] = v[k] > T(0) ? 1 : -1;
 }
 
 }  // namespace dmm

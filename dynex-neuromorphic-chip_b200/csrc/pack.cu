@@ -2854,11 +2854,14 @@ dmm_status Pack::assignments(const std::vector<int32_t>& idx, std::vector<int8_t
   int8_t* dst = reinterpret_cast<int8_t*>(base + o_out);
   const auto* di = reinterpret_cast<const int32_t*>(base + o_idx);
   const auto* doff = reinterpret_cast<const int64_t*>(base);
+  int32_t most = 1;
+  for (int32_t i : idx) most = std::max(most, inst_h_[i].n);
+  const dim3 grid((unsigned)idx.size(), (unsigned)std::min((most + 4 * kThreads - 1) / (4 * kThreads), 64));
   if (prec_ == DMM_FP64)
-    k_signs_all<double><<<(unsigned)idx.size(), kThreads, 0, stream_>>>(
+    k_signs_all<double><<<grid, kThreads, 0, stream_>>>(
         inst_d_, ctrl_d_, di, doff, static_cast<const double*>(cand_), caps_.vars, dst);
   else
-    k_signs_all<float><<<(unsigned)idx.size(), kThreads, 0, stream_>>>(
+    k_signs_all<float><<<grid, kThreads, 0, stream_>>>(
         inst_d_, ctrl_d_, di, doff, static_cast<const float*>(cand_), caps_.vars, dst);
   DMM_CUDA(cudaGetLastError());
   DMM_CUDA(cudaMemcpyAsync(out->data(), dst, (size_t)total, cudaMemcpyDeviceToHost, stream_));
