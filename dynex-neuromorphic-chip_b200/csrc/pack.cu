@@ -2181,10 +2181,15 @@ dmm_status Pack::plan_clusters(const std::vector<int32_t>& cand, std::vector<int
   // that holds the formula.  Formulas of one size and clause kind share a launch.
   int q0 = kClusterSizes - 1;
   while (q0 > 0 && ((int64_t)list.size() << q0) > sms_) q0--;
+  // With more formulas than SMs (FP64: the FP32 ones run one block each) the clusters run in many
+  // waves, and few of 16 blocks are resident at once: formulas that need them are faster in the
+  // tile forms (200 formulas, clauses each, blocks, us per step against them: 8,600, 8, 101 / 130;
+  // 12,000, 8, 137 / 177; 12,900, 16, 218 / 194; 16,000, 16, 255 / 219).
+  const int sizes = (int)list.size() > sms_ ? kClusterSizes - 1 : kClusterSizes;
   std::vector<std::vector<int32_t>> member;
   for (int32_t i : list) {
     const InstDesc& I = inst_h_[i];
-    for (int q = q0; q < kClusterSizes; q++) {
+    for (int q = q0; q < sizes; q++) {
       const bool general = I.k3 == 0;
       size_t g = 0;
       while (g < clusters_.size() && (clusters_[g].R != 1 << q || clusters_[g].general != general)) g++;

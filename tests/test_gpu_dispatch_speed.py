@@ -1,0 +1,37 @@
+"""The form that runs a formula by default is not slower than the tile forms, which launch_mode 2
+selects, where they are the better ones: large batches of formulas that need the largest clusters."""
+import pytest
+
+import dmm_b200 as dmm
+
+pytestmark = pytest.mark.gpu
+
+STEPS = 64
+SLOWER = 1.06  # times of equal launches differ by 1 %; the cases below were 9 to 20 % slower
+
+
+def batch_ms(sizes, ratio, precision, mode):
+    """Device time of STEPS steps of a batch, the least of four runs."""
+    fs = {n: dmm.generate_planted(n, int(ratio * n), 0.08, 0.58, seed=1)[0] for n in set(sizes)}
+    b = dmm.Batch.for_formulas([fs[n] for n in sizes], precision=precision)
+    b.set_tuning(launch_mode=mode)
+    xs = [dmm.initial_state_uniform(fs[n], 5 + k) for k, n in enumerate(sizes)]
+    for n, x in zip(sizes, xs):
+        b.add(fs[n], x, max_steps=STEPS)
+    ms = []
+    for _ in range(5):
+        for k, x in enumerate(xs):
+            b.set_state_at(k, x, 0.0)
+        ms.append(b.run()["device_ms"])
+    b.close()
+    return min(ms[1:])
+
+
+@pytest.mark.parametrize("sizes,ratio,precision", [
+    ([2000] * 200, 8.0, "fp64"),   # more formulas than SMs, clusters of 16 blocks
+    ([3000] * 200, 4.3, "fp64"),
+])
+def test_batch_not_slower_than_the_tile_forms(sizes, ratio, precision):
+    default = batch_ms(sizes, ratio, precision, 0)
+    tiles = batch_ms(sizes, ratio, precision, 2)
+    assert default <= SLOWER * tiles, (default, tiles)
