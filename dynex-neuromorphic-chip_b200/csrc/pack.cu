@@ -1649,6 +1649,11 @@ dmm_status Pack::plan_grid(const std::vector<int32_t>& cand, std::vector<int32_t
       // 16.9 / 15.5; FP64 70,000 31.6 / 32.5, 100,000, with two tiles per block, 58 / 44)
       if (list.size() == 1 && ((!fp64 && I.k3 && L / B[k] > 9000) || (fp64 && g.kc + g.kv > 2)))
         fits = false;
+      // several in FP64: the tile forms once a block goes through more than four tiles of a kind
+      // (formulas x variables at 4.3 or 8 clauses each, tiles of a kind, us per step against them:
+      // 5 x 40,000 at 4.3, 3, 56 / 63; 2 x 60,000 at 8, 4, 68 / 74; 3 x 70,000 at 4.3, 5, 69 / 63;
+      // 4 x 60,000 at 4.3, 10, 91 / 84)
+      if (fp64 && g.kc > 4) fits = false;
       if (!fits) continue;
       g.TC = ((I.m + g.B * g.kc - 1) / (g.B * g.kc) + 3) & ~3;
       g.TV = ((I.n + g.B * g.kv - 1) / (g.B * g.kv) + 3) & ~3;
