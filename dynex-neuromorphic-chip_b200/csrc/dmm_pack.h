@@ -237,6 +237,11 @@ class Pack {
   void drop_grid_tables();
   double cluster_step_us() const;
   double grid_step_us(const std::vector<int32_t>& list) const;
+  double tile_step_us(const std::vector<int32_t>& list) const;
+  std::vector<int32_t> without(const std::vector<int32_t>& all,
+                               const std::vector<int32_t>& some) const;
+  bool grid_pays(const std::vector<int32_t>& all, const std::vector<int32_t>& list,
+                 const std::vector<GridGroup>& groups) const;
   dmm_status grid_buffer(int which, int64_t bytes);
   dmm_status prepare_xpose(int32_t idx, int TC, int TV, bool mt, bool* ok);
   // several-tiles-per-block staged form for a formula too large for one tile per block:

@@ -1306,6 +1306,68 @@ double Pack::grid_step_us(const std::vector<int32_t>& list) const {
                  : (fp64 ? 7.0 + 5.2e-3 * share : 4.9 + 3.2e-3 * share);
 }
 
+// The formulas of `all` that are not among `some`.
+std::vector<int32_t> Pack::without(const std::vector<int32_t>& all,
+                                   const std::vector<int32_t>& some) const {
+  std::vector<char> taken(live_.size(), 0);
+  for (int32_t i : some) taken[i] = 1;
+  std::vector<int32_t> rest;
+  for (int32_t i : all)
+    if (!taken[i]) rest.push_back(i);
+  return rest;
+}
+
+// Estimated microseconds per step of several formulas in the tile forms, fitted to some 560 batches
+// of 2 to 148 formulas of 50 to 400,000 variables at 4.3 and 8 clauses per variable (error 6 to 7 %),
+// other clause lengths at 6.6 (7 %): waves of clause and variable tiles, and what they hold.
+double Pack::tile_step_us(const std::vector<int32_t>& list) const {
+  const bool fp64 = prec_ == DMM_FP64;
+  const int block = persist_threads(prec_);
+  double ct = 0, vt = 0, m = 0;
+  bool general = false;
+  for (int32_t i : list) {
+    ct += (inst_h_[i].m + 4 * block - 1) / (4 * block);
+    vt += (inst_h_[i].n + block - 1) / block;
+    m += 1e-6 * inst_h_[i].m;
+    general |= inst_h_[i].k3 == 0;
+  }
+  ct /= sms_;
+  vt /= sms_;
+  if (list.empty()) return 0.0;
+  // (one formula: its tiles are balanced over the grid)
+  if (list.size() == 1)
+    return general ? (fp64 ? 13 + 94 * m : 11 + 66 * m) : (fp64 ? 9 + 50 * m : 8 + 39 * m);
+  const double c = 0.01 * (double)list.size(), cw = std::ceil(ct), vw = std::ceil(vt);
+  if (general)
+    return fp64 ? 2.2 + 12.7 * cw + 17.5 * vw + 53.8 * m - 23.2 * c
+                : 7.9 + 14.2 * cw + 15.1 * vw + 35.9 * m - 15.3 * c;
+  return fp64 ? -0.6 + 5.6 * cw + 13.0 * vw + 4.5 * ct - 12.2 * vt + 35.1 * m - 7.4 * c
+              : 7.0 + 5.7 * cw + 12.9 * vw + 14.1 * ct - 10.2 * vt + 1.9 * m - 11.1 * c;
+}
+
+// Whether several formulas `all` run faster when `groups` (the formulas `list`) take the resident
+// grid form and the others the tile forms after it, than all together in the tile forms: the grid
+// form's step is that of its most loaded block, and the launch for the others comes on top.  The
+// former by the largest share of the clauses and the tiles of a block, fitted to the same batches
+// (error 10 to 13 %).  Of 413 such batches 24 were 3 to 30 % slower with the grid form wherever
+// tables could be built, 3 are where this says so (us per step, grid form / tile forms: four of
+// n = 60,000, FP64 at 4.3 clauses per variable, 91 / 84; 60 of 100 to 10,000, FP32, mixed lengths,
+// 115 / 88; 16 of 500 to 20,000, FP32 at 8, 18 / 43).
+bool Pack::grid_pays(const std::vector<int32_t>& all, const std::vector<int32_t>& list,
+                     const std::vector<GridGroup>& groups) const {
+  const bool fp64 = prec_ == DMM_FP64;
+  double share = 0, tiles = 0;
+  bool general = false;
+  for (const GridGroup& g : groups) {
+    share = std::max(share, 1e-3 * g.TC * g.kc);
+    tiles = std::max(tiles, (double)(g.kc + g.kv));
+    general |= g.k3 == 0;
+  }
+  const double grid = general ? (fp64 ? 2.4 + 8.7 * share + 4.7 * tiles : -13.3 + 6.3 * share + 9.0 * tiles)
+                              : (fp64 ? 2.9 + 4.3 * share + 3.7 * tiles : -3.4 + 2.0 * share + 6.0 * tiles);
+  return grid + tile_step_us(without(all, list)) < tile_step_us(all);
+}
+
 dmm_status Pack::grid_buffer(int which, int64_t bytes) {
   bytes = std::max<int64_t>(bytes, 16);
   if (bytes <= gbuf_cap_[which]) return DMM_OK;
@@ -1649,11 +1711,6 @@ dmm_status Pack::plan_grid(const std::vector<int32_t>& cand, std::vector<int32_t
       // 16.9 / 15.5; FP64 70,000 31.6 / 32.5, 100,000, with two tiles per block, 58 / 44)
       if (list.size() == 1 && ((!fp64 && I.k3 && L / B[k] > 9000) || (fp64 && g.kc + g.kv > 2)))
         fits = false;
-      // several in FP64: the tile forms once a block goes through more than four tiles of a kind
-      // (formulas x variables at 4.3 or 8 clauses each, tiles of a kind, us per step against them:
-      // 5 x 40,000 at 4.3, 3, 56 / 63; 2 x 60,000 at 8, 4, 68 / 74; 3 x 70,000 at 4.3, 5, 69 / 63;
-      // 4 x 60,000 at 4.3, 10, 91 / 84)
-      if (fp64 && g.kc > 4) fits = false;
       if (!fits) continue;
       g.TC = ((I.m + g.B * g.kc - 1) / (g.B * g.kc) + 3) & ~3;
       g.TV = ((I.n + g.B * g.kv - 1) / (g.B * g.kv) + 3) & ~3;
@@ -1675,6 +1732,7 @@ dmm_status Pack::plan_grid(const std::vector<int32_t>& cand, std::vector<int32_t
       continue;
     }
     if (z.ux > INT32_MAX / 2 || z.row > INT32_MAX / 2) return DMM_OK;
+    if (cand.size() > 1 && !grid_pays(cand, list, groups)) return DMM_OK;
     // (the tables of the same formulas in the same tiles are still valid: only this function
     // writes them, and a live formula's device arrays do not change)
     std::vector<uint64_t> key;
@@ -1994,12 +2052,6 @@ dmm_status Pack::commit_tiles() {
     gr_groups_.clear();
     const bool open_shape = tun_.launch_mode == 0 && tun_.u_layout == 0 && tun_.clause_tile == 0 &&
                             tun_.var_tile == 0;
-    auto without = [](const std::vector<int32_t>& all, const std::vector<int32_t>& some) {
-      std::vector<int32_t> rest;
-      for (int32_t i : all)
-        if (std::find(some.begin(), some.end(), i) == some.end()) rest.push_back(i);
-      return rest;
-    };
     if (open_shape && !no_cluster_) DMM_TRY(plan_clusters(others, &cluster_list));
     if (open_shape && !no_grid_ && !fixed_grid_) {
       const std::vector<int32_t> rest = without(others, cluster_list);

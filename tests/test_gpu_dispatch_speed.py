@@ -1,6 +1,7 @@
 """The form that runs a formula by default is not slower than the tile forms, which launch_mode 2
 selects, where they are the better ones: large batches of formulas that need the largest clusters,
-a few formulas of many tiles per block."""
+a few formulas of many tiles per block, formulas of which some do not fit the resident grid form."""
+import numpy as np
 import pytest
 
 import dmm_b200 as dmm
@@ -8,6 +9,8 @@ import dmm_b200 as dmm
 pytestmark = pytest.mark.gpu
 
 STEPS = 64
+# 60 sizes from 100 to 20,000, spread over their logarithm
+SPREAD = [int(np.exp(u)) for u in np.random.default_rng(0).uniform(np.log(100), np.log(20000), 60)]
 SLOWER = 1.06  # times of equal launches differ by 1 %; the cases below were 8 to 20 % slower
 
 
@@ -33,6 +36,7 @@ def batch_ms(sizes, ratio, precision, mode):
     ([3000] * 200, 4.3, "fp64"),
     ([70000] * 3, 4.3, "fp64"),    # many tiles per block of the resident grid form
     ([60000] * 4, 4.3, "fp64"),
+    (SPREAD, 4.3, "fp32"),         # two formulas left over for the tile forms
 ])
 def test_batch_not_slower_than_the_tile_forms(sizes, ratio, precision):
     default = batch_ms(sizes, ratio, precision, 0)
