@@ -357,6 +357,7 @@ class Pack {
   // cluster form: launches over formulas order_d_[first, first + count), one cluster each
   struct ClusterLaunch {
     int32_t first = 0, count = 0, R = 1, smem = 0;
+    int32_t resident = 1;  // clusters on the device at once
     bool general = false;
     ClusterCaps caps{};
   };

@@ -1270,7 +1270,9 @@ static const void* staged_fn(int G, bool mt) {
 
 // Estimated microseconds per step, fitted to single formulas of 500 to 30,000 variables at 4.3
 // and 8 clauses per variable: the cluster form by a block's clauses (FP32 3.1 us at 250 and
-// 4.8 at 1,000; FP64 4.7 and 9.9), in waves when the clusters do not all fit at once; the
+// 4.8 at 1,000; FP64 4.7 and 9.9), in waves when the clusters do not all fit at once (blocks of a
+// cluster share a GPC: few clusters of 16 are resident together; 16 formulas of n = 8,000 at 4.3,
+// FP32: 28.2 us in clusters of 16, 26.8 in the tile forms, 15.8 in the resident grid form); the
 // resident grid form by a block's share of the clauses (FP32 5.1 us at 54, 9.8 at 1,600; FP64
 // 7.5 and 15.9).  The two meet at about 18,000 clauses (FP32) and 13,000 (FP64) for one formula.
 // Clauses of other lengths have their own fits, at 3.5 and 6.6 clauses per variable (cluster
@@ -1280,15 +1282,15 @@ static const void* staged_fn(int G, bool mt) {
 // FP32 7.2 / 6.3; at 10,500: FP64 10.6 / 8.8).
 double Pack::cluster_step_us() const {
   const bool fp64 = prec_ == DMM_FP64;
-  int64_t blocks = 0;
-  double most = 0;
+  double blocks = 0, full = 0, most = 0;
   for (const ClusterLaunch& L : clusters_) {
-    blocks += (int64_t)L.R * L.count;
+    blocks += (double)L.R * L.count;
+    full += (double)L.count / L.resident;
     const double us = L.general ? (fp64 ? 4.2 + 8.2e-3 * L.caps.tc : 2.6 + 5.6e-3 * L.caps.tc)
                                 : (fp64 ? 3.6 + 5.0e-3 * L.caps.tc : 2.6 + 2.2e-3 * L.caps.tc);
     most = std::max(most, us);
   }
-  return (double)((blocks + sms_ - 1) / sms_) * most;
+  return std::ceil(std::max(blocks / sms_, full)) * most;
 }
 
 double Pack::grid_step_us(const std::vector<int32_t>& list) const {
@@ -2273,6 +2275,7 @@ dmm_status Pack::plan_clusters(const std::vector<int32_t>& cand, std::vector<int
           cudaGetLastError();
           continue;
         }
+        L.resident = act;
         clusters_.push_back(L);
         member.emplace_back();
       }
