@@ -204,6 +204,11 @@ class Pack {
   dmm_status resolve_long_lists();
   dmm_status ensure_stage(int64_t doubles);
   dmm_status capture(int32_t steps);
+  // tile tables of the formulas `live` (alone: no other form runs any formula)
+  dmm_status plan_tiles(const std::vector<int32_t>& live, bool alone);
+  // tile tables for launches of up to short_steps() steps, made when the first is launched
+  int32_t short_steps() const;
+  dmm_status plan_short();
   dmm_status launch_persist(int32_t nsteps);
   dmm_status launch_inst(int32_t nsteps);
   dmm_status launch_cluster(int32_t nsteps);
@@ -375,6 +380,7 @@ class Pack {
   int32_t gr_blocks_ = 0;
   bool gr_general_ = false;
   int gr_resident_ = 0;
+  enum class ShortPlan { none, ready, refused } short_ = ShortPlan::none;
   bool stream_active_ = false;
   bool stream_general_ = false;
   StreamLayout stream_layout_{};

@@ -2023,9 +2023,8 @@ dmm_status Pack::prepare_xpose_mt(int32_t idx, bool* ok) {
 
 dmm_status Pack::commit_tiles() {
   DMM_TRY(resolve_long_lists());
-  xp_active_ = false;
-  one_active_ = false;
   stream_active_ = false;
+  short_ = ShortPlan::none;
   ctiles_h_.clear();
   vtiles_h_.clear();
   std::vector<int32_t> live_list;
@@ -2081,6 +2080,12 @@ dmm_status Pack::commit_tiles() {
     DMM_CUDA(cudaMemcpyAsync(order_d_, small_list.data(), small_list.size() * sizeof(int32_t),
                              cudaMemcpyHostToDevice, stream_));
   for (auto& c : clusters_) c.first += n_small_;
+  return plan_tiles(live_list, small_list.empty());
+}
+
+dmm_status Pack::plan_tiles(const std::vector<int32_t>& live_list, bool alone) {
+  xp_active_ = false;
+  one_active_ = false;
   // grids
   int bc, bv;
   if (prec_ == DMM_FP64) {
@@ -2131,7 +2136,7 @@ dmm_status Pack::commit_tiles() {
   }
   // one formula on the cooperative path: two grid barriers per step; FP32 with the
   // default layout and tiles: the staged form when it fits
-  one_active_ = coop && live_list.size() == 1 && small_list.empty();
+  one_active_ = coop && live_list.size() == 1 && alone;
   if (one_active_ && tun_.u_layout == 0 && tun_.clause_tile == 0 && tun_.var_tile == 0) {
     const int32_t one = live_list[0];
     if (prec_ == DMM_FP32) DMM_TRY(prepare_xpose(one, TC, TV, false, &xp_active_));
@@ -2169,6 +2174,51 @@ dmm_status Pack::commit_tiles() {
   grid_v_ = new_v;
   if (!fixed_grid_) graph_stale_ = true;
   DMM_CUDA(cudaStreamSynchronize(stream_));
+  return DMM_OK;
+}
+
+// Launches of up to this many steps leave a formula of the cluster or resident grid form to the
+// tile forms: those forms bring the formula and their tables into shared memory when a launch
+// starts, which only the following steps win back.  us per call of step(k), resident or cluster
+// / tile forms: FP32 at 8 clauses of three literals per variable, n = 2,000 (cluster) k = 1
+// 108 / 102, 4 118 / 126; 20,000 k = 1 116 / 100, 4 143 / 128, 16 237 / 238; 50,000 k = 4
+// 166 / 145, 16 312 / 304, 32 503 / 515; FP64 at 4.3, 50,000 k = 1 130 / 106, 4 171 / 161, 16
+// 332 / 381; clauses of 1 to 8 literals FP32 n = 30,000 k = 1 124 / 109, 4 156 / 174.
+int32_t Pack::short_steps() const {
+  if (fixed_grid_ || tun_.launch_mode == 1 || !ctiles_h_.empty() || !vtiles_h_.empty() ||
+      n_small_ > 0)
+    return 0;
+  if (gr_groups_.empty() && clusters_.size() == 1 && clusters_[0].count == 1) {
+    const int32_t m = clusters_[0].R * clusters_[0].caps.tc;
+    return clusters_[0].general || m < 8600 ? 0 : m / 5000;
+  }
+  if (gr_groups_.size() != 1 || !clusters_.empty()) return 0;
+  return gr_general_ ? 2 : 2 + gr_groups_[0].m / (prec_ == DMM_FP64 ? 100000 : 20000);
+}
+
+dmm_status Pack::plan_short() {
+  if (short_ != ShortPlan::none) return DMM_OK;
+  short_ = ShortPlan::refused;
+  int32_t one = -1, count = 0;
+  for (int32_t i = 0; i < (int32_t)live_.size(); i++)
+    if (live_[i]) {
+      one = i;
+      count++;
+    }
+  if (count != 1) return DMM_OK;
+  no_grid_ = true;  // the streaming form's tables share the resident grid form's memory
+  const dmm_status st = plan_tiles({one}, true);
+  no_grid_ = false;
+  // the committed forms stay as they are: these tiles are launched by short launches alone
+  ctiles_h_.clear();
+  vtiles_h_.clear();
+  if (st == DMM_ERR_NOMEM) {
+    clear_error();
+    xp_active_ = one_active_ = false;
+    return DMM_OK;
+  }
+  DMM_TRY(st);
+  short_ = ShortPlan::ready;
   return DMM_OK;
 }
 
@@ -2485,6 +2535,10 @@ dmm_status Pack::launch_steps(int32_t nsteps) {
       gr_groups_.empty())
     return DMM_OK;
   const int32_t S = tun_.steps_per_graph;
+  if (nsteps <= short_steps()) {
+    DMM_TRY(plan_short());
+    if (short_ == ShortPlan::ready) return nsteps > 0 ? launch_persist(nsteps) : DMM_OK;
+  }
   if (tun_.launch_mode != 1) {
     // cluster launches alone take all the steps at once: their steps are a few microseconds,
     // and a launch's prologue costs about as much as two of them

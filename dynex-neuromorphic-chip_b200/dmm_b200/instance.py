@@ -208,7 +208,8 @@ class Instance:
 
     @property
     def step_kernel(self) -> str:
-        """Kernel that step/solve launch with the current tuning (see STEP_KERNELS)."""
+        """Kernel that step/solve launch with the current tuning (see STEP_KERNELS); steps of a few
+        at a time run the `launch_form` instead of "cluster" and "resident-grid"."""
         k = lib().dmm_instance_step_kernel(self._h)
         if k < 0:
             check(k)

@@ -264,6 +264,8 @@ int32_t dmm_instance_launch_form(const dmm_instance* inst);
  * dmm_instance_launch_form, and for the three that these stand in for
  *   7  one thread-block cluster per formula
  *   8  blocks of the whole grid with resident voltages
+ *      (calls of dmm_instance_step for few steps - one to about twenty, more for larger formulas -
+ *      leave a formula of 7 or 8 to the form that dmm_instance_launch_form reports)
  *   9  tables and voltage lists streamed through the blocks' shared memory
  * A negative dmm_status on error. */
 int32_t dmm_instance_step_kernel(const dmm_instance* inst);
