@@ -236,15 +236,14 @@ __device__ __forceinline__ float row_sum(const float* u, const uint2* row, const
   return r;
 }
 
-// Left-to-right sum of the d <= N smallest contributions of one thread's row (N <= 32 places,
-// eight per 16-byte word, words of neighbouring rows side by side; places past the list lead
-// to +inf) after sorting them.  Kernels that keep a formula in shared memory call it with
-// N = 32 alone, also for shorter lists: a block runs the code once or twice per step, so that
-// warps in two or three networks' straight-line code fetch it instead of sharing it (FP64 step
-// at n = 1,000: 5.94 us with networks of 16, 24 and 32 chosen by the warp's longest list, 5.81
+// Left-to-right sum of the d <= 32 smallest contributions of one thread's row (32 places, eight per
+// 16-byte word, words of neighbouring rows side by side; places past the list lead to +inf) after
+// sorting them.  One network also for shorter lists: a block runs the code once or twice per step,
+// so that warps in two or three networks' straight-line code fetch it instead of sharing it (FP64
+// step at n = 1,000: 5.94 us with networks of 16, 24 and 32 chosen by the warp's longest list, 5.81
 // with one; n = 10,000: 10.7 and 10.4).
-template <int N>
 __device__ __forceinline__ double row_net_sum(const double* u, const uint4* row, int d) {
+  constexpr int N = 32;
   double a[N];
 #pragma unroll
   for (int c = 0; c < N / 8; c++) {
@@ -560,8 +559,8 @@ __global__ void __launch_bounds__(sizeof(T) == 8 ? kClusterThreads64 : kClusterT
         if (valid) kmax = max(kmax, gb ? __ffs(gb) - 1 : kTrials);
       }
     } else {
-      // FP64 reference sums: one thread per variable (lists of up to 32), the warp's network
-      // chosen by its longest list; longer lists are queued and summed by whole warps
+      // FP64 reference sums: one thread per variable (lists of up to 32); longer lists are queued
+      // and summed by whole warps
       const double* ud = reinterpret_cast<const double*>(bk);
       auto finish = [&](int i, T dv) {
         const T V = sV[v0 + i];
@@ -596,7 +595,7 @@ __global__ void __launch_bounds__(sizeof(T) == 8 ? kClusterThreads64 : kClusterT
         const bool small = i < nv && d <= 32;
         const int ds = small ? d : 0;
         const uint4* row = reinterpret_cast<const uint4*>(row_s) + 4 * vb + lane;
-        const double dv = row_net_sum<32>(ud, row, ds);
+        const double dv = row_net_sum(ud, row, ds);
         if (small) finish(i, T(dv));
       }
       // lists past the queue's end

@@ -743,7 +743,7 @@ __global__ void __launch_bounds__(sizeof(T) == 8 ? kGridThreads64 : kGridThreads
           const int i = min(vb + lane, i1 - 1), r = i - i0;
           const int2 list = s_list[i];
           const uint4* row = reinterpret_cast<const uint4*>(rt) + (r >> 5) * 128 + (r & 31);
-          const double dv = row_net_sum<32>(ud, row, list.y);
+          const double dv = row_net_sum(ud, row, list.y);
           if (vb + lane < i1) finish(i, T(dv));
         }
         queue();

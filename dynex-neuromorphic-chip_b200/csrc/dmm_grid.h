@@ -81,7 +81,7 @@ struct GridCaps {
 constexpr int kGridSyncBytes = 256;  // per group
 // Byte offsets of a block's dynamic shared memory.
 struct GridLayout {
-  int sv, raw, cur, dv, vend, unit, pinfo, rank;
+  int sv, raw, cur, dv, vend, unit, rank;
   int xs, xl, cp, lit, spos, off, ord, wdst, row, csr, snd, total;
 };
 
@@ -102,17 +102,15 @@ cudaError_t grid_build(const GridGroup* groups, const int32_t* list_group, int n
                        const int32_t* upos, const int32_t* vend, const int32_t* coff,
                        const GridTables& t, bool fp64, cudaStream_t s);
 
-// ---- streaming form (dmm_stream.cuh)
-constexpr int kStreamThreads = 1024;   // block size
-constexpr int kStreamThreads64 = 512;  // ... in FP64
+// ---- streaming form (dmm_stream.cuh), FP32
+constexpr int kStreamThreads = 1024;  // block size
 constexpr int kStreamSmemMax = 222 * 1024;
 struct StreamLayout {
   int v0, v1, stage;  // A: two voltage lists (one in use, one arriving), staging area
   int b0, b1;         // B: two buckets, each behind one padding word
-  int rank;           // FP64: ranking areas
   int total;          // C: the block's voltages, from 0
 };
-StreamLayout stream_shape(int dl, int st, int bk, int tv, bool fp64);
-const void* stream_kernel(bool fp64, bool general);
+StreamLayout stream_shape(int dl, int st, int bk, int tv);
+const void* stream_kernel(bool general);
 
 }  // namespace dmm

@@ -1,4 +1,4 @@
-// Streaming form of the integration step for one large formula, whose blocks cannot keep the
+// Streaming form of the FP32 integration step for one large formula, whose blocks cannot keep the
 // voltages of all their clauses: clause tiles and variable tiles pass through shared memory one
 // after another, many steps per cooperative launch, three grid barriers per step.
 //
@@ -42,14 +42,15 @@ __device__ __forceinline__ void cp_async_wait() {
 
 // Steps of the launch: counters in the launch area of the pack (StepAcc slots alternate by step,
 // as in k_staged).
-template <class T, bool GENERAL>
-__global__ void __launch_bounds__(sizeof(T) == 8 ? kStreamThreads64 : kStreamThreads, 1)
-    k_stream(PackView<T> P, GridTables tb, const GridGroup* __restrict__ groups, StreamLayout LY,
-             T* __restrict__ dv_all, int nsteps, unsigned int* bar, double* __restrict__ epart,
-             int* err) {
-  constexpr int NT = sizeof(T) == 8 ? kStreamThreads64 : kStreamThreads;
+template <bool GENERAL>
+__global__ void __launch_bounds__(kStreamThreads, 1)
+    k_stream(PackView<float> P, GridTables tb, const GridGroup* __restrict__ groups,
+             StreamLayout LY, float* __restrict__ dv_all, int nsteps, unsigned int* bar,
+             double* __restrict__ epart, int* err) {
+  using T = float;
+  constexpr int NT = kStreamThreads;
   constexpr int W = NT / 32;
-  constexpr int kw = 16 / (int)sizeof(T);  // values per 16-byte word
+  constexpr int kw = 4;  // values per 16-byte word
   extern __shared__ __align__(16) unsigned char st_smem[];
   __shared__ InstDesc I;
   __shared__ GridGroup g;
@@ -57,8 +58,7 @@ __global__ void __launch_bounds__(sizeof(T) == 8 ? kStreamThreads64 : kStreamThr
   __shared__ ClauseConsts<T> s_kc;
   __shared__ int cnt[3][W];
   __shared__ double red[W];
-  __shared__ int s_ok, s_nlong, s_next, s_last;
-  __shared__ int32_t s_long[kLongQueue];
+  __shared__ int s_ok, s_last;
   {
     unsigned have;
     asm volatile("mov.u32 %0, %%dynamic_smem_size;" : "=r"(have));
@@ -116,12 +116,11 @@ __global__ void __launch_bounds__(sizeof(T) == 8 ? kStreamThreads64 : kStreamThr
     int2 si = tb.sinfo[g.o_blk + b];
     if (!lists) si.y = 0;
     const uint32_t* const sdst = tb.sdst + g.o_push + si.x;
-    using Ids = typename std::conditional<sizeof(T) == 8, unsigned int, uint2>::type;
-    const Ids* const ids = reinterpret_cast<const Ids*>(tb.ids + (g.o_push + si.x) * kw);
+    const uint2* const ids = reinterpret_cast<const uint2*>(tb.ids + (g.o_push + si.x) * kw);
     int4* const in = reinterpret_cast<int4*>(inbox);
     for (int q0 = tid; q0 < si.y; q0 += 4 * NT) {
       uint32_t at[4];
-      Ids e[4];
+      uint2 e[4];
 #pragma unroll
       for (int r = 0; r < 4; r++)
         if (q0 + r * NT < si.y) {
@@ -246,7 +245,7 @@ __global__ void __launch_bounds__(sizeof(T) == 8 ? kStreamThreads64 : kStreamThr
           auto pos = [&](int k) {
             return (int)((k & 1) ? (qw[k >> 1] >> 16) : (qw[k >> 1] & 0xffffu));
           };
-          using T2 = typename std::conditional<sizeof(T) == 8, double2, float2>::type;
+          using T2 = float2;
           const T2 xs2 = __ldcs(reinterpret_cast<const T2*>(Xs + c));
           const T2 xl2 = __ldcs(reinterpret_cast<const T2*>(Xl + c));
           T2 cp2, al2;
@@ -316,7 +315,7 @@ __global__ void __launch_bounds__(sizeof(T) == 8 ? kStreamThreads64 : kStreamThr
       const int bb = tb.boff[g.o_vt + vt], be = tb.boff[g.o_vt + vt + 1];
       T* const dst = reinterpret_cast<T*>(st_smem + ((j & 1) ? LY.b1 : LY.b0));
       for (int q = tid; q < (be - bb) / kw; q += NT) cp_async16(dst + kw * (q + 1), ux + bb + kw * q);
-      if (tid == 0) dst[0] = sizeof(T) == 4 ? T(0) : inf_val<T>();
+      if (tid == 0) dst[0] = T(0);
       cp_async_commit();
     };
     int kmax = 0;
@@ -330,101 +329,43 @@ __global__ void __launch_bounds__(sizeof(T) == 8 ? kStreamThreads64 : kStreamThr
       } else {
         cp_async_wait<0>();
       }
-      if (tid == 0) s_nlong = s_next = 0;
       __syncthreads();
       if (j == 0) trace_stamp(P, s, 5);
       const T* const raw = reinterpret_cast<const T*>(st_smem + ((j & 1) ? LY.b1 : LY.b0));
       const uint16_t* const rt = tb.rows + g.o_row + (int64_t)vt * g.TVr * 32;
       const uint16_t* const idx = tb.idx + g.o_slot;
-      if constexpr (sizeof(T) == 4) {
-        constexpr int VPP = NT / 4;
-        const int gl = tid & 3;
-        uint4 q = make_uint4(0, 0, 0, 0);
-        if (i0 + tid / 4 < i1) q = __ldg(reinterpret_cast<const uint4*>(rt) + tid);
-        for (int vb = i0; vb < i1; vb += VPP) {
-          const int v = vb + tid / 4;
-          const bool valid = v < i1;
-          const uint4 qc = q;
-          if (v + VPP < i1) q = __ldg(reinterpret_cast<const uint4*>(rt) + 4 * (v + VPP - i0) + gl);
-          int d = 0, e0 = 0;
-          T V = T(0);
-          if (valid) {
-            const int e1 = __ldg(vend + v);
-            e0 = v > 0 ? __ldg(vend + v - 1) : 0;
-            d = e1 - e0;
-            V = cur[v];
-          }
-          const T dv = row_sum4<true>(reinterpret_cast<const float*>(raw), qc, idx + e0, d, gl);
-          bool acc_k = false;
-          if (valid) {  // lane k forms candidate k
-            if (gl == 0) dv_g[v] = dv;
-            const int8_t un = GENERAL ? P.unit[I.var0 + v] : 0;
-            const T h = gl == 0 ? T(0.125) : gl == 1 ? T(0.0625) : gl == 2 ? T(0.03125)
-                                                                           : T(0.015625);
-            T c = add(V, mul(h, dv));
-            if (un != 0) c = T(un);
-            c = clampv(c, T(-1), T(1));
-            acc_k = !(fabs((double)c - (double)V) >= 1.0);
-          }
-          const unsigned bal = __ballot_sync(0xffffffffu, acc_k);
-          const unsigned gb = (bal >> (lane & ~3)) & 15u;
-          if (valid) kmax = max(kmax, gb ? __ffs(gb) - 1 : kTrials);
+      constexpr int VPP = NT / 4;
+      const int gl = tid & 3;
+      uint4 q = make_uint4(0, 0, 0, 0);
+      if (i0 + tid / 4 < i1) q = __ldg(reinterpret_cast<const uint4*>(rt) + tid);
+      for (int vb = i0; vb < i1; vb += VPP) {
+        const int v = vb + tid / 4;
+        const bool valid = v < i1;
+        const uint4 qc = q;
+        if (v + VPP < i1) q = __ldg(reinterpret_cast<const uint4*>(rt) + 4 * (v + VPP - i0) + gl);
+        int d = 0, e0 = 0;
+        T V = T(0);
+        if (valid) {
+          const int e1 = __ldg(vend + v);
+          e0 = v > 0 ? __ldg(vend + v - 1) : 0;
+          d = e1 - e0;
+          V = cur[v];
         }
-      } else {
-        const double* ud = reinterpret_cast<const double*>(raw);
-        double* const rank_s = reinterpret_cast<double*>(st_smem + LY.rank) + 2 * kRankMax * w;
-        auto finish = [&](int v, T dv) {
-          const T V = cur[v];
+        const T dv = row_sum4<true>(raw, qc, idx + e0, d, gl);
+        bool acc_k = false;
+        if (valid) {  // lane k forms candidate k
+          if (gl == 0) dv_g[v] = dv;
           const int8_t un = GENERAL ? P.unit[I.var0 + v] : 0;
-          int kv = kTrials;
-#pragma unroll
-          for (int k = kTrials - 1; k >= 0; k--) {
-            const T h = T(0.125 / (double)(1 << k));
-            T c = add(V, mul(h, dv));
-            if (un != 0) c = T(un);
-            c = clampv(c, T(-1), T(1));
-            if (!(fabs((double)c - (double)V) >= 1.0)) kv = k;
-          }
-          kmax = max(kmax, kv);
-          dv_g[v] = dv;
-        };
-        auto warp_sum = [&](int v) {
-          const int e0 = v > 0 ? __ldg(vend + v - 1) : 0, d = __ldg(vend + v) - e0;
-          const double dv = d <= kRankMax ? rank_sum<true>(ud, idx + e0, d, rank_s, lane)
-                                          : sorted_sum<false, uint16_t, true>(ud, idx + e0, d, lane);
-          if (lane == 0) finish(v, T(dv));
-        };
-        for (int vb = i0 + 32 * w; vb < i1; vb += NT) {
-          const int v = vb + lane;
-          int d = 0;
-          if (v < i1) d = __ldg(vend + v) - (v > 0 ? __ldg(vend + v - 1) : 0);
-          const bool small = v < i1 && d <= 32;
-          const int ds = small ? d : 0;
-          const int dm = redux_max(ds);
-          const uint4* row = reinterpret_cast<const uint4*>(rt) + 4 * (vb - i0) + lane;
-          const double dv = dm <= 16   ? row_net_sum<16>(ud, row, ds)
-                            : dm <= 24 ? row_net_sum<24>(ud, row, ds)
-                                       : row_net_sum<32>(ud, row, ds);
-          if (small) finish(v, T(dv));
-          int qs = kLongQueue;
-          if (v < i1 && !small) qs = atomicAdd(&s_nlong, 1);
-          if (v < i1 && !small && qs < kLongQueue) s_long[qs] = v;
-          unsigned over = __ballot_sync(0xffffffffu, v < i1 && !small && qs >= kLongQueue);
-          while (over) {  // past the queue's end (warp-uniform)
-            const int vl = vb + __ffs(over) - 1;
-            over &= over - 1;
-            warp_sum(vl);
-          }
+          const T h = gl == 0 ? T(0.125) : gl == 1 ? T(0.0625) : gl == 2 ? T(0.03125)
+                                                                         : T(0.015625);
+          T c = add(V, mul(h, dv));
+          if (un != 0) c = T(un);
+          c = clampv(c, T(-1), T(1));
+          acc_k = !(fabs((double)c - (double)V) >= 1.0);
         }
-        __syncthreads();
-        const int nq = min(s_nlong, kLongQueue);
-        for (;;) {
-          int q = 0;
-          if (lane == 0) q = atomicAdd(&s_next, 1);
-          q = __shfl_sync(0xffffffffu, q, 0);
-          if (q >= nq) break;
-          warp_sum(s_long[q]);
-        }
+        const unsigned bal = __ballot_sync(0xffffffffu, acc_k);
+        const unsigned gb = (bal >> (lane & ~3)) & 15u;
+        if (valid) kmax = max(kmax, gb ? __ffs(gb) - 1 : kTrials);
       }
       __syncthreads();  // before the next bucket but one arrives in this place
     }

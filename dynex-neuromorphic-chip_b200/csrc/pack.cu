@@ -1525,10 +1525,10 @@ dmm_status Pack::grid_tables(const std::vector<GridGroup>& groups, const std::ve
 dmm_status Pack::plan_stream(int32_t idx, bool* ok) {
   *ok = false;
   const InstDesc& I = inst_h_[idx];
-  const bool fp64 = prec_ == DMM_FP64;
   // chunks of whole 32-byte sectors: a sector written by two blocks in halves is filled from
   // memory when the buckets exceed the L2
-  const int T = (int)tsize_, kw = 16 / T, B = sms_, pad = 32 / T;
+  constexpr int kw = 4, pad = 8;
+  const int B = sms_;
   if (I.m <= 0 || I.nslots <= 0) return DMM_OK;
   int kc_min = 1, kv_min = 1;
   for (int round = 0; round < 4; round++) {
@@ -1544,7 +1544,7 @@ dmm_status Pack::plan_stream(int32_t idx, bool* ok) {
         const double bk = L / ((double)B * v) * 1.06 + 0.5 * pad * B * c + 64;
         const double tv = n / B + 8 * v;
         if (dl > kGridMaxDistinct || st > 65000 || bk > 65000 || tv > 65000) continue;
-        if (stream_shape((int)dl, (int)st, (int)bk, (int)tv, fp64).total > kStreamSmemMax) continue;
+        if (stream_shape((int)dl, (int)st, (int)bk, (int)tv).total > kStreamSmemMax) continue;
         kc = c;
         kv = v;
       }
@@ -1588,7 +1588,7 @@ dmm_status Pack::plan_stream(int32_t idx, bool* ok) {
       return DMM_OK;
     }
     DMM_TRY(st);
-    const StreamLayout lay = stream_shape(out[1], out[2], out[3], g.TV * g.kv, fp64);
+    const StreamLayout lay = stream_shape(out[1], out[2], out[3], g.TV * g.kv);
     if (out[0] == 3 || (out[0] == 0 && lay.total > kStreamSmemMax && out[3] > out[2])) {
       kv_min = kv + 1;
       continue;
@@ -1598,8 +1598,7 @@ dmm_status Pack::plan_stream(int32_t idx, bool* ok) {
       continue;
     }
     stream_general_ = I.k3 == 0;
-    if (occupancy_blocks(stream_kernel(fp64, stream_general_), fp64 ? kStreamThreads64 : kStreamThreads,
-                         lay.total, kStreamSmemMax) < 1)
+    if (occupancy_blocks(stream_kernel(stream_general_), kStreamThreads, lay.total, kStreamSmemMax) < 1)
       return DMM_OK;
     stream_layout_ = lay;
     gr_tables_ = t;
@@ -1611,30 +1610,20 @@ dmm_status Pack::plan_stream(int32_t idx, bool* ok) {
 }
 
 dmm_status Pack::launch_stream(int32_t nsteps) {
-  const bool fp64 = prec_ == DMM_FP64;
-  PackView<float> vf;
-  PackView<double> vd;
-  void* view;
-  if (fp64) {
-    fill_view<double>(&vd);
-    view = &vd;
-  } else {
-    fill_view<float>(&vf);
-    view = &vf;
-  }
+  PackView<float> view;
+  fill_view<float>(&view);
   unsigned int* bar = reinterpret_cast<unsigned int*>(misc_d_ + kMiscLaunch);
   if (!launch_area_clean_)
     DMM_CUDA(cudaMemsetAsync(bar, 0, kLaunchAreaInts * sizeof(int32_t), stream_));
   launch_area_clean_ = true;
-  const void* fn = stream_kernel(fp64, stream_general_);
+  const void* fn = stream_kernel(stream_general_);
   DMM_CUDA(allow_smem(fn, kStreamSmemMax));
   const void* groups = gbuf_[kGrGroups];
   void* dv = gbuf_[kGrDv];
   void* epart = gbuf_[kGrEpart];
   int* err = error_d_;
-  void* args[] = {view, &gr_tables_, &groups, &stream_layout_, &dv, &nsteps, &bar, &epart, &err};
-  DMM_CUDA(cudaLaunchCooperativeKernel(fn, dim3((unsigned)sms_),
-                                       dim3(fp64 ? kStreamThreads64 : kStreamThreads), args,
+  void* args[] = {&view, &gr_tables_, &groups, &stream_layout_, &dv, &nsteps, &bar, &epart, &err};
+  DMM_CUDA(cudaLaunchCooperativeKernel(fn, dim3((unsigned)sms_), dim3(kStreamThreads), args,
                                        (size_t)stream_layout_.total, stream_));
   return DMM_OK;
 }
@@ -2632,8 +2621,10 @@ dmm_status Pack::preload_kernels() {
   fns.push_back(cluster_kernel(prec_ == DMM_FP64, false));
   fns.push_back(cluster_kernel(prec_ == DMM_FP64, true));
   grid_functions(prec_ == DMM_FP64, &fns);
-  fns.push_back(stream_kernel(prec_ == DMM_FP64, false));
-  fns.push_back(stream_kernel(prec_ == DMM_FP64, true));
+  if (prec_ == DMM_FP32) {
+    fns.push_back(stream_kernel(false));
+    fns.push_back(stream_kernel(true));
+  }
   for (const void* f : fns) {
     cudaFuncAttributes a;
     DMM_CUDA(cudaFuncGetAttributes(&a, f));
@@ -2649,7 +2640,7 @@ int Pack::launch_form() const {
   if (ctiles_h_.empty() && vtiles_h_.empty() && gr_groups_.size() == 1)
     return prec_ == DMM_FP32 && !gr_general_ ? 4 : 3;
   if (xp_active_) return xp_mt_ ? 6 : 4;
-  if (stream_active_) return prec_ == DMM_FP32 && !stream_general_ ? 6 : 3;
+  if (stream_active_) return !stream_general_ ? 6 : 3;
   if (one_active_) return 3;
   return 2;
 }

@@ -5,14 +5,12 @@
 
 namespace dmm {
 
-const void* stream_kernel(bool fp64, bool general) {
-  if (fp64)
-    return general ? (const void*)k_stream<double, true> : (const void*)k_stream<double, false>;
-  return general ? (const void*)k_stream<float, true> : (const void*)k_stream<float, false>;
+const void* stream_kernel(bool general) {
+  return general ? (const void*)k_stream<true> : (const void*)k_stream<false>;
 }
 
-StreamLayout stream_shape(int dl, int st, int bk, int tv, bool fp64) {
-  const int T = fp64 ? 8 : 4;
+StreamLayout stream_shape(int dl, int st, int bk, int tv) {
+  constexpr int T = 4;
   auto al = [](int x) { return (x + 15) & ~15; };
   StreamLayout L{};
   L.v0 = 0;
@@ -21,8 +19,7 @@ StreamLayout stream_shape(int dl, int st, int bk, int tv, bool fp64) {
   const int a = L.stage + al(T * st);
   L.b0 = 0;
   L.b1 = 16 + al(T * bk);
-  L.rank = L.b1 + 16 + al(T * bk);
-  const int bend = L.rank + (fp64 ? 16 * kRankMax * (kStreamThreads64 / 32) : 0);
+  const int bend = L.b1 + 16 + al(T * bk);
   L.total = std::max(std::max(a, bend), al(T * tv));
   return L;
 }
