@@ -1223,14 +1223,21 @@ dmm_status Pack::enqueue_step(bool rhs_only, void* dv_out) {
   return DMM_OK;
 }
 
-// cap: the kernel's largest dynamic shared memory (allow_smem)
-static int occupancy_blocks(const void* fn, int threads, size_t smem = 0, int cap = 0) {
-  int b = 1;
-  if (smem > 0 && allow_smem(fn, cap) != cudaSuccess) {
+// Blocks of a kernel that an SM holds at once, 0 when it cannot hold one: a cooperative launch
+// would be refused.  cap: the kernel's largest dynamic shared memory (allow_smem)
+static int resident_blocks(const void* fn, int threads, size_t smem, int cap) {
+  int b = 0;
+  if (allow_smem(fn, cap) != cudaSuccess ||
+      cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, fn, threads, smem) != cudaSuccess) {
     cudaGetLastError();
     return 0;
   }
-  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, fn, threads, smem) != cudaSuccess) {
+  return b;
+}
+
+static int occupancy_blocks(const void* fn, int threads) {
+  int b = 1;
+  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, fn, threads, 0) != cudaSuccess) {
     cudaGetLastError();
     b = 4;
   }
@@ -1598,7 +1605,7 @@ dmm_status Pack::plan_stream(int32_t idx, bool* ok) {
       continue;
     }
     stream_general_ = I.k3 == 0;
-    if (occupancy_blocks(stream_kernel(stream_general_), kStreamThreads, lay.total, kStreamSmemMax) < 1)
+    if (resident_blocks(stream_kernel(stream_general_), kStreamThreads, lay.total, kStreamSmemMax) < 1)
       return DMM_OK;
     stream_layout_ = lay;
     gr_tables_ = t;
@@ -1789,7 +1796,7 @@ dmm_status Pack::plan_grid(const std::vector<int32_t>& cand, std::vector<int32_t
       gr_resident_--;
     gr_layout_ = grid_shape(caps, fp64, general, gr_resident_);
     const void* fn = grid_kernel(fp64, general, gr_resident_);
-    if (occupancy_blocks(fn, fp64 ? kGridThreads64 : kGridThreads, gr_layout_.total, kGridSmemMax) < 1)
+    if (resident_blocks(fn, fp64 ? kGridThreads64 : kGridThreads, gr_layout_.total, kGridSmemMax) < 1)
       return DMM_OK;
     gr_general_ = general;
     gr_tables_ = t;
@@ -1932,7 +1939,7 @@ dmm_status Pack::prepare_xpose(int32_t idx, int TC, int TV, bool mt, bool* ok) {
   const int smem = mt ? xp_layout_mt(sv_cap, st_cap, bk_cap, TV).total
                       : xp_layout(sv_cap, bk_cap, TV).total;
   if (smem > staged_smem_max(mt)) return DMM_OK;
-  if (occupancy_blocks(staged_fn(tun_.var_group, mt), kStagedThreads, smem, staged_smem_max(mt)) * sms_ !=
+  if (resident_blocks(staged_fn(tun_.var_group, mt), kStagedThreads, smem, staged_smem_max(mt)) * sms_ !=
       grid_p_)
     return DMM_OK;
   xsv_cap_ = sv_cap;
