@@ -30,7 +30,8 @@
 // ends.  The energy of the last right-hand side is summed from the kept C_m at the end.
 //
 // The arithmetic is the other forms' (same clause, canonical-sum and candidate code), so the
-// states are identical to theirs; an FP64 energy differs in its last bits, as with any tiling.
+// states are identical to theirs; an FP64 energy, here the exact sum rounded once, differs from the
+// tile forms' plain sums in its last bits.
 #pragma once
 
 #include "dmm_cluster.h"
@@ -300,17 +301,46 @@ __device__ __forceinline__ double rank_sum(const double* u, const uint16_t* idx,
   return nan ? __longlong_as_double(0x7ff8000000000000ll) : acc;
 }
 
+// A sum with its rounding errors carried along (Knuth's two-sum): the energies of the forms that split
+// a formula over blocks come out as the exact sum of the C_m rounded once, whatever the split.  As
+// plain sums they were up to one unit in the last place off, in one formula's case or another's
+// depending on the split; the sums run once per launch.
+struct Sum2 {
+  double s = 0.0, c = 0.0;
+  __device__ __forceinline__ void add(double x) {
+    const double t = __dadd_rn(s, x), b = __dsub_rn(t, s);
+    c = __dadd_rn(c, __dadd_rn(__dsub_rn(s, __dsub_rn(t, b)), __dsub_rn(x, b)));
+    s = t;
+  }
+  __device__ __forceinline__ void add(const Sum2& o) {
+    add(o.s);
+    c = __dadd_rn(c, o.c);
+  }
+  __device__ __forceinline__ double value() const { return __dadd_rn(s, c); }
+};
+// The lanes' sum, in every lane.
+__device__ __forceinline__ Sum2 warp_sum2(Sum2 a) {
+#pragma unroll
+  for (int off = 16; off >= 1; off >>= 1) {
+    Sum2 o;
+    o.s = __shfl_xor_sync(0xffffffffu, a.s, off);
+    o.c = __shfl_xor_sync(0xffffffffu, a.c, off);
+    a.add(o);
+  }
+  return a;
+}
+
 struct ClusterShared {
   InstDesc I;
   InstCtrl S;
   int4 x[kClusterMax];      // from every block: unsatisfied, strict failures, trial index
-  double e[kClusterMax];    // energy partials (block 0, at the end of the launch)
+  double e[kClusterMax][2];  // energy partials (block 0, at the end of the launch)
   int base[kClusterMax + 1];  // CSR position where each block's variables start
   int nout[kClusterMax];      // contributions this block sends to each block
   int nin[kClusterMax];       // ... and receives from each
   int rin[kClusterMax];       // where this block's chunk starts in each block's bucket
   int soff[kClusterMax + 1];  // where each block's chunk starts in the staging area
-  double red[32];
+  double red[32][2];
   int cnt[3][32];
   int nlong;
   int32_t longq[kLongQueue];
@@ -675,24 +705,43 @@ __global__ void __launch_bounds__(sizeof(T) == 8 ? kClusterThreads64 : kClusterT
     T* cur = P.cand + (int64_t)(set * kTrials + kcur) * P.var_cap + I.var0;
     for (int i = tid; i < nv; i += NT) cur[v0 + i] = sV[v0 + i];
   }
-  double e = 0.0;
+  Sum2 e;
   for (int c = tid; c < tc; c += NT) {
     P.Xs[I.cls0 + c0 + c] = xs_s[c];
     P.Xl[I.cls0 + c0 + c] = xl_s[c];
     const T C = cp_s[c];
     P.Cp[I.cls0 + c0 + c] = C;
-    e = __dadd_rn(e, (double)C);  // FP32: exact (multiples of 2^-25)
+    e.add((double)C);
   }
-  e = warp_sum_d(e);
-  if (lane == 0) sc.red[w] = e;
+  e = warp_sum2(e);
+  if (lane == 0) {
+    sc.red[w][0] = e.s;
+    sc.red[w][1] = e.c;
+  }
   __syncthreads();
-  if (w == 0) e = warp_sum_d(lane < W ? sc.red[lane] : 0.0);
-  if (tid == 0)
-    st_cluster(cluster_map((unsigned)__cvta_generic_to_shared(&sc.e[0]) + 8 * rank, 0), e);
+  if (w == 0) {
+    Sum2 p;
+    if (lane < W) {
+      p.s = sc.red[lane][0];
+      p.c = sc.red[lane][1];
+    }
+    e = warp_sum2(p);
+  }
+  if (tid == 0) {
+    const unsigned at = cluster_map((unsigned)__cvta_generic_to_shared(&sc.e[0][0]) + 16 * rank, 0);
+    st_cluster(at, e.s);
+    st_cluster(at + 8, e.c);
+  }
   cluster_sync(R);
   if (rank == 0 && tid == 0) {
-    double es = 0.0;
-    for (unsigned r = 0; r < R; r++) es = __dadd_rn(es, sc.e[r]);
+    Sum2 total;
+    for (unsigned r = 0; r < R; r++) {
+      Sum2 p;
+      p.s = sc.e[r][0];
+      p.c = sc.e[r][1];
+      total.add(p);
+    }
+    const double es = total.value();
     InstCtrl* S = P.ctrl + sc.S.pad0;
     S->step = step;
     S->set = set;

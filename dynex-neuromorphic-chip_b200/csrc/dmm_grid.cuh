@@ -256,7 +256,7 @@ template <class T, bool GENERAL, int RES>
 __global__ void __launch_bounds__(sizeof(T) == 8 ? kGridThreads64 : kGridThreads, 1)
     k_grid(PackView<T> P, GridTables tb, const GridGroup* __restrict__ groups,
            const int32_t* __restrict__ blk_group, GridLayout LY, int nsteps, GridSync* sync_all,
-           double* __restrict__ epart, int* err) {
+           double2* __restrict__ epart, int* err) {
   constexpr int NT = sizeof(T) == 8 ? kGridThreads64 : kGridThreads;
   constexpr int W = NT / 32;
   constexpr int kw = 16 / (int)sizeof(T);  // values per 16-byte word
@@ -267,7 +267,7 @@ __global__ void __launch_bounds__(sizeof(T) == 8 ? kGridThreads64 : kGridThreads
   __shared__ GridPtrs<T> sp;
   __shared__ ClauseConsts<T> s_kc;
   __shared__ int cnt[3][W];
-  __shared__ double red[W];
+  __shared__ double red[W][2];
   __shared__ int s_ok, s_last, s_unsat, s_next;
   __shared__ int s_nq[kGridMaxTiles];  // lists of each variable tile that whole warps sum
   {
@@ -899,7 +899,7 @@ __global__ void __launch_bounds__(sizeof(T) == 8 ? kGridThreads64 : kGridThreads
   if (!gave_up && steps_run > 0) {
     T* cur = sp.cand + (int64_t)(lc.set * kTrials + lc.kcur) * P.var_cap;
     for (int i = tid; i < nv; i += NT) cur[var_at(i)] = s_cur[i];
-    double e = 0.0;
+    Sum2 e;
     for (int c = tid; c < c1 - c0; c += NT) {
       T C;
       if constexpr (RES == 2) {
@@ -910,14 +910,22 @@ __global__ void __launch_bounds__(sizeof(T) == 8 ? kGridThreads64 : kGridThreads
       } else {
         C = sp.Cp[c];
       }
-      e = __dadd_rn(e, (double)C);  // FP32: exact (multiples of 2^-25)
+      e.add((double)C);
     }
-    e = warp_sum_d(e);
-    if (lane == 0) red[w] = e;
+    e = warp_sum2(e);
+    if (lane == 0) {
+      red[w][0] = e.s;
+      red[w][1] = e.c;
+    }
     __syncthreads();
     if (w == 0) {
-      e = warp_sum_d(lane < W ? red[lane] : 0.0);
-      if (lane == 0) epart[blockIdx.x] = e;
+      Sum2 p;
+      if (lane < W) {
+        p.s = red[lane][0];
+        p.c = red[lane][1];
+      }
+      e = warp_sum2(p);
+      if (lane == 0) epart[blockIdx.x] = make_double2(e.s, e.c);
     }
   }
   if (b == 0 && w == W - 1 && lane == 0) {
@@ -932,11 +940,20 @@ __global__ void __launch_bounds__(sizeof(T) == 8 ? kGridThreads64 : kGridThreads
     s_last = atomicAdd(&gs->exits, 1u) == (unsigned)B - 1;
   }
   __syncthreads();
-  if (s_last && tid == 0) {  // the last block of the group to leave
+  Sum2 energy;
+  if (s_last && w == 0) {  // the last block of the group to leave
     __threadfence();
+    for (int q = lane; q < B; q += 32) {
+      const double2 v = __ldcg(epart + g.blk0 + q);
+      Sum2 p;
+      p.s = v.x;
+      p.c = v.y;
+      energy.add(p);
+    }
+    energy = warp_sum2(energy);
+  }
+  if (s_last && tid == 0) {
     if (!gave_up && steps_run > 0) {
-      double e = 0.0;
-      for (int q = 0; q < B; q++) e = __dadd_rn(e, __ldcg(epart + g.blk0 + q));
       InstCtrl* S = P.ctrl + g.inst;
       S->step = lc.step;
       S->set = lc.set;
@@ -948,7 +965,7 @@ __global__ void __launch_bounds__(sizeof(T) == 8 ? kGridThreads64 : kGridThreads
       S->vfail = *reinterpret_cast<volatile int*>(&gs->vfail);
       S->t = lc.t;
       S->h_state = lc.h;
-      S->energy = e;
+      S->energy = energy.value();
       if (lc.done == 1) {
         S->solved_step = lc.step - 1;
         S->solved_t = lc.solved_t;

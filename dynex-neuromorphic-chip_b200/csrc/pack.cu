@@ -1477,7 +1477,7 @@ dmm_status Pack::grid_tables(const std::vector<GridGroup>& groups, const std::ve
   bytes[kGrDlo] = z.bb * 4;
   bytes[kGrOut] = G * kGridOut * 4;
   bytes[kGrSync] = G * kGridSyncBytes;
-  bytes[kGrEpart] = (int64_t)nblocks * 8;
+  bytes[kGrEpart] = (int64_t)nblocks * 16;
   bytes[kGrBtot] = z.vt * 4;
   bytes[kGrPtot] = z.blks * 4;
   if (stream) bytes[kGrDv] = caps_.vars * T;
