@@ -187,8 +187,10 @@ class Pack {
   int64_t free_clauses() const { return cls_alloc_.largest_free(); }
   int64_t free_slots() const { return slot_alloc_.largest_free(); }
   int32_t free_insts() const;
-  int64_t tile_count(int which) const {
-    return which == 0 ? (int64_t)ctiles_h_.size() : (int64_t)vtiles_h_.size();
+  // the last commit left some formula to launch, in whichever form
+  bool planned() const {
+    return !ctiles_h_.empty() || !vtiles_h_.empty() || n_small_ > 0 || !clusters_.empty() ||
+           !gr_groups_.empty();
   }
   int sm_count() const { return sms_; }
 

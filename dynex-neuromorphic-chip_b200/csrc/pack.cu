@@ -393,9 +393,7 @@ dmm_status Pack::set_tuning(const dmm_tuning* t) {
   }
   tun_ = n;
   graph_stale_ = true;
-  if (!ctiles_h_.empty() || !vtiles_h_.empty() || n_small_ > 0 || !clusters_.empty() ||
-      !gr_groups_.empty())
-    return commit_tiles();
+  if (planned()) return commit_tiles();
   return DMM_OK;
 }
 
@@ -2527,9 +2525,7 @@ dmm_status Pack::capture(int32_t steps) {
 
 dmm_status Pack::launch_steps(int32_t nsteps) {
   DMM_CUDA(cudaSetDevice(dev_));
-  if (ctiles_h_.empty() && vtiles_h_.empty() && n_small_ == 0 && clusters_.empty() &&
-      gr_groups_.empty())
-    return DMM_OK;
+  if (!planned()) return DMM_OK;
   const int32_t S = tun_.steps_per_graph;
   if (nsteps <= short_steps()) {
     DMM_TRY(plan_short());

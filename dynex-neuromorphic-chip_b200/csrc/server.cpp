@@ -229,7 +229,7 @@ dmm_status dmm_server_pump(dmm_server* s, int32_t* resident, int32_t* queued) {
   DMM_TRY(retire(s));
   bool changed = false;
   DMM_TRY(admit(s, &changed));
-  if (changed || s->pack->tile_count(0) + s->pack->tile_count(1) == 0 ||
+  if (changed || !s->pack->planned() ||
       (int64_t)s->resident.size() != (int64_t)s->pack->num_live())
     DMM_TRY(s->pack->commit_tiles());
   if (!s->resident.empty()) {
