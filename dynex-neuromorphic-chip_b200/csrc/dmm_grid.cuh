@@ -459,19 +459,35 @@ __global__ void __launch_bounds__(sizeof(T) == 8 ? kGridThreads64 : kGridThreads
           }
           T xs = Xs[c], xl = Xl[c], C;
           const T al = acm ? acm[c] : kc.alpha;
-          if (o1 - o == 3) {
-            C = one(llit[o], llit[o + 1], llit[o + 2], spos[o], spos[o + 1], spos[o + 2], xs, xl,
-                    Cp[c], al);
+          if (pending) advance_memory(xs, xl, Cp[c], al, kc);
+          bool ss, three = o1 - o == 3;
+          int l0 = 0, l1 = 0, l2 = 0;
+          T V0 = T(0), V1 = T(0), V2 = T(0);
+          if (three) {
+            l0 = llit[o];
+            l1 = llit[o + 1];
+            l2 = llit[o + 2];
+            V0 = sV[abs(l0) - 1];
+            V1 = sV[abs(l1) - 1];
+            V2 = sV[abs(l2) - 1];
+            // a NaN is passed over by the general clause's minimum, not by clause3's
+            const T t = add(add(V0, V1), V2);
+            three = t == t;
+          }
+          if (three) {
+            T u0, u1, u2;
+            C = clause3(l0, l1, l2, V0, V1, V2, xs, xl, kc, u0, u1, u2, ss);
+            stage[spos[o]] = u0;
+            stage[spos[o + 1]] = u1;
+            stage[spos[o + 2]] = u2;
           } else {
-            if (pending) advance_memory(xs, xl, Cp[c], al, kc);
-            bool ss;
             C = clause_any<T>(
                 o1 - o, [&](int j) { return (int)llit[o + j]; },
                 [&](int l) { return sV[abs(l) - 1]; }, xs, xl, kc,
                 [&](int j) { return (int)spos[o + j]; }, [&](int p, T u) { stage[p] = u; }, ss);
-            unsat += !(C < T(0.5));
-            vf += !ss;
           }
+          unsat += !(C < T(0.5));
+          vf += !ss;
           Xs[c] = xs;
           Xl[c] = xl;
           Cp[c] = C;
