@@ -319,6 +319,15 @@ def repo_libraries() -> list[str]:
     return sorted(found)
 
 
+def reference_missing() -> str | None:
+    """Why the reference arm and the CPU baseline cannot run here, or None when they can."""
+    from oracle.oracle import REF_SO, reference_available
+
+    if reference_available():
+        return None
+    return f"{os.path.relpath(REF_SO, ROOT)} was not built: the reference's sources are not here"
+
+
 def cpu_reference(steps: int, warmup: int, procs: int):
     """The unmodified reference integrator (oracle/_ref, dynex.cc's own right-hand side and
     Euler step) on `procs` host processes at once, all on the bench instance and initial
@@ -371,6 +380,10 @@ def prior_art_child(steps: int, warmup: int) -> dict | None:
 def run_reference_arm(a):
     rank = int(os.environ.get("RANK", "0"))
     if rank != 0:
+        return
+    why = reference_missing()
+    if why:
+        print(json.dumps({"impl": "reference", "unavailable": why}), flush=True)
         return
     procs = a.procs or max(1, os.cpu_count() or 1)
     steps, warmup = a.steps, max(3, a.warmup)
@@ -637,7 +650,9 @@ def main():
     launch_ms = t_max / K  # one cooperative launch = one step
 
     cpu = None
-    if rank == 0 and world == 1 and not a.no_cpu_baseline:
+    if rank == 0 and world == 1 and not a.no_cpu_baseline and (why := reference_missing()):
+        cpu = {"unavailable": why}
+    elif rank == 0 and world == 1 and not a.no_cpu_baseline:
         v, info = cpu_reference(CPU_SAMPLE_STEPS, 3, 1)
         cpu = {"value": v, "unit": "clause-updates/s", "cores": 1, "kind": "reference",
                "sample": f"{CPU_SAMPLE_STEPS} steps (after 3 untimed) of the same formula and "
