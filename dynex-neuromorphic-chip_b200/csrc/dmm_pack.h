@@ -357,8 +357,8 @@ class Pack {
   cudaEvent_t ev_[4] = {nullptr, nullptr, nullptr, nullptr};
   int32_t* pinned_ = nullptr;  // page-locked copies of the status words and control records
   int32_t* live_d_ = nullptr;  // indices of the instances with tiles
-  int32_t* misc_d_ = nullptr;  // [0] live count, [1] barrier error, [2] barrier counter,
-                               // [3] formula queue of the one-block-per-formula kernel
+  int32_t* misc_d_ = nullptr;  // [0] live count, [3] formula queue of the
+                               // one-block-per-formula kernel; from kMiscLaunch the launch area
   int32_t* order_d_ = nullptr; // formulas run one block each, largest first
   int32_t n_small_ = 0;
   // cluster form: launches over formulas order_d_[first, first + count), one cluster each

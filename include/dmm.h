@@ -279,11 +279,13 @@ int32_t dmm_instance_step_kernel(const dmm_instance* inst);
 dmm_status dmm_instance_test_barrier_timeout(dmm_instance* inst);
 /* Benchmark helper: runs nsteps steps as plain launches with CUDA events around each of
  * the two step kernels; before each step it writes flush_bytes of scratch (0: none) so
- * the step starts with a cold L2.  Returns the summed device times (ms). */
+ * the step starts with a cold L2.  Returns the summed device times (ms).  These are the kernels of
+ * the two-kernel form (launch_mode 1), for which the formula is tiled anew and back, not those of
+ * dmm_instance_step_kernel. */
 dmm_status dmm_instance_profile(dmm_instance* inst, int32_t nsteps, int64_t flush_bytes,
                                 double* clause_ms, double* var_ms);
-/* Benchmark helper: device time (ms) of nsteps steps launched as the solver launches them
- * (CUDA-graph chunks, state resident on the device), one event pair around all of them. */
+/* Benchmark helper: device time (ms) of nsteps steps launched as dmm_instance_step launches them
+ * (state resident on the device), one event pair around all of them. */
 dmm_status dmm_instance_time_steps(dmm_instance* inst, int32_t nsteps, double* ms);
 /* Benchmark helper: nsteps steps, each launched on its own (one cooperative launch per
  * step, or the two phase kernels) after writing flush_bytes of scratch so that it starts
@@ -297,7 +299,8 @@ dmm_status dmm_instance_time_steps_flushed(dmm_instance* inst, int32_t nsteps,
  * over blocks of the microseconds from point k to point k+1 (point 10: the next step's
  * start), averaged over steps; out[20] = the SM clock (MHz) over the traced steps;
  * out[21], out[22] = mean microseconds from kernel entry to the first step (launch set-up)
- * and from the last step's end to kernel exit (staged kernel; 0 for the others).
+ * and from the last step's end to kernel exit (staged, resident grid and streaming kernels; 0 for
+ * the others).  A formula of the cluster kernel is traced in the form it would have without it.
  * DMM_ERR_STATE on the two-kernel launch form. */
 dmm_status dmm_instance_trace_phases(dmm_instance* inst, int32_t nsteps, double* out);
 
